@@ -472,7 +472,13 @@ bool q4_cuda_moe_exec_noalloc(const uint8_t *base, uint64_t stride, const int32_
                               uint64_t od, const float *d_x, float *d_h, float *d_y,
                               uint32_t n_ff, uint32_t in_dim, uint32_t n_embd, void *stream);
 
-/* Resident storage format of an arena.  By default q4_hip_experts_put*_a rewrites
+/* A tiled arena also gets a second copy of its tiles in a form of 4.25 bits a weight that the streaming and
+ * tensor-core products decode with a fraction of the instructions, while half of the device's memory stays
+ * free after taking it (1.24 times the arena; Q4B_WIDE=0 in the environment turns it off, and the products
+ * then decode the tiles).  It is brought up to date by q4_hip_experts_put*_a and retile_a, the two calls
+ * that change a tiled arena's bytes, and freed with the arena.
+ *
+ * Resident storage format of an arena.  By default q4_hip_experts_put*_a rewrites
  * each pack, in place and at the same size, into the library's tiled form of
  * IQ3_S (every run of eight 110-byte super-blocks regrouped by field so that all
  * device loads are aligned); base/stride/offset addressing is unchanged and every

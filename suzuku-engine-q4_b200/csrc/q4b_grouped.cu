@@ -678,12 +678,15 @@ bool launch_grouped_any(const uint8_t *w, uint64_t expert_stride, const int32_t 
     if (max_rows_hint == 0 || max_rows_hint > total_rows) max_rows_hint = total_rows;
     const bool tiled = q4b_ptr_tiled(w);
     const bool tc_ok = g_tc_mode != 0 && g_tc_mode != 2 && mmqtc::g_ready && mmqtc::shape_ok(w_rows, cols);
-    const bool few_ok = g_tc_mode != 2 && g_tc_mode != 1 && tiled && few::shape_ok(w_rows, cols, n_entries);
+    const bool wide_ok = g_tc_mode != 2 && g_tc_mode != 1 && tiled && wide::shape_ok(w, expert_stride, w_rows, cols, n_entries);
+    const bool few_ok = wide_ok || (g_tc_mode != 2 && g_tc_mode != 1 && tiled && few::shape_ok(w_rows, cols, n_entries));
     // rows an entry needs before the tensor cores take it
     uint32_t tc_min = 0xffffffffu;
     // a prefill-sized call (thousands of rows): the tensor-core kernel is running anyway and takes
     // entries from 6 rows (2048 tokens: 1.083 ms against 1.097 at 12, 1.086 at 4 and at 8)
-    const uint32_t split_rows = total_rows >= 4096u ? 6u : TC_MIN_ROWS;
+    // (on the wide form the streaming kernel takes every entry of a small call, and in a large one those of
+    // up to 64 rows: 370 experts of 32 rows take it 279 us, 512 of 17 rows take the tensor-core kernel 740)
+    const uint32_t split_rows = wide_ok ? (total_rows >= 4096u ? 65u : 0xffffffffu) : total_rows >= 4096u ? 6u : TC_MIN_ROWS;
     if (tc_ok) tc_min = g_tc_mode == 1 ? 1u : (few_ok ? split_rows : 0xffffffffu);
     if (tc_ok && g_tc_mode == -1 && !few_ok && total_rows >= 8ull * n_entries) tc_min = 1u;
     const bool run_tc = tc_min != 0xffffffffu && max_rows_hint >= tc_min;
@@ -706,6 +709,30 @@ bool launch_grouped_any(const uint8_t *w, uint64_t expert_stride, const int32_t 
         g_q4b_launches++;
         if (!ok || !q4b_launch_ok("mmq_tc")) return false;
         if (tc_min <= 1u) return true;
+    }
+    if (wide_ok) {
+        wide::Args a = {};
+        a.w = w;
+        a.expert_stride = expert_stride;
+        a.act = act;
+        a.n_act = n_act;
+        a.n_entries = n_entries;
+        a.bounds = bounds;
+        a.xq = xq.q;
+        a.xd = xq.d;
+        a.cols = cols;
+        a.w_rows = w_rows;
+        a.dst = dst;
+        a.ld_dst = ld_dst;
+        a.err = g_q4b.err_d;
+        a.max_rows = run_tc ? tc_min - 1u : 0x7fffffffu;
+        const bool ok = wide::launch(a);
+        g_q4b_launches++;
+        if (!ok || !q4b_launch_ok("wide_rows")) return false;
+        if (side && (cudaEventRecord(g_q4b.ev_join, g_q4b.aux_stream) != cudaSuccess ||
+                     cudaStreamWaitEvent(g_q4b.stream, g_q4b.ev_join, 0) != cudaSuccess))
+            return false;
+        return true;
     }
     if (few_ok) {
         few::Args a;
@@ -765,7 +792,7 @@ bool q4b_mmq_tc_warm() {
         cudaGetLastError();
         return false;
     }
-    const bool f = few::warm();
+    const bool f = few::warm() && wide::warm();
     return mmqtc::warm() && f;
 }
 extern "C" bool q4_cuda_mmq_tc_mode(int mode) {

@@ -37,6 +37,7 @@ struct Arena {
     uint64_t stride;
     uint64_t bytes;
     bool tiled;  // slots hold the tiled IQ3_S format (q4b_tile.cuh)
+    uint8_t *wide;   // the same tiles in the wide form, tile for tile, or NULL (no room for it)
 };
 Arena g_arena[4] = {};
 
@@ -110,6 +111,67 @@ bool launch_tile_permute(uint8_t *data, uint64_t bytes, bool forward, cudaStream
         tile_permute_k<false><<<nb, 256, 0, st>>>(data, n_tiles);
     g_q4b_launches++;
     return q4b_launch_ok("tile_permute");
+}
+
+// Tiled -> wide form, a warp per tile.  Runs behind every upload or conversion of arena bytes; bound by
+// the bytes it moves (880 read, 1088 written per tile).
+__global__ void __launch_bounds__(256) tile_widen_k(const uint8_t *__restrict__ tiled, uint8_t *__restrict__ wide,
+                                                    uint64_t n_tiles, const uint32_t *__restrict__ codes) {
+    __shared__ uint32_t tab[512];
+    for (uint32_t i = threadIdx.x; i < 512u; i += blockDim.x) tab[i] = __ldg(codes + i);
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint64_t t = (uint64_t)blockIdx.x * 8u + (threadIdx.x >> 5); t < n_tiles; t += (uint64_t)gridDim.x * 8u) {
+        const uint8_t *s = tiled + t * Q4B_TILE_BYTES;
+        uint8_t *o = wide + t * Q4B_WIDE_BYTES;
+        const uint4 qs = *reinterpret_cast<const uint4 *>(s + Q4B_TILE_OFF_QS + 16u * lane);
+        const uint2 sg = *reinterpret_cast<const uint2 *>(s + Q4B_TILE_OFF_SG + 8u * lane);
+        const uint32_t qh = *reinterpret_cast<const uint16_t *>(s + Q4B_TILE_OFF_QH + 2u * lane);
+        uint32_t n[2][8];   // c' of the lane's two groups, one nibble per byte, in weight order
+#pragma unroll
+        for (uint32_t h = 0; h < 2; h++)
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k++) {
+                const uint32_t w = h ? (k < 4 ? qs.z : qs.w) : (k < 4 ? qs.x : qs.y);
+                const uint32_t idx = ((w >> (8u * (k & 3u))) & 0xffu) | (((qh >> (8u * h + k)) & 1u) << 8);
+                const uint32_t t4 = (h ? sg.y : sg.x) << k;
+                n[h][k] = (tab[idx] ^ q4b_prmt(t4, t4, 0xba98u)) & 0x0f0f0f0fu;   // c or ~c
+            }
+#pragma unroll
+        for (uint32_t t4 = 0; t4 < 4; t4++)
+            *reinterpret_cast<uint2 *>(o + Q4B_WIDE_PART * t4 + 8u * lane) =
+                make_uint2(n[0][2 * t4] | (n[0][2 * t4 + 1] << 4), n[1][2 * t4] | (n[1][2 * t4 + 1] << 4));
+        if (lane < 8)
+            *reinterpret_cast<uint2 *>(o + Q4B_WIDE_PART * (lane >> 1) + 256u + 8u * (lane & 1u)) =
+                make_uint2(*reinterpret_cast<const uint16_t *>(s + Q4B_TILE_OFF_D + 2u * lane),
+                           *reinterpret_cast<const uint32_t *>(s + Q4B_TILE_OFF_SC + 4u * lane));
+    }
+}
+
+// Arena bytes [off, off + bytes) have changed: bring their wide form up to date on the same stream.
+bool launch_widen(const Arena &a, uint64_t off, uint64_t bytes, cudaStream_t st) {
+    const uint64_t n = bytes / Q4B_TILE_BYTES;
+    if (!a.wide || n == 0) return true;
+    const uint64_t nb = (n + 7) / 8;
+    tile_widen_k<<<(unsigned)(nb < 8u * 148u ? nb : 8u * 148u), 256, 0, st>>>(
+        a.base + off, a.wide + off / Q4B_TILE_BYTES * Q4B_WIDE_BYTES, n, g_q4b.codes_d);
+    g_q4b_launches++;
+    return q4b_launch_ok("tile_widen");
+}
+
+// The wide copy of a new arena: taken while half of the device's memory stays free after it, so that a
+// program whose memory is planned for the packs alone keeps fitting; without it the kernels that decode
+// the tiles themselves run.  Q4B_WIDE=0 turns it off.
+void alloc_wide(Arena *a) {
+    const char *e = getenv("Q4B_WIDE");
+    if (!a->tiled || (e && e[0] == '0')) return;
+    const uint64_t bytes = (a->stride / Q4B_TILE_BYTES) * (uint64_t)a->n_slots * Q4B_WIDE_BYTES;
+    size_t mem_free = 0, mem_all = 0;
+    if (cudaMemGetInfo(&mem_free, &mem_all) != cudaSuccess || mem_free < bytes + mem_all / 2 ||
+        cudaMalloc(&a->wide, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        a->wide = nullptr;
+    }
 }
 
 cudaEvent_t g_ev0, g_ev1;
@@ -227,6 +289,7 @@ extern "C" void q4_hip_shutdown(void) {
     cudaDeviceSynchronize();
     for (int a = 0; a < 4; a++) {
         if (g_arena[a].base) cudaFree(g_arena[a].base);
+        if (g_arena[a].wide) cudaFree(g_arena[a].wide);
         g_arena[a] = Arena{};
     }
     q4b_elem_shutdown();
@@ -363,6 +426,7 @@ extern "C" bool q4_hip_experts_alloc_a(int arena, uint32_t n_slots, uint64_t slo
     // the engine's byte order; the exec calls refuse a non-IQ3_S part on a tiled arena before
     // anything is enqueued).
     a.tiled = tiled_default() && (slot_bytes % (g_tiled_default == 2 ? Q4B_TILE_BYTES : 84480u)) == 0;
+    alloc_wide(&a);
     return true;
 }
 extern "C" void q4_hip_experts_free_a(int arena) {
@@ -370,6 +434,7 @@ extern "C" void q4_hip_experts_free_a(int arena) {
     if (g_arena[arena].base) {
         cudaDeviceSynchronize();
         cudaFree(g_arena[arena].base);
+        if (g_arena[arena].wide) cudaFree(g_arena[arena].wide);
     }
     g_arena[arena] = Arena{};
 }
@@ -384,7 +449,8 @@ extern "C" bool q4_hip_experts_put_async_a(int arena, uint32_t slot, const uint8
     if (a.tiled && (n % Q4B_TILE_BYTES)) return false;
     Q4B_CHECK(cudaMemcpyAsync(a.base + (uint64_t)slot * a.stride, host, n, cudaMemcpyHostToDevice,
                               g_q4b.copy_stream));
-    if (a.tiled && !launch_tile_permute(a.base + (uint64_t)slot * a.stride, n, true, g_q4b.copy_stream))
+    if (a.tiled && (!launch_tile_permute(a.base + (uint64_t)slot * a.stride, n, true, g_q4b.copy_stream) ||
+                    !launch_widen(a, (uint64_t)slot * a.stride, n, g_q4b.copy_stream)))
         return false;
     return true;
 }
@@ -539,6 +605,16 @@ bool q4b_ptr_tiled(const void *p) {
             return true;
     return q4b_wbuf_tiled(p);   // a gathered copy of a tiled arena keeps its byte order
 }
+// The wide copy of the tile at p (a tile boundary inside a tiled arena that has one), else NULL.
+const uint8_t *q4b_wide_of(const void *p) {
+    const uint8_t *q = (const uint8_t *)p;
+    for (int a = 0; a < 4; a++)
+        if (g_arena[a].wide && q >= g_arena[a].base && q < g_arena[a].base + g_arena[a].bytes) {
+            const uint64_t off = (uint64_t)(q - g_arena[a].base);
+            return off % Q4B_TILE_BYTES ? nullptr : g_arena[a].wide + off / Q4B_TILE_BYTES * Q4B_WIDE_BYTES;
+        }
+    return nullptr;
+}
 extern "C" void q4_cuda_set_tiled_default(int on) { g_tiled_default = on == 2 ? 2 : (on ? 1 : 0); }
 extern "C" int q4_cuda_experts_tiled_a(int arena) {
     return (arena >= 0 && arena < 4 && g_arena[arena].base && g_arena[arena].tiled) ? 1 : 0;
@@ -548,7 +624,8 @@ extern "C" bool q4_cuda_experts_retile_a(int arena, uint32_t first_slot, uint32_
     Arena &a = g_arena[arena];
     if (!a.base || !a.tiled || (uint64_t)first_slot + n_slots > a.n_slots || n_slots == 0) return false;
     return launch_tile_permute(a.base + (uint64_t)first_slot * a.stride, (uint64_t)n_slots * a.stride,
-                               true, g_q4b.stream);
+                               true, g_q4b.stream) &&
+           launch_widen(a, (uint64_t)first_slot * a.stride, (uint64_t)n_slots * a.stride, g_q4b.stream);
 }
 extern "C" bool q4_cuda_experts_get_a(int arena, uint32_t slot, uint8_t *host, uint64_t n) {
     if (!g_q4b.ok || arena < 0 || arena >= 4 || !host) return false;

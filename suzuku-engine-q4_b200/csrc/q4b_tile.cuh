@@ -49,6 +49,23 @@ __host__ __device__ inline uint32_t q4b_sign_unpermute(uint32_t w) {
     return o;
 }
 
+// The wide form: a second copy of a tile that costs a fraction of the instructions to decode.  A weight
+// of the codebook is an odd integer 2c' + 1 with c' in -8..7, so sign and codebook entry fit one
+// two's-complement nibble: with the nibble in the high half of a byte and 8 in the low half the byte IS
+// the signed number 8 (2c' + 1), one AND-OR for four weights, and neither table lookup nor sign mask is
+// left.  4.25 instead of 3.44 bits a weight.  A tile is four parts of 272 bytes, part t:
+//
+//   offset 272 t      q[64]   word t of every 32-weight group: weights 8t..8t+3 in the low nibbles of its
+//                             bytes, 8t+4..8t+7 in the high ones
+//          272 t+256  rec[2]  8 bytes for each of the super-blocks 2t, 2t+1: fp16 d, two spare bytes,
+//                             the 4 sub-scale bytes
+//
+// so that both readers are free of bank conflicts: a lane that owns groups 2l, 2l+1 (8 bytes of each
+// part), and the lanes (g, t) of an integer mma fragment (16 bytes of part t in each of 8 rows: 272 bytes
+// step four banks per part, 1088 step sixteen per tile).
+#define Q4B_WIDE_BYTES 1088u
+#define Q4B_WIDE_PART 272u
+
 #ifdef __CUDACC__
 
 __device__ __forceinline__ uint32_t q4b_prmt(uint32_t a, uint32_t b, uint32_t sel) {
@@ -89,6 +106,10 @@ __device__ __forceinline__ int32_t q4b_tile_group_idot(uint32_t qs_lo, uint32_t 
     }
     return 2 * (acc0 + acc1) + qsum;
 }
+
+// A word of the wide form -> four weights each as bytes 8w: the low nibbles, the high nibbles.
+__device__ __forceinline__ uint32_t q4b_wide_lo(uint32_t x) { return ((x << 4) & 0xf0f0f0f0u) | 0x08080808u; }
+__device__ __forceinline__ uint32_t q4b_wide_hi(uint32_t x) { return (x & 0xf0f0f0f0u) | 0x08080808u; }
 
 // One lane's share of a tile: block l/4, groups 2(l%4) and 2(l%4)+1.
 // q: 16 activation words of those 64 columns; dx/bs: their two group scales and

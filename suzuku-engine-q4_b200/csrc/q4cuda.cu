@@ -8,6 +8,7 @@
 #include "q4b_stack.cu"
 #include "q4b_mmq_tc.cu"
 #include "q4b_few.cu"
+#include "q4b_wide.cu"
 #include "q4b_grouped.cu"
 #include "q4b_elem.cu"
 #include "q4b_mmvq.cu"
