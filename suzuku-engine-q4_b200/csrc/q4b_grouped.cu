@@ -665,6 +665,9 @@ int g_tc_mode = -1;  // -1 split by rows, 0 CUDA cores only, 1 tensor cores when
 // an 8-way expert-parallel rank (8 own tokens, weights cold) moves to the tensor cores with its
 // four helper launches per layer: 9.3 ms per step against 7.8 ms with the split at 12.
 constexpr uint32_t TC_MIN_ROWS = 12;
+// 370 experts, gate/up: 16 rows 153 us streamed, 17 to 32 rows 284 (two passes over the weights), on the tensor cores
+// 255 with 17, 268 with 32, 321 with 64.
+constexpr uint32_t WIDE_TC_ROWS = 20;
 bool launch_grouped_any(const uint8_t *w, uint64_t expert_stride, const int32_t *act,
                         const uint32_t *n_act, uint32_t n_entries, const int32_t *bounds, Q8View xq,
                         uint64_t total_rows, uint32_t cols, uint32_t w_rows, float *dst,
@@ -679,15 +682,22 @@ bool launch_grouped_any(const uint8_t *w, uint64_t expert_stride, const int32_t 
     const bool tiled = q4b_ptr_tiled(w);
     const bool tc_ok = g_tc_mode != 0 && g_tc_mode != 2 && mmqtc::g_ready && mmqtc::shape_ok(w_rows, cols);
     const bool wide_ok = g_tc_mode != 2 && g_tc_mode != 1 && tiled && wide::shape_ok(w, expert_stride, w_rows, cols, n_entries);
+    // On the wide form one kernel takes the whole call: the tensor-core kernel from an average of
+    // WIDE_TC_ROWS rows per possible entry on (or in mode 1), the streaming kernel below.
+    if (tiled && tc_ok && mmqtc::wide_ok(w, expert_stride, total_rows, w_rows, cols, n_entries) &&
+        (g_tc_mode == 1 || (wide_ok && total_rows >= (uint64_t)WIDE_TC_ROWS * n_entries))) {
+        const bool ok = mmqtc::launch_wide(w, expert_stride, act, n_act, n_entries, bounds, xq.q, xq.d, xq.h1, xq.h2, xq.rs,
+                                           total_rows, cols, w_rows, dst, ld_dst);
+        g_q4b_launches += 3;
+        return ok && q4b_launch_ok("mmq_wide");
+    }
     const bool few_ok = wide_ok || (g_tc_mode != 2 && g_tc_mode != 1 && tiled && few::shape_ok(w_rows, cols, n_entries));
     // rows an entry needs before the tensor cores take it
     uint32_t tc_min = 0xffffffffu;
     // a prefill-sized call (thousands of rows): the tensor-core kernel is running anyway and takes
     // entries from 6 rows (2048 tokens: 1.083 ms against 1.097 at 12, 1.086 at 4 and at 8)
-    // (on the wide form the streaming kernel takes every entry of a small call, and in a large one those of
-    // up to 64 rows: 370 experts of 32 rows take it 279 us, 512 of 17 rows take the tensor-core kernel 740)
-    const uint32_t split_rows = wide_ok ? (total_rows >= 4096u ? 65u : 0xffffffffu) : total_rows >= 4096u ? 6u : TC_MIN_ROWS;
-    if (tc_ok) tc_min = g_tc_mode == 1 ? 1u : (few_ok ? split_rows : 0xffffffffu);
+    const uint32_t split_rows = total_rows >= 4096u ? 6u : TC_MIN_ROWS;
+    if (tc_ok && !wide_ok) tc_min = g_tc_mode == 1 ? 1u : (few_ok ? split_rows : 0xffffffffu);
     if (tc_ok && g_tc_mode == -1 && !few_ok && total_rows >= 8ull * n_entries) tc_min = 1u;
     const bool run_tc = tc_min != 0xffffffffu && max_rows_hint >= tc_min;
     // When a call is split, the two kernels touch disjoint entries and rows: the tensor-core
@@ -793,7 +803,7 @@ bool q4b_mmq_tc_warm() {
         return false;
     }
     const bool f = few::warm() && wide::warm();
-    return mmqtc::warm() && f;
+    return mmqtc::warm() && mmqtc::warm_wide() && f;
 }
 extern "C" bool q4_cuda_mmq_tc_mode(int mode) {
     if (mode < -1 || mode > 2 || (mode == 1 && !mmqtc::g_ready)) return false;

@@ -583,7 +583,10 @@ __global__ void __launch_bounds__(NT, 1) mmq_tc_k(const Args a, const __grid_con
 // The fp16 planes of the quantised activation rows: x = q * dq (the value the 8-bit row stands
 // for), divided by the power of two rs that brings the row's largest magnitude below 1, as
 // h1 = fp16(x / rs) and h2 = fp16(x / rs - h1).  A row is taken by tpr = min(256, cols / 8)
-// threads, eight values each per turn; a CTA of 256 threads holds 256 / tpr rows.
+// threads, eight values each per turn; a CTA of 256 threads holds 256 / tpr rows.  WIDE: in the
+// order in which the wide form's decode leaves the weights: the eight values of a chunk as 0 2 4 6 1 3 5 7, the 16
+// chunks of 128 values transposed as a 4 x 4 matrix.
+template <bool WIDE>
 __global__ void __launch_bounds__(256) planes_k(const int8_t *__restrict__ q, const float *__restrict__ dq,
                                                 uint64_t rows, uint32_t cols, uint32_t tpr,
                                                 __half *__restrict__ h1, __half *__restrict__ h2,
@@ -616,8 +619,10 @@ __global__ void __launch_bounds__(256) planes_k(const int8_t *__restrict__ q, co
         uint32_t p1[4], p2[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const uint32_t word = i < 2 ? w.x : w.y;
-            const int qa = (int)(int8_t)(word >> (16 * (i & 1))), qb = (int)(int8_t)(word >> (16 * (i & 1) + 8));
+            // values 2i, 2i + 1 of the chunk; WIDE: 4 (i & 1) + (i >> 1) and two further
+            const uint32_t word = WIDE ? ((i & 1) ? w.y : w.x) : (i < 2 ? w.x : w.y);
+            const int at = WIDE ? 8 * (i >> 1) : 16 * (i & 1), gap = WIDE ? 16 : 8;
+            const int qa = (int)(int8_t)(word >> at), qb = (int)(int8_t)(word >> (at + gap));
             const float xa = (float)qa * sc, xb = (float)qb * sc;
             const __half2 a1 = __floats2half2_rn(xa, xb);
             const float2 back = __half22float2(a1);
@@ -625,8 +630,9 @@ __global__ void __launch_bounds__(256) planes_k(const int8_t *__restrict__ q, co
             p1[i] = *reinterpret_cast<const uint32_t *>(&a1);
             p2[i] = *reinterpret_cast<const uint32_t *>(&a2);
         }
-        *reinterpret_cast<uint4 *>(o1 + c) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
-        *reinterpret_cast<uint4 *>(o2 + c) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+        const uint32_t k = c >> 3, to = WIDE ? ((k & ~15u) | ((k & 3u) << 2) | ((k >> 2) & 3u)) << 3 : c;
+        *reinterpret_cast<uint4 *>(o1 + to) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+        *reinterpret_cast<uint4 *>(o2 + to) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
     }
 }
 
@@ -713,7 +719,7 @@ bool launch(const uint8_t *w, uint64_t expert_stride, const int32_t *act, const 
     {
         const uint32_t tpr = cols / 8u < 256u ? cols / 8u : 256u;   // cols % 256 == 0: a multiple of 32
         const uint32_t rpb = 256u / tpr;
-        planes_k<<<(unsigned)((rows + rpb - 1) / rpb), 256, 0, stream>>>(q, dq, rows, cols, tpr, h1, h2, rs);
+        planes_k<false><<<(unsigned)((rows + rpb - 1) / rpb), 256, 0, stream>>>(q, dq, rows, cols, tpr, h1, h2, rs);
     }
     Args a;
     a.w = w;

@@ -26,6 +26,7 @@ bool q4b_route_small_warm();   // q4b_decode.cu: counters of the one-launch rout
 void q4b_route_small_shutdown();
 void q4b_mmvq_shutdown();
 bool q4b_wbuf_tiled(const void *p);
+bool q4b_router_tc_warm();   // q4b_router.cu: shared-memory limit of the batch router product
 bool q4b_mmq_tc_warm();  // q4b_grouped.cu: tensor-core grouped product (optional)
 std::atomic<uint64_t> g_q4b_launches{0};
 
@@ -190,6 +191,7 @@ bool alloc_scratch() {
     Q4B_CHECK(cudaMalloc(&s.r_wts, (size_t)Q4B_MAX_TOK * 64 * sizeof(float)));
     Q4B_CHECK(cudaMalloc(&s.r_cnt, (size_t)Q4B_MAX_TOK * sizeof(int32_t)));
     Q4B_CHECK(cudaMalloc(&s.hbuf, nq * sizeof(float)));
+    q4b_router_tc_warm();
     q4b_mmq_tc_warm();  // without it the grouped product stays on the CUDA cores
     return q4b_fused_warm() && q4b_window_warm() && q4b_elem_warm() && q4b_mmvq_warm() && q4b_route_small_warm();
 }

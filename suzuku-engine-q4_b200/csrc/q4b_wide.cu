@@ -12,9 +12,9 @@
 //   1 or 2 rows  a lane owns a tile's groups 2l, 2l+1 (block l/4), its 64 activation bytes a row live
 //                in registers, dp4a; the sums of a warp's tiles are reduced together, so four tiles
 //                cost six shuffles a row instead of twenty
-//   3..16 rows   integer mma m16n8k32 (16 activation rows x 8 weight rows x one 32-group): the weight
-//                word of lane (g, t) IS the B fragment after one AND-OR per half, the activations are
-//                the A fragment as they lie in shared memory.  Warps split a unit of 8 weight rows
+//   3..16 rows   integer mma m16n8k32 (16 weight rows x 8 activation rows x one 32-group): the weight
+//                words of lane (g, t) ARE the A fragment after one AND-OR per half, the activations are
+//                the B fragment as they lie in shared memory.  Warps split a unit of 16 weight rows
 //                along k when a chunk has fewer than 16 units.
 // Both form the exact integer dot of every 32-group (times 8) and then the expression and the order of
 // additions of grouped_rows_k (pairs of groups, blocks of four pairs, blocks pairwise), so for 1, 2, 4 or 8
@@ -33,20 +33,20 @@ namespace wide {
 constexpr uint32_t NCW = 16;                     // warps
 constexpr uint32_t NT = 32 * NCW;
 constexpr uint32_t MAX_ENTRIES = 1024;
-constexpr uint32_t RBLK = 16;                    // activation rows of an item
+constexpr uint32_t RBLK = 16;                    // activation rows of an item at most
 constexpr uint32_t MAX_STAGE = 8;
 constexpr uint32_t WAIT_LIMIT = 1u << 21;        // tries before a wait gives up ...
 constexpr unsigned long long WAIT_NS = 500000000ull;   // ... or half a second, whichever comes first
 constexpr uint32_t ERR_WIDE = 0x1000u;
 
 struct Smem {
-    unsigned long long full[MAX_STAGE];
+    unsigned long long full[MAX_STAGE], act_full[2];
     uint32_t done[MAX_STAGE];                    // warps that are through with a stage's chunk
-    // where the stream stands: entry of the live list, block of rows, chunk, items so far
-    uint32_t p_li, p_blk, p_ch, p_item, p_rows;
-    int32_t p_r0;
+    // where the two streams stand (entry of the live list, block of rows): chunks, activation rows
+    uint32_t p_li, p_blk, p_ch, p_nb, x_li, x_blk, x_item;
+    bool p_new;
     const uint8_t *p_mat;
-    float red[NCW - 2][32][4];                   // partial sums of warps that share a unit (all but one of each unit)
+    alignas(16) float red[NCW - 2][32][4];                // partial sums of warps that share a unit (all but one of each unit)
     uint32_t live[MAX_ENTRIES];                  // entries with rows
     uint32_t cost[MAX_ENTRIES + 1];              // cost of everything before entry i of that list
     uint32_t wl[NCW], wc[NCW];                   // per-warp sums of the scan
@@ -123,15 +123,28 @@ __device__ __forceinline__ void sub_scale(uint32_t s, uint32_t at, float &l, flo
 // smem strides of an activation row and of its scales (padding against bank conflicts)
 __host__ __device__ inline uint32_t act_stride(uint32_t cols) { return cols + 32u; }
 __host__ __device__ inline uint32_t scale_stride(uint32_t cols) { return (cols >> 5) * 4u + 16u; }
-__host__ __device__ inline uint32_t act_bytes(uint32_t cols) { return RBLK * (act_stride(cols) + scale_stride(cols)); }
-__host__ __device__ inline uint32_t smem_bytes(uint32_t cols, uint32_t ct, uint32_t n_stage) {
-    return (uint32_t)((sizeof(Smem) + 127u) & ~127u) + 2u * ((act_bytes(cols) + 127u) & ~127u) + n_stage * ct * Q4B_WIDE_BYTES;
+__host__ __device__ inline uint32_t act_bytes(uint32_t cols) {
+    return (RBLK * (act_stride(cols) + scale_stride(cols)) + 127u) & ~127u;
 }
-// Relative cost of a chunk for a block of rows: the stream of its bytes until the rows' own work exceeds it.
-__device__ __forceinline__ uint32_t block_cost(uint32_t rows) { return rows <= 2u ? 7u + rows : rows <= 8u ? 12u : 17u; }
-__device__ __forceinline__ uint32_t entry_cost(uint32_t rows, uint32_t cpe) {
+__host__ __device__ inline uint32_t smem_bytes(uint32_t cols, uint32_t ct, uint32_t n_stage) {
+    return (uint32_t)((sizeof(Smem) + 127u) & ~127u) + 2u * act_bytes(cols) + n_stage * ct * Q4B_WIDE_BYTES;
+}
+// Relative cost of a chunk for a block of rows: the stream of its bytes until the rows' own work exceeds it
+// (370 experts, gate/up: 72 us with 1 row, 80 with 2, 105 with up to 8, 145 with up to 16).
+__device__ __forceinline__ uint32_t block_cost(uint32_t rows) {
+    return rows <= 2u ? 7u + rows : rows <= 8u ? 12u : 17u;
+}
+// An entry's rows are split evenly over as few blocks of RBLK as hold them.
+struct Split {
+    uint32_t nb, per;
+};
+__device__ __forceinline__ Split split_rows(uint32_t rows) {
     const uint32_t nb = (rows + RBLK - 1u) / RBLK;
-    return cpe * ((nb - 1u) * block_cost(RBLK) + block_cost(rows - (nb - 1u) * RBLK));
+    return {nb, nb == 1u ? rows : (rows + nb - 1u) / nb};
+}
+__device__ __forceinline__ uint32_t entry_cost(uint32_t rows, uint32_t cpe) {
+    const Split sp = split_rows(rows);
+    return cpe * sp.nb * block_cost(sp.per);
 }
 
 // BB: super-blocks per weight row, 1, 2, 4 or 8; 0 = another number (mma form only).  TPW: tiles a warp takes
@@ -141,7 +154,7 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     Smem &s = *reinterpret_cast<Smem *>(smem_raw);
     uint8_t *const actb = smem_raw + ((sizeof(Smem) + 127u) & ~127u);
-    const uint32_t act_sz = (act_bytes(a.cols) + 127u) & ~127u;
+    const uint32_t act_sz = act_bytes(a.cols), sc_off = RBLK * act_stride(a.cols);
     uint8_t *const stage = actb + 2u * act_sz;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t n_ent = a.n_act ? min(*a.n_act, a.n_entries) : a.n_entries;
@@ -153,6 +166,8 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s.full[i])), "r"(1u));
             s.done[i] = 0;
         }
+        for (uint32_t i = 0; i < 2; i++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s.act_full[i])), "r"(1u));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // ---- the live entries and the prefix of their costs: a thread takes two neighbouring entries ----
@@ -209,7 +224,7 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
             else hi = mid;
         }
         const uint32_t e = s.live[lo], rows = (uint32_t)(a.bounds[e + 1] - a.bounds[e]);
-        const uint32_t n = (rows + RBLK - 1u) / RBLK * cpe, ec = s.cost[lo + 1] - s.cost[lo];
+        const uint32_t n = split_rows(rows).nb * cpe, ec = s.cost[lo + 1] - s.cost[lo];
         const uint32_t w = (uint32_t)(((target - s.cost[lo]) * n + ec - 1u) / ec);
         ent = w >= n ? lo + 1u : lo;
         idx = w >= n ? 0u : w;
@@ -218,51 +233,55 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
     locate((uint64_t)total_cost * blockIdx.x / gridDim.x, li, ix);
     locate((uint64_t)total_cost * (blockIdx.x + 1ull) / gridDim.x, li_end, ix_end);
 
-    // ---- the stream ----
-    // The warp that is last through a chunk refills its stage with the next chunk of this CTA's share (one
-    // lane; refills come in order, because a warp leaves chunk k + 1 only after it has refilled behind
-    // chunk k).  The first chunk of an item brings its activation rows along.  Two buffers of rows are
-    // enough: the chunks in flight and in use belong to at most two items while the ring is no deeper
-    // than the chunks of an item plus one.
+    // ---- the streams ----
+    // The warp that is last through a chunk refills its stage with the next chunk of this CTA's share, and the one that
+    // is last through an item's last chunk brings the activation rows of the item after the next into the buffer
+    // that has become free (one lane; refills come in order, because a warp leaves chunk k + 1 only after it has
+    // refilled behind chunk k).
     const uint32_t blk_end = ix_end / cpe, ch_end = ix_end - blk_end * cpe, chunk_bytes = a.ct * Q4B_WIDE_BYTES;
     const uint32_t last_tiles = n_tiles - (cpe - 1u) * a.ct;
+    auto rows_of = [&](uint32_t e) { return (uint32_t)(__ldg(a.bounds + e + 1) - __ldg(a.bounds + e)); };
     auto refill = [&](uint32_t st) {
         uint32_t pl = s.p_li, pb = s.p_blk, pc = s.p_ch;
         if (pl == li_end && pb == blk_end && pc == ch_end) return;
-        const uint32_t item = s.p_item;
-        const bool first = item == 0 || pc == 0;
-        if (item == 0 || (pc == 0 && pb == 0)) {
+        if (s.p_new) {
             const uint32_t e = s.live[pl];
-            s.p_r0 = __ldg(a.bounds + e);
-            s.p_rows = (uint32_t)(__ldg(a.bounds + e + 1) - s.p_r0);
+            s.p_nb = split_rows(rows_of(e)).nb;
             s.p_mat = a.w + (uint64_t)(a.act ? __ldg(a.act + e) : (int32_t)e) * a.expert_stride;
         }
-        const uint32_t rows = s.p_rows, sb = (a.cols >> 5) * 4u;
         const uint32_t bytes = pc + 1u == cpe ? last_tiles * Q4B_WIDE_BYTES : chunk_bytes;
-        const uint32_t arows = first ? min(rows - pb * RBLK, RBLK) : 0u;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&s.full[st])),
-                     "r"(bytes + arows * (a.cols + sb))
-                     : "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&s.full[st])), "r"(bytes) : "memory");
         bulk_g2s(stage + st * chunk_bytes, s.p_mat + (uint64_t)pc * chunk_bytes, bytes, &s.full[st]);
-        if (first) {
-            uint8_t *const ab = actb + (item & 1u) * act_sz;
-            const uint64_t rr = (uint64_t)s.p_r0 + pb * RBLK;
-            for (uint32_t i = 0; i < arows; i++) {
-                bulk_g2s(ab + i * act_stride(a.cols), a.xq + (rr + i) * a.cols, a.cols, &s.full[st]);
-                bulk_g2s(ab + RBLK * act_stride(a.cols) + i * scale_stride(a.cols), a.xd + (rr + i) * (a.cols >> 5), sb,
-                         &s.full[st]);
-            }
-            s.p_item = item + 1u;
-        }
+        bool next = false;
         if (++pc == cpe) {
             pc = 0;
-            if (++pb * RBLK >= rows) pb = 0, pl++;
+            if (++pb == s.p_nb) pb = 0, pl++, next = true;
         }
-        s.p_li = pl, s.p_blk = pb, s.p_ch = pc;
+        s.p_li = pl, s.p_blk = pb, s.p_ch = pc, s.p_new = next;
     };
-    if (tid == 0) {
-        s.p_li = li, s.p_blk = ix / cpe, s.p_ch = ix % cpe, s.p_item = 0;
+    auto refill_rows = [&]() {
+        uint32_t xl = s.x_li, xb = s.x_blk;
+        if (xl > li_end || (xl == li_end && (xb > blk_end || (xb == blk_end && ch_end == 0)))) return;   // past the share
+        const uint32_t e = s.live[xl], rows = rows_of(e), buf = s.x_item & 1u, sb = (a.cols >> 5) * 4u;
+        const Split sp = split_rows(rows);
+        const uint32_t nr = min(sp.per, rows - xb * sp.per);
+        const uint64_t r0 = (uint64_t)__ldg(a.bounds + e) + xb * sp.per;
+        uint8_t *const ab = actb + buf * act_sz;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&s.act_full[buf])),
+                     "r"(nr * (a.cols + sb))
+                     : "memory");
+        for (uint32_t i = 0; i < nr; i++) {
+            bulk_g2s(ab + i * act_stride(a.cols), a.xq + (r0 + i) * a.cols, a.cols, &s.act_full[buf]);
+            bulk_g2s(ab + sc_off + i * scale_stride(a.cols), a.xd + (r0 + i) * (a.cols >> 5), sb, &s.act_full[buf]);
+        }
+        if (++xb == sp.nb) xb = 0, xl++;
+        s.x_li = xl, s.x_blk = xb, s.x_item++;
+    };
+    if (tid == 0 && (li != li_end || ix != ix_end)) {
+        s.p_li = s.x_li = li, s.p_blk = s.x_blk = ix / cpe, s.p_ch = ix % cpe, s.p_new = true, s.x_item = 0;
+        refill_rows();
         for (uint32_t i = 0; i < a.n_stage; i++) refill(i);
+        refill_rows();
     }
 
     // ---- the warps ----
@@ -274,15 +293,20 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
     const uint32_t b_lo = (B * ks) >> a.ks_log, b_hi = (B * (ks + 1u)) >> a.ks_log;
     bool entry = true;
     uint32_t rows = 0;
+    Split sp = {1u, 0u};
     // one item: a chunk after the other
     while (li != li_end || blk != blk_end || ch != ch_end) {
         const uint32_t e = s.live[li];
         const int32_t r0 = __ldg(a.bounds + e);
-        if (entry) rows = (uint32_t)(__ldg(a.bounds + e + 1) - r0);
+        if (entry) {
+            rows = (uint32_t)(__ldg(a.bounds + e + 1) - r0);
+            sp = split_rows(rows);
+        }
         entry = false;
-        const uint32_t nr = min(rows - blk * RBLK, RBLK);
-        float *const out = a.dst + (uint64_t)((uint32_t)r0 + blk * RBLK) * a.ld_dst;
-        const uint8_t *const ab = actb + (item & 1u) * act_sz, *const sbase = ab + RBLK * act_stride(a.cols);
+        const uint32_t nr = min(sp.per, rows - blk * sp.per), buf = item & 1u;
+        float *const out = a.dst + (uint64_t)((uint32_t)r0 + blk * sp.per) * a.ld_dst;
+        const uint8_t *const ab = actb + buf * act_sz, *const sbase = ab + sc_off;
+        if (!mbar_wait(&s.act_full[buf], (item >> 1) & 1u, limit, a.err)) limit = 1024u;
         const uint32_t ch_stop = li == li_end && blk == blk_end ? ch_end : cpe;
         auto acquire = [&]() {
             if (!mbar_wait(&s.full[st], ph, limit, a.err)) limit = 1024u;
@@ -295,6 +319,7 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
                 asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(n) : "r"(smem_u32(&s.done[st])) : "memory");
                 if (n == NCW - 1u) {
                     s.done[st] = 0;
+                    if (ch + 1u == cpe) refill_rows();   // the item's last chunk: its buffer is free
                     refill(st);
                 }
             }
@@ -501,7 +526,7 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
         if (ch_stop != cpe) break;         // the end of this CTA's share
         item++;
         ch = 0, blk++;
-        if (blk * RBLK >= rows) blk = 0, li++, entry = true;
+        if (blk == sp.nb) blk = 0, li++, entry = true;
     }
 }
 
@@ -518,8 +543,10 @@ bool warm() {
     return g_ready;
 }
 
-// Chunk and ring of a call.  Chunks of 64 tiles pay the barriers once per four tiles of a warp; a call with
-// little work per CTA takes 32, so that its shares differ by less and its pipeline fills sooner.
+// Chunk and ring of a call.  Chunks of 64 tiles pay the barriers once per four tiles of a warp; a call with little
+// work per CTA takes 32, so that its shares differ by less and its pipeline fills sooner.  (Items of 32 rows, three or
+// four fragments a warp, were slower than two passes of 16: they spill, and their rows leave room for 32 tiles a
+// chunk only: 370 experts of 32 rows 425 us against 284.)
 static bool plan(Args &a) {
     const uint32_t B = a.cols >> 8;
     const uint64_t tiles = (uint64_t)(a.w_rows >> 3) * B * a.n_entries;
@@ -531,8 +558,7 @@ static bool plan(Args &a) {
         a.ct = units * 2u * B;
         a.ks_log = 0;
         while ((units << (a.ks_log + 1u)) <= NCW && (2u << a.ks_log) <= B && a.ks_log < 3u) a.ks_log++;
-        const uint32_t cpe = (((a.w_rows >> 3) * B) + a.ct - 1u) / a.ct;   // the two buffers of rows allow cpe + 1
-        a.n_stage = cpe + 1u < MAX_STAGE ? cpe + 1u : MAX_STAGE;
+        a.n_stage = MAX_STAGE;
         while (a.n_stage >= 2u && smem_bytes(a.cols, a.ct, a.n_stage) > SMEM_MAX) a.n_stage--;
         if (a.n_stage >= 2u || want < 4u * B) break;
     }

@@ -7,6 +7,8 @@
 #include "q4b_synth.cu"
 #include "q4b_stack.cu"
 #include "q4b_mmq_tc.cu"
+#include "q4b_wide_tc.cu"
+#include "q4b_router.cu"
 #include "q4b_few.cu"
 #include "q4b_wide.cu"
 #include "q4b_grouped.cu"

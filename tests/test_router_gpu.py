@@ -1,0 +1,30 @@
+"""The router product of more than 256 tokens (csrc/q4b_router.cu: fp32 operands as three bf16 parts on the
+tensor cores) against the product in double: edges of its tiles (128 tokens, 64 experts, 128 columns), one
+row with an outlier, and error no larger than that of fp32 additions in sequence."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n_tok,n_exp,n", [(257, 48, 1024), (300, 195, 2048), (512, 512, 2048), (641, 130, 2560), (259, 3, 132)])
+def test_batch_router_product(dev, n_tok, n_exp, n):
+    rng = np.random.default_rng(n_tok + n)
+    x = rng.standard_normal((n_tok, n)).astype(np.float32)
+    x[5, 7] = 4000.0
+    w = (rng.standard_normal((n_exp, n)) * 0.02).astype(np.float32)
+    d_y = dev.malloc(n_tok * n_exp * 4)
+    dev.write(d_y, np.full((n_tok, n_exp), 7.5, np.float32))
+    assert dev.lib.q4_hip_gemv_dd_n(0, dev.upload(w), n_exp, n, dev.upload(x), d_y, 0.5, n_tok)
+    y = dev.download(d_y, (n_tok, n_exp), np.float32)
+    want = 0.5 * x.astype(np.float64) @ w.astype(np.float64).T
+    seq = np.zeros((n_tok, n_exp), np.float32)
+    for h in range(n):
+        seq += x[:, h:h + 1] * w[:, h]
+    err, err_seq = np.abs(y - want), np.abs(0.5 * seq - want)
+    plain = np.arange(n_tok) != 5                       # without the outlier's row
+    print("router product: error %.3g (%.3g), of fp32 additions in sequence %.3g (%.3g)" %
+          (err.max(), np.linalg.norm(err[plain]), err_seq.max(), np.linalg.norm(err_seq[plain])))
+    assert err[5].max() <= max(err_seq[5].max(), 2.0 ** -21 * np.abs(want[5]).max())
+    assert np.linalg.norm(err[plain]) <= np.linalg.norm(err_seq[plain])
+    assert dev.lib.q4_cuda_device_error() == 0
