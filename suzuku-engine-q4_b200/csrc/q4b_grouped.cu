@@ -665,8 +665,8 @@ int g_tc_mode = -1;  // -1 split by rows, 0 CUDA cores only, 1 tensor cores when
 // an 8-way expert-parallel rank (8 own tokens, weights cold) moves to the tensor cores with its
 // four helper launches per layer: 9.3 ms per step against 7.8 ms with the split at 12.
 constexpr uint32_t TC_MIN_ROWS = 12;
-// 370 experts, gate/up: 16 rows 153 us streamed, 17 to 32 rows 284 (two passes over the weights), on the tensor cores
-// 255 with 17, 268 with 32, 321 with 64.
+// 370 experts, gate/up + down, us: 16 rows 161 + 87 streamed, 17 rows 262 + 138, 20 rows 293 + 154 (two passes over the
+// weights), 32 rows 299 + 156; on the tensor cores 266 + 157, 264 + 160, 269 + 162, 283 + 165, and 338 + 190 with 64 rows.
 constexpr uint32_t WIDE_TC_ROWS = 20;
 bool launch_grouped_any(const uint8_t *w, uint64_t expert_stride, const int32_t *act,
                         const uint32_t *n_act, uint32_t n_entries, const int32_t *bounds, Q8View xq,

@@ -12,7 +12,7 @@
 //   - weights come by 16-byte cp.async into a ring that is private to each warp: no block barrier and
 //     no dependence on what the L1 cache keeps
 //   - the decoded operand goes to tensor memory (tcgen05.st), not to shared memory: writing 32 KB a step
-//     there and having the MMAs read it back took 510 of the 1330 cycles of a step, and a proxy fence
+//     there and having the MMAs read it back takes 512 cycles of a step's shared-memory bandwidth, and a fence
 //   - a thread takes word t of the four groups of a step of its row: one AND-XOR and one fused half2
 //     multiply-add for two weights, the four sub-scales by the same trick.  The k order that results (the
 //     16 chunks of 8 values of a step transposed as 4 x 4, a chunk as 0 2 4 6 1 3 5 7) is the order in which
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(NT, 1) mmq_wide_k(const WArgs a, const __grid_
     tc_fence_after();
     const uint32_t tmem = s.tmem_base;
     // Bounded: half a second, then the error word, and from there on short waits.  A waiting warp sleeps between looks:
-    // polling took issue slots from the decode warps (512 experts of 128 rows: 508 -> 463 us).
+    // polling took issue slots from the decode warps (measured with sleeping waits that had no time limit: 512 experts of 128 rows, 508 -> 463 us under ncu).
     unsigned long long patience = 500000000ull;
     auto wait = [&](unsigned long long *bar, uint32_t parity, uint32_t code) {
         if (mbar_look(bar, parity)) return;
