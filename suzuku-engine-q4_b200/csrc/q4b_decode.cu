@@ -35,6 +35,7 @@ __global__ void quant8_k(const float *__restrict__ x, uint64_t xs, uint32_t gps,
                          uint64_t n_groups, int8_t *__restrict__ q, float *__restrict__ d,
                          int32_t *__restrict__ bs, uint64_t q_slice, uint64_t d_slice,
                          const int32_t *__restrict__ n_dev) {
+    q4b_pdl_wait();
     const uint64_t g = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (g >= n_groups) return;
     const uint32_t lane = threadIdx.x & 31u;
@@ -58,7 +59,7 @@ __global__ void quant8_k(const float *__restrict__ x, uint64_t xs, uint32_t gps,
 // ------------------------------------------------------------------ RMSNorm (+ Q8-A)
 // One block of 256 per (group, token) row.  The sum of squares is kept in
 // fp64 like the scalar reference (src/q4_quant.c:697-706).
-__global__ void rms_q8_k(const float *__restrict__ x, const float *__restrict__ w,
+__global__ void __launch_bounds__(256) rms_q8_k(const float *__restrict__ x, const float *__restrict__ w,
                          float *__restrict__ y, uint32_t n, uint32_t hc, float eps,
                          int8_t *__restrict__ q, float *__restrict__ d, int32_t *__restrict__ bs,
                          uint64_t q_slice, uint64_t d_slice) {
@@ -66,20 +67,33 @@ __global__ void rms_q8_k(const float *__restrict__ x, const float *__restrict__ 
     const uint64_t row = (uint64_t)tok * hc + c;
     const float *xc = x + row * n;
     const float *wc = w ? w + (uint64_t)c * n : nullptr;
+    q4b_pdl_wait();
+    // up to RMS_REG values and weights of a thread stay in registers: all loads in flight at once, x read once
+    constexpr uint32_t RMS_REG = 10;
+    float xr[RMS_REG], wr[RMS_REG];
+#pragma unroll
+    for (uint32_t j = 0; j < RMS_REG; j++) {
+        const uint32_t i = threadIdx.x + 256u * j;
+        xr[j] = i < n ? xc[i] : 0.f;
+        wr[j] = wc && i < n ? wc[i] : 1.f;
+    }
     double ss = 0.0;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) ss += (double)xc[i] * (double)xc[i];
+#pragma unroll
+    for (uint32_t j = 0; j < RMS_REG; j++) ss += (double)xr[j] * (double)xr[j];
+    for (uint32_t i = threadIdx.x + 256u * RMS_REG; i < n; i += 256u) ss += (double)xc[i] * (double)xc[i];
     __shared__ double sh[8];
 #pragma unroll
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((threadIdx.x & 31u) == 0) sh[threadIdx.x >> 5] = ss;
     __syncthreads();
     double tot = 0.0;
-    for (uint32_t i = 0; i < (blockDim.x >> 5); i++) tot += sh[i];
+#pragma unroll
+    for (uint32_t i = 0; i < 8u; i++) tot += sh[i];
     const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn((float)(tot / (double)n), eps)));
     const uint32_t lane = threadIdx.x & 31u;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        float v = __fmul_rn(xc[i], scale);
-        if (wc) v = __fmul_rn(v, wc[i]);
+    auto put = [&](uint32_t i, float xv, float wv) {
+        float v = __fmul_rn(xv, scale);
+        if (wc) v = __fmul_rn(v, wv);
         if (y) y[row * n + i] = v;
         if (q) {  // n % 32 == 0 and blockDim % 32 == 0: a warp holds one whole group
             const float a = q4b_warp_max(fabsf(v));
@@ -95,7 +109,11 @@ __global__ void rms_q8_k(const float *__restrict__ x, const float *__restrict__ 
                 bs[row * d_slice + (i >> 5)] = sum;
             }
         }
-    }
+    };
+#pragma unroll
+    for (uint32_t j = 0; j < RMS_REG; j++)
+        if (threadIdx.x + 256u * j < n) put(threadIdx.x + 256u * j, xr[j], wr[j]);
+    for (uint32_t i = threadIdx.x + 256u * RMS_REG; i < n; i += 256u) put(i, xc[i], wc ? wc[i] : 1.f);
 }
 
 // ------------------------------------------------------------------ hyper-connection streams
@@ -147,18 +165,23 @@ __global__ void __launch_bounds__(256) hc_streams_k(float *__restrict__ res, con
 }
 
 // ------------------------------------------------------------------ fp32 GEMV (router)
-// One warp per weight row; grid.y = batch.
-__global__ void gemv_f32_k(const float *__restrict__ W, uint64_t nrows, uint64_t ncols,
+// One warp per weight row, four a CTA (a router of 512 rows then covers 128 SMs); grid.y = batch.  The row is asked
+// into L2 before the wait for x.
+__global__ void __launch_bounds__(128) gemv_f32_k(const float *__restrict__ W, uint64_t nrows, uint64_t ncols,
                            const float *__restrict__ x, float *__restrict__ y, float scale) {
-    const uint64_t r = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (r >= nrows) return;
+    const uint64_t r = (uint64_t)blockIdx.x * 4u + (threadIdx.x >> 5);
     const uint32_t lane = threadIdx.x & 31u;
     const float *wr = W + r * ncols;
+    if (r < nrows && blockIdx.y == 0)
+        for (uint64_t i = lane * 32u; i < ncols; i += 1024u) q4b_l2_prefetch(wr + i);
+    q4b_pdl_wait();
+    if (r >= nrows) return;
     const float *xb = x + (uint64_t)blockIdx.y * ncols;
     float acc = 0.f;
     if ((ncols & 3u) == 0) {
         const float4 *w4 = reinterpret_cast<const float4 *>(wr);
         const float4 *x4 = reinterpret_cast<const float4 *>(xb);
+#pragma unroll 8
         for (uint64_t i = lane; i < ncols / 4; i += 32) {
             const float4 a = __ldg(w4 + i), b = x4[i];
             acc += a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
@@ -314,79 +337,83 @@ __global__ void iq3s_idot_k(const uint8_t *__restrict__ w, uint64_t nrows, uint3
 // values keep the lower index; weights renormalised over the picks in rank
 // order (src/q4_quant.c:715-755).  Optionally appends the shared expert's slot
 // with weight 1 and writes the entry count.
-__device__ __forceinline__ void softmax_topk_warp(const float *__restrict__ l, uint32_t n, uint32_t k,
-                                                  int32_t *__restrict__ ids, float *__restrict__ wts,
-                                                  int32_t shared_slot, int32_t *__restrict__ n_out,
-                                                  float *p, float *wsel, uint32_t lane) {
+// NPL: logits a lane holds in registers (n <= 32 NPL), logit i in lane i % 32.  A round is two warp reductions on
+// 32-bit keys; the lane that owned the pick looks through its registers for its next best.  (With the probabilities in
+// shared memory a round was five shuffles of 64-bit keys and a walk over them.)
+template <uint32_t NPL>
+__device__ __forceinline__ void softmax_topk_regs(const float *__restrict__ l, uint32_t n, uint32_t k,
+                                                  int32_t *__restrict__ ids, float *__restrict__ wts, int32_t shared_slot,
+                                                  int32_t *__restrict__ n_out, uint32_t lane) {
+    constexpr uint32_t full = 0xffffffffu;
+    float p[NPL];
     float m = -INFINITY;
-    for (uint32_t i = lane; i < n; i += 32) m = fmaxf(m, __ldcg(l + i));
+#pragma unroll
+    for (uint32_t j = 0; j < NPL; j++) {
+        p[j] = lane + 32u * j < n ? __ldcg(l + lane + 32u * j) : -INFINITY;
+        m = fmaxf(m, p[j]);
+    }
     m = q4b_warp_max(m);
     float s = 0.f;
-    for (uint32_t i = lane; i < n; i += 32) {
-        const float e = expf(__ldcg(l + i) - m);
-        p[i] = e;
-        s += e;
-    }
+#pragma unroll
+    for (uint32_t j = 0; j < NPL; j++)
+        if (lane + 32u * j < n) {
+            p[j] = expf(p[j] - m);
+            s += p[j];
+        }
     s = q4b_warp_sum(s);
     const float inv = s > 0.f ? __fdiv_rn(1.0f, s) : 0.f;
-    for (uint32_t i = lane; i < n; i += 32) p[i] = __fmul_rn(p[i], inv);
-    __syncwarp();
-    // key: value bits above, inverted index below -> max key = largest value,
-    // lowest index among equals.  p >= 0 so the bit pattern orders like the value.
-    auto scan = [&]() {
-        unsigned long long best = 0ull;
-        for (uint32_t i = lane; i < n; i += 32) {
-            const float v = p[i];
-            if (v < 0.f) continue;  // taken
-            const unsigned long long key =
-                ((unsigned long long)__float_as_uint(v) << 32) | (0xffffffffu - i);
-            best = key > best ? key : best;
-        }
-        return best;
-    };
-    unsigned long long mine = scan();
-    if (k > n) k = n;
-    for (uint32_t t = 0; t < k; t++) {
-        unsigned long long best = mine;
+    // key: the bits of the probability plus one (it is not negative, so they order like the value); 0 = taken or none
+    uint32_t key[NPL], best = 0u, at = full;
 #pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-            best = other > best ? other : best;
+    for (uint32_t j = 0; j < NPL; j++) {
+        key[j] = lane + 32u * j < n ? __float_as_uint(__fmul_rn(p[j], inv)) + 1u : 0u;
+        if (key[j] > best) best = key[j], at = lane + 32u * j;   // the lower index among equals
+    }
+    if (k > n) k = n;
+    float sum = 0.f, v0 = 0.f, v1 = 0.f;
+    int32_t i0 = 0, i1 = 0;
+    for (uint32_t t = 0; t < k; t++) {
+        const uint32_t top = __reduce_max_sync(full, best);
+        const uint32_t idx = __reduce_min_sync(full, best == top ? at : full);
+        const float v = __uint_as_float(top - 1u);
+        sum = __fadd_rn(sum, v);
+        if (lane == (t & 31u)) {
+            if (t < 32u) v0 = v, i0 = (int32_t)idx;
+            else v1 = v, i1 = (int32_t)idx;
         }
-        const uint32_t idx = 0xffffffffu - (uint32_t)(best & 0xffffffffu);
-        if (lane == 0) {
-            ids[t] = (int32_t)idx;
-            wsel[t] = __uint_as_float((uint32_t)(best >> 32));
-        }
-        if ((idx & 31u) == lane) {
-            p[idx] = -1.f;
-            mine = scan();
+        if (idx == at) {
+            best = 0u, at = full;
+#pragma unroll
+            for (uint32_t j = 0; j < NPL; j++) {
+                if (lane + 32u * j == idx) key[j] = 0u;
+                if (key[j] > best) best = key[j], at = lane + 32u * j;
+            }
         }
     }
-    __syncwarp();
+    const float wi = sum > 0.f ? __fdiv_rn(1.0f, sum) : 1.f;
+    if (lane < k) ids[lane] = i0, wts[lane] = sum > 0.f ? __fmul_rn(v0, wi) : v0;
+    if (lane + 32u < k) ids[lane + 32u] = i1, wts[lane + 32u] = sum > 0.f ? __fmul_rn(v1, wi) : v1;
     if (lane == 0) {
-        float sum = 0.f;
-        for (uint32_t t = 0; t < k; t++) sum = __fadd_rn(sum, wsel[t]);
-        const float wi = sum > 0.f ? __fdiv_rn(1.0f, sum) : 1.f;
-        for (uint32_t t = 0; t < k; t++) wts[t] = sum > 0.f ? __fmul_rn(wsel[t], wi) : wsel[t];
-        uint32_t cnt = k;
-        if (shared_slot >= 0) {
-            ids[k] = shared_slot;
-            wts[k] = 1.0f;
-            cnt++;
-        }
-        if (n_out) *n_out = (int32_t)cnt;
+        if (shared_slot >= 0) ids[k] = shared_slot, wts[k] = 1.0f;
+        if (n_out) *n_out = (int32_t)(k + (shared_slot >= 0 ? 1u : 0u));
     }
 }
-__global__ void softmax_topk_k(const float *__restrict__ logits, uint32_t n, uint32_t k,
-                               int32_t *__restrict__ ids, float *__restrict__ wts,
-                               uint32_t out_stride, int32_t shared_slot,
-                               int32_t *__restrict__ n_out) {
-    __shared__ float p[1024];
-    __shared__ float wsel[64];
-    softmax_topk_warp(logits + (uint64_t)blockIdx.x * n, n, k, ids + (uint64_t)blockIdx.x * out_stride,
-                      wts + (uint64_t)blockIdx.x * out_stride, shared_slot, n_out ? n_out + blockIdx.x : nullptr, p,
-                      wsel, threadIdx.x);
+__device__ __forceinline__ void softmax_topk_warp(const float *__restrict__ l, uint32_t n, uint32_t k,
+                                                  int32_t *__restrict__ ids, float *__restrict__ wts, int32_t shared_slot,
+                                                  int32_t *__restrict__ n_out, uint32_t lane) {
+    if (n <= 512u) softmax_topk_regs<16>(l, n, k, ids, wts, shared_slot, n_out, lane);
+    else softmax_topk_regs<32>(l, n, k, ids, wts, shared_slot, n_out, lane);
+}
+// A warp per token.
+__global__ void __launch_bounds__(128) softmax_topk_k(const float *__restrict__ logits, uint32_t n, uint32_t k,
+                                                      int32_t *__restrict__ ids, float *__restrict__ wts,
+                                                      uint32_t out_stride, int32_t shared_slot,
+                                                      int32_t *__restrict__ n_out, uint32_t n_tok) {
+    q4b_pdl_wait();
+    const uint64_t t = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (t >= n_tok) return;
+    softmax_topk_warp(logits + t * n, n, k, ids + t * out_stride, wts + t * out_stride, shared_slot,
+                      n_out ? n_out + t : nullptr, threadIdx.x & 31u);
 }
 
 // RMSNorm, router product and softmax / top-k of a batch of tokens in ONE launch (n_embd == 2048): what
@@ -401,12 +428,14 @@ __global__ void __launch_bounds__(256) route_small_k(const float *__restrict__ x
                                                      uint32_t n_tok, uint32_t topk, float *__restrict__ xn_out,
                                                      float *__restrict__ logits, int32_t *__restrict__ ids,
                                                      float *__restrict__ wts, unsigned int *__restrict__ counters) {
-    extern __shared__ __align__(16) float rs_rows[];   // [8][2048]; the last CTA reuses it for the probabilities
-    __shared__ float wsel[8][64];
+    extern __shared__ __align__(16) float rs_rows[];   // [8][2048]
     __shared__ uint32_t is_last;
     constexpr uint32_t n = 2048;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t t0 = blockIdx.y * 8u, nt = min(8u, n_tok - t0);
+    if (blockIdx.x * 8u + warp < n_expert)   // this warp's router row, into L2 before the wait
+        for (uint32_t i = lane * 32u; i < n; i += 1024u) q4b_l2_prefetch(W + (uint64_t)(blockIdx.x * 8u + warp) * n + i);
+    q4b_pdl_wait();
     if (warp < nt) {
         const float4 *x4 = reinterpret_cast<const float4 *>(x + (uint64_t)(t0 + warp) * n);
         float4 v[16];
@@ -464,11 +493,11 @@ __global__ void __launch_bounds__(256) route_small_k(const float *__restrict__ x
     __threadfence();
     if (warp < nt)
         softmax_topk_warp(logits + (uint64_t)(t0 + warp) * n_expert, n_expert, topk, ids + (uint64_t)(t0 + warp) * topk,
-                          wts + (uint64_t)(t0 + warp) * topk, -1, nullptr, rs_rows + warp * 1024u, wsel[warp], lane);
+                          wts + (uint64_t)(t0 + warp) * topk, -1, nullptr, lane);
 }
 
 // ------------------------------------------------------------------ gate/up + SwiGLU
-// grid (n_ff/8, experts), 8 warps per block, one warp per hidden unit f:
+// grid (n_ff/8, experts or fewer), 8 warps per block, one warp per hidden unit f, experts in strides of grid.y:
 // h[e][f] = silu(gate_f . xq) * (up_f . xq).
 template <bool TILED>
 __global__ void moe_gu_k(const uint8_t *__restrict__ bg, const uint8_t *__restrict__ bu,
@@ -482,9 +511,10 @@ __global__ void moe_gu_k(const uint8_t *__restrict__ bg, const uint8_t *__restri
     const uint32_t ng = in_dim >> 5;
     float *sd = reinterpret_cast<float *>(smem + 2048 + in_dim);
     int *sb = reinterpret_cast<int *>(smem + 2048 + in_dim + 4 * ng);
-    const uint32_t e = blockIdx.y;
-    if (n_dev && e >= (uint32_t)*n_dev) return;
     q4b_fill_code_table(tab);
+    q4b_pdl_wait();
+    const uint32_t n = n_dev ? (uint32_t)*n_dev : gridDim.y;
+    if (blockIdx.y >= n) return;
     for (uint32_t i = threadIdx.x; i < in_dim / 4; i += blockDim.x)
         sq[i] = reinterpret_cast<const int *>(xq)[i];
     for (uint32_t i = threadIdx.x; i < ng; i += blockDim.x) {
@@ -496,27 +526,30 @@ __global__ void moe_gu_k(const uint8_t *__restrict__ bg, const uint8_t *__restri
     if (f >= n_ff) return;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t nbr = in_dim >> 8;  // super-blocks per row
-    const uint8_t *wg = bg + (uint64_t)slots[e] * stride, *wu = bu + (uint64_t)slots[e] * stride;
-    float ag = 0.f, au = 0.f;
-    for (uint32_t g = lane; g < ng; g += 32) {
-        const uint64_t bi = (uint64_t)f * nbr + (g >> 3);
-        const int *qv = sq + g * 8u;
-        const float dx = sd[g];
-        const int qsum = sb[g];
-        {
-            const Iq3Fields fg = iq3_fields<TILED>(wg, bi, g & 7u);
-            const int I = iq3_idot<TILED>(fg, tab, qv, qsum);
-            ag = fmaf(__fmul_rn(fg.d, dx), (float)(I * (int)fg.ls), ag);
+    for (uint32_t e = blockIdx.y; e < n; e += gridDim.y) {
+        const uint8_t *wg = bg + (uint64_t)slots[e] * stride, *wu = bu + (uint64_t)slots[e] * stride;
+        float ag = 0.f, au = 0.f;
+#pragma unroll 2
+        for (uint32_t g = lane; g < ng; g += 32) {
+            const uint64_t bi = (uint64_t)f * nbr + (g >> 3);
+            const int *qv = sq + g * 8u;
+            const float dx = sd[g];
+            const int qsum = sb[g];
+            {
+                const Iq3Fields fg = iq3_fields<TILED>(wg, bi, g & 7u);
+                const int I = iq3_idot<TILED>(fg, tab, qv, qsum);
+                ag = fmaf(__fmul_rn(fg.d, dx), (float)(I * (int)fg.ls), ag);
+            }
+            {
+                const Iq3Fields fg = iq3_fields<TILED>(wu, bi, g & 7u);
+                const int I = iq3_idot<TILED>(fg, tab, qv, qsum);
+                au = fmaf(__fmul_rn(fg.d, dx), (float)(I * (int)fg.ls), au);
+            }
         }
-        {
-            const Iq3Fields fg = iq3_fields<TILED>(wu, bi, g & 7u);
-            const int I = iq3_idot<TILED>(fg, tab, qv, qsum);
-            au = fmaf(__fmul_rn(fg.d, dx), (float)(I * (int)fg.ls), au);
-        }
+        ag = q4b_warp_sum(ag);
+        au = q4b_warp_sum(au);
+        if (lane == 0) h[(uint64_t)e * n_ff + f] = q4b_swiglu(ag, au);
     }
-    ag = q4b_warp_sum(ag);
-    au = q4b_warp_sum(au);
-    if (lane == 0) h[(uint64_t)e * n_ff + f] = q4b_swiglu(ag, au);
 }
 
 // ------------------------------------------------------------------ down + weighted combine
@@ -533,6 +566,7 @@ __global__ void moe_ya_k(const uint8_t *__restrict__ bd, uint64_t stride,
     __shared__ uint32_t tab[512];
     q4b_fill_code_table(tab);
     __syncthreads();
+    q4b_pdl_wait();
     const uint32_t r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= n_embd) return;
     const uint32_t lane = threadIdx.x & 31u;
@@ -540,6 +574,7 @@ __global__ void moe_ya_k(const uint8_t *__restrict__ bd, uint64_t stride,
     const uint32_t ng = n_ff >> 5;
     const uint32_t nbr = n_ff >> 8;
     float acc = 0.f;
+#pragma unroll 4   // several items' loads in flight: a trip is a chain of three
     for (uint32_t it = lane; it < n * ng; it += 32) {
         const uint32_t e = it / ng, g = it - e * ng;
         const Iq3Fields fg = iq3_fields<TILED>(bd + (uint64_t)slots[e] * stride,
@@ -648,30 +683,32 @@ __global__ void moe_gu4_k(const uint8_t *__restrict__ bg, const uint8_t *__restr
     __shared__ uint16_t pair[256];
     iq4_fill_pair_table(pair);
     __syncthreads();
-    const uint32_t e = blockIdx.y;
-    if (n_dev && e >= (uint32_t)*n_dev) return;
+    q4b_pdl_wait();
     const uint32_t f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (f >= n_ff) return;
-    const uint32_t lane = threadIdx.x & 31u, ng = in_dim >> 5;
+    const uint32_t lane = threadIdx.x & 31u, ng = in_dim >> 5, n = n_dev ? (uint32_t)*n_dev : gridDim.y;
     const uint64_t rb = iq4_row_bytes(T, in_dim);
-    const uint8_t *rg = bg + (uint64_t)slots[e] * stride + (uint64_t)f * rb;
-    const uint8_t *ru = bu + (uint64_t)slots[e] * stride + (uint64_t)f * rb;
-    float ag = 0.f, au = 0.f;
-    for (uint32_t g = lane; g < ng; g += 32) {
-        int qv[8];
+    for (uint32_t e = blockIdx.y; e < n; e += gridDim.y) {
+        const uint8_t *rg = bg + (uint64_t)slots[e] * stride + (uint64_t)f * rb;
+        const uint8_t *ru = bu + (uint64_t)slots[e] * stride + (uint64_t)f * rb;
+        float ag = 0.f, au = 0.f;
+#pragma unroll 2
+        for (uint32_t g = lane; g < ng; g += 32) {
+            int qv[8];
 #pragma unroll
-        for (int k = 0; k < 8; k++) qv[k] = reinterpret_cast<const int *>(xq)[g * 8u + k];
-        const float dx = xd[g];
-        int lsf;
-        float d;
-        const uint8_t *cg = iq4_group<T>(rg, g, &lsf, &d);
-        ag = fmaf(__fmul_rn(d, dx), (float)(iq4_codes_idot(cg, pair, qv) * lsf), ag);
-        const uint8_t *cu = iq4_group<T>(ru, g, &lsf, &d);
-        au = fmaf(__fmul_rn(d, dx), (float)(iq4_codes_idot(cu, pair, qv) * lsf), au);
+            for (int k = 0; k < 8; k++) qv[k] = reinterpret_cast<const int *>(xq)[g * 8u + k];
+            const float dx = xd[g];
+            int lsf;
+            float d;
+            const uint8_t *cg = iq4_group<T>(rg, g, &lsf, &d);
+            ag = fmaf(__fmul_rn(d, dx), (float)(iq4_codes_idot(cg, pair, qv) * lsf), ag);
+            const uint8_t *cu = iq4_group<T>(ru, g, &lsf, &d);
+            au = fmaf(__fmul_rn(d, dx), (float)(iq4_codes_idot(cu, pair, qv) * lsf), au);
+        }
+        ag = q4b_warp_sum(ag);
+        au = q4b_warp_sum(au);
+        if (lane == 0) h[(uint64_t)e * n_ff + f] = q4b_swiglu(ag, au);
     }
-    ag = q4b_warp_sum(ag);
-    au = q4b_warp_sum(au);
-    if (lane == 0) h[(uint64_t)e * n_ff + f] = q4b_swiglu(ag, au);
 }
 
 // Down projection with rows of type T: the counterpart of moe_ya_k (same reduction shape).
@@ -683,6 +720,7 @@ __global__ void moe_ya4_k(const uint8_t *__restrict__ bd, uint64_t stride, const
     __shared__ uint16_t pair[256];
     iq4_fill_pair_table(pair);
     __syncthreads();
+    q4b_pdl_wait();
     const uint32_t r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= n_embd) return;
     const uint32_t lane = threadIdx.x & 31u;
@@ -690,6 +728,7 @@ __global__ void moe_ya4_k(const uint8_t *__restrict__ bd, uint64_t stride, const
     const uint32_t ng = n_ff >> 5;
     const uint64_t rb = iq4_row_bytes(T, n_ff);
     float acc = 0.f;
+#pragma unroll 4   // several items' loads in flight: a trip is a chain of three
     for (uint32_t it = lane; it < n * ng; it += 32) {
         const uint32_t e = it / ng, g = it - e * ng;
         const int *qg = reinterpret_cast<const int *>(hq + (uint64_t)e * q_slice) + g * 8u;
@@ -779,8 +818,7 @@ bool launch_quant8(const float *x, uint64_t xs, uint32_t slen, uint32_t ns, int8
                    int32_t *bs, uint64_t q_slice, uint64_t d_slice, const int32_t *n_dev) {
     const uint32_t gps = slen >> 5;
     const uint64_t ngr = (uint64_t)gps * ns;
-    quant8_k<<<(unsigned)((ngr + 7) / 8), 256, 0, g_q4b.stream>>>(x, xs, gps, ngr, q, d, bs,
-                                                                 q_slice, d_slice, n_dev);
+    q4b_launch(quant8_k, (unsigned)((ngr + 7) / 8), 256, 0, g_q4b.stream, x, xs, gps, ngr, q, d, bs, q_slice, d_slice, n_dev);
     g_q4b_launches++;
     return q4b_launch_ok("quant8");
 }
@@ -799,48 +837,44 @@ bool moe_exec_tail(const uint8_t *base, uint64_t stride, const int32_t *d_slots,
     const int32_t *xbs = s.xbs + (size_t)Q4B_X_SLICE * (Q4B_XQ_MAXLEN / 32);
     const size_t sm = 2048 + in_dim + 8 * (in_dim >> 5);
     const bool tiled = q4b_ptr_tiled(base);
+    // a count on the device: the grid is cut for 16 experts, more are walked in strides of it
+    const dim3 gg((n_ff + 7) / 8, d_n ? 16u : n_host);
     if (gt == Q4_T_IQ3_XXS)
-        moe_gux_k<Q4_T_IQ3_XXS><<<dim3((n_ff + 7) / 8, ne), 256, 0, s.stream>>>(
-            base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff, s.grid3xxs_d, s.grid2s_d, d_h);
+        q4b_launch(moe_gux_k<Q4_T_IQ3_XXS>, gg, 256, 0, s.stream, base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff,
+                   s.grid3xxs_d, s.grid2s_d, d_h);
     else if (gt == Q4_T_IQ2_S)
-        moe_gux_k<Q4_T_IQ2_S><<<dim3((n_ff + 7) / 8, ne), 256, 0, s.stream>>>(
-            base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff, s.grid3xxs_d, s.grid2s_d, d_h);
+        q4b_launch(moe_gux_k<Q4_T_IQ2_S>, gg, 256, 0, s.stream, base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff,
+                   s.grid3xxs_d, s.grid2s_d, d_h);
     else if (gt == Q4_T_IQ4_NL)
-        moe_gu4_k<Q4_T_IQ4_NL><<<dim3((n_ff + 7) / 8, ne), 256, 0, s.stream>>>(
-            base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff, d_h);
+        q4b_launch(moe_gu4_k<Q4_T_IQ4_NL>, gg, 256, 0, s.stream, base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff, d_h);
     else if (gt == Q4_T_IQ4_XS)
-        moe_gu4_k<Q4_T_IQ4_XS><<<dim3((n_ff + 7) / 8, ne), 256, 0, s.stream>>>(
-            base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff, d_h);
+        q4b_launch(moe_gu4_k<Q4_T_IQ4_XS>, gg, 256, 0, s.stream, base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff, d_h);
     else if (tiled)
-        moe_gu_k<true><<<dim3((n_ff + 7) / 8, ne), 256, sm, s.stream>>>(
-            base + og, base + ou, stride, d_slots, d_n, xq, xd, xbs, in_dim, n_ff, d_h);
+        q4b_launch(moe_gu_k<true>, gg, 256, sm, s.stream, base + og, base + ou, stride, d_slots, d_n, xq, xd, xbs, in_dim, n_ff, d_h);
     else
-        moe_gu_k<false><<<dim3((n_ff + 7) / 8, ne), 256, sm, s.stream>>>(
-            base + og, base + ou, stride, d_slots, d_n, xq, xd, xbs, in_dim, n_ff, d_h);
+        q4b_launch(moe_gu_k<false>, gg, 256, sm, s.stream, base + og, base + ou, stride, d_slots, d_n, xq, xd, xbs, in_dim, n_ff, d_h);
     g_q4b_launches++;
     if (!q4b_launch_ok("moe_gu")) return false;
     if (!launch_quant8(d_h, n_ff, n_ff, ne, s.xq, s.xd, s.xbs, Q4B_XQ_MAXLEN, Q4B_XQ_MAXLEN / 32,
                        d_n))
         return false;
+    const unsigned gy = (n_embd + 7) / 8;
+    const uint64_t qsl = Q4B_XQ_MAXLEN, dsl = Q4B_XQ_MAXLEN / 32;
     if (dt == Q4_T_Q2_0)
-        moe_ya20_k<<<(n_embd + 7) / 8, 256, 0, s.stream>>>(base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd,
-                                                          s.xbs, Q4B_XQ_MAXLEN, Q4B_XQ_MAXLEN / 32, n_ff, n_embd, d_y);
+        q4b_launch(moe_ya20_k, gy, 256, 0, s.stream, base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, s.xbs, qsl, dsl, n_ff,
+                   n_embd, d_y);
     else if (dt == Q4_T_IQ4_NL)
-        moe_ya4_k<Q4_T_IQ4_NL><<<(n_embd + 7) / 8, 256, 0, s.stream>>>(
-            base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, Q4B_XQ_MAXLEN, Q4B_XQ_MAXLEN / 32, n_ff,
-            n_embd, d_y);
+        q4b_launch(moe_ya4_k<Q4_T_IQ4_NL>, gy, 256, 0, s.stream, base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, qsl, dsl,
+                   n_ff, n_embd, d_y);
     else if (dt == Q4_T_IQ4_XS)
-        moe_ya4_k<Q4_T_IQ4_XS><<<(n_embd + 7) / 8, 256, 0, s.stream>>>(
-            base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, Q4B_XQ_MAXLEN, Q4B_XQ_MAXLEN / 32, n_ff,
-            n_embd, d_y);
+        q4b_launch(moe_ya4_k<Q4_T_IQ4_XS>, gy, 256, 0, s.stream, base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, qsl, dsl,
+                   n_ff, n_embd, d_y);
     else if (tiled)
-        moe_ya_k<true><<<(n_embd + 7) / 8, 256, 0, s.stream>>>(
-            base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, s.xbs, Q4B_XQ_MAXLEN,
-            Q4B_XQ_MAXLEN / 32, n_ff, n_embd, d_y);
+        q4b_launch(moe_ya_k<true>, gy, 256, 0, s.stream, base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, s.xbs, qsl, dsl,
+                   n_ff, n_embd, d_y);
     else
-        moe_ya_k<false><<<(n_embd + 7) / 8, 256, 0, s.stream>>>(
-            base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, s.xbs, Q4B_XQ_MAXLEN,
-            Q4B_XQ_MAXLEN / 32, n_ff, n_embd, d_y);
+        q4b_launch(moe_ya_k<false>, gy, 256, 0, s.stream, base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, s.xbs, qsl, dsl,
+                   n_ff, n_embd, d_y);
     g_q4b_launches++;
     return q4b_launch_ok("moe_ya");
 }
@@ -925,7 +959,7 @@ extern "C" bool q4_hip_softmax_topk_launch(const float *d_logits, uint32_t n, ui
                                            int32_t *d_ids, float *d_wts) {
     if (!g_q4b.ok || !d_logits || !d_ids || !d_wts || n == 0 || n > 1024 || k == 0 || k > 64)
         return false;
-    softmax_topk_k<<<1, 32, 0, g_q4b.stream>>>(d_logits, n, k, d_ids, d_wts, k, -1, nullptr);
+    q4b_launch(softmax_topk_k, 1, 32, 0, g_q4b.stream, d_logits, n, k, d_ids, d_wts, k, -1, nullptr, 1u);
     g_q4b_launches++;
     return q4b_launch_ok("softmax_topk");
 }
@@ -947,8 +981,7 @@ extern "C" bool q4_hip_softmax_topk(const float *d_logits, uint32_t n, uint32_t 
 extern "C" bool q4_hip_grouped_rms_n(const float *x, const float *w, float *y, uint32_t n_embd,
                                      uint32_t hc, float eps, uint32_t n_tok) {
     if (!g_q4b.ok || !x || !y || n_embd == 0 || hc == 0 || n_tok == 0) return false;
-    rms_q8_k<<<dim3(hc, n_tok), 256, 0, g_q4b.stream>>>(x, w, y, n_embd, hc, eps, nullptr, nullptr,
-                                                       nullptr, 0, 0);
+    q4b_launch(rms_q8_k, dim3(hc, n_tok), 256, 0, g_q4b.stream, x, w, y, n_embd, hc, eps, nullptr, nullptr, nullptr, 0, 0);
     g_q4b_launches++;
     return q4b_launch_ok("grouped_rms");
 }
@@ -1001,8 +1034,8 @@ extern "C" bool q4_hip_gemv_dd_n(uint32_t ggml_type, const uint8_t *d_w, uint64_
         gemv_f32_x16_k<<<dim3((unsigned)((nrows + 7) / 8), (n_batch + 15) / 16), 256, 0, g_q4b.stream>>>(
             reinterpret_cast<const float *>(d_w), nrows, d_x, n_batch, d_y, scale);
     } else if (ggml_type == Q4_T_F32) {
-        gemv_f32_k<<<grid, 256, 0, g_q4b.stream>>>(reinterpret_cast<const float *>(d_w), nrows,
-                                                  ncols, d_x, d_y, scale);
+        q4b_launch(gemv_f32_k, dim3((unsigned)((nrows + 3) / 4), n_batch), 128, 0, g_q4b.stream,
+                   reinterpret_cast<const float *>(d_w), nrows, ncols, d_x, d_y, scale);
     } else if (ggml_type == Q4_T_IQ3_S) {
         if (ncols % Q4B_QK) return false;
         if (q4b_ptr_tiled(d_w))
@@ -1152,16 +1185,13 @@ extern "C" bool q4_cuda_moe_decode(const uint8_t *base, uint64_t stride, uint64_
     int8_t *xq = s.xq + (size_t)Q4B_X_SLICE * Q4B_XQ_MAXLEN;
     float *xd = s.xd + (size_t)Q4B_X_SLICE * (Q4B_XQ_MAXLEN / 32);
     int32_t *xbs = s.xbs + (size_t)Q4B_X_SLICE * (Q4B_XQ_MAXLEN / 32);
-    rms_q8_k<<<dim3(1, 1), 256, 0, s.stream>>>(d_x, d_norm_w, s.xn, n_embd, 1, eps, xq, xd, xbs, 0,
-                                              0);
+    q4b_launch(rms_q8_k, 1, 256, 0, s.stream, d_x, d_norm_w, s.xn, n_embd, 1, eps, xq, xd, xbs, 0, 0);
     g_q4b_launches++;
     if (!q4b_launch_ok("rms_q8")) return false;
-    gemv_f32_k<<<dim3((n_expert + 7) / 8, 1), 256, 0, s.stream>>>(d_router, n_expert, n_embd, s.xn,
-                                                                 s.logits, 1.0f);
+    q4b_launch(gemv_f32_k, (n_expert + 3) / 4, 128, 0, s.stream, d_router, n_expert, n_embd, s.xn, s.logits, 1.0f);
     g_q4b_launches++;
     if (!q4b_launch_ok("router_gemv")) return false;
-    softmax_topk_k<<<1, 32, 0, s.stream>>>(s.logits, n_expert, topk, s.r_ids, s.r_wts, 64,
-                                          shared_slot, s.r_cnt);
+    q4b_launch(softmax_topk_k, 1, 32, 0, s.stream, s.logits, n_expert, topk, s.r_ids, s.r_wts, 64u, shared_slot, s.r_cnt, 1u);
     g_q4b_launches++;
     if (!q4b_launch_ok("softmax_topk")) return false;
     if (cudaMemsetAsync(d_y, 0, (size_t)n_embd * sizeof(float), s.stream) != cudaSuccess)
@@ -1278,7 +1308,9 @@ extern "C" bool q4_cuda_decode_plan_host(void *plan, const float *h_x, float *h_
 // ---- helpers shared with the many-token path (q4b_grouped.cu) ----
 bool q4b_route_tokens(const float *d_rlog, int32_t *d_ids, float *d_wts, uint32_t n_tok,
                       uint32_t n_exp, uint32_t topk) {
-    softmax_topk_k<<<n_tok, 32, 0, g_q4b.stream>>>(d_rlog, n_exp, topk, d_ids, d_wts, topk, -1, nullptr);
+    const uint32_t w = n_tok < 4u ? n_tok : 4u;   // tokens a CTA
+    q4b_launch(softmax_topk_k, (n_tok + w - 1u) / w, 32u * w, 0, g_q4b.stream, d_rlog, n_exp, topk, d_ids, d_wts, topk, -1,
+               nullptr, n_tok);
     g_q4b_launches++;
     return q4b_launch_ok("route_tokens");
 }
@@ -1305,15 +1337,14 @@ bool q4b_route_small(const float *x, const float *norm_w, float eps, const float
     if (!g_route_counter || n_embd != 2048u || n_tok == 0 || n_tok > ROUTE_MAX_TOK || n_expert > 1024u ||
         topk > 64u || (((uintptr_t)router | (uintptr_t)x | (uintptr_t)norm_w | (uintptr_t)xn) & 15u))
         return false;
-    route_small_k<<<dim3((n_expert + 7u) / 8u, (n_tok + 7u) / 8u), 256, 8u * 2048u * 4u, g_q4b.stream>>>(
+    q4b_launch(route_small_k, dim3((n_expert + 7u) / 8u, (n_tok + 7u) / 8u), 256, 8u * 2048u * 4u, g_q4b.stream,
         x, norm_w, eps, router, n_expert, n_tok, topk, xn, logits, ids, wts, g_route_counter);
     g_q4b_launches++;
     return q4b_launch_ok("route_small");
 }
 bool q4b_rms_rows(const float *x, const float *w, float *y, uint32_t n_embd, float eps,
                   uint32_t n_tok) {
-    rms_q8_k<<<dim3(1, n_tok), 256, 0, g_q4b.stream>>>(x, w, y, n_embd, 1, eps, nullptr, nullptr,
-                                                      nullptr, 0, 0);
+    q4b_launch(rms_q8_k, dim3(1, n_tok), 256, 0, g_q4b.stream, x, w, y, n_embd, 1, eps, nullptr, nullptr, nullptr, 0, 0);
     g_q4b_launches++;
     return q4b_launch_ok("rms_rows");
 }

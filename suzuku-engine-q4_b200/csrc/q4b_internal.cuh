@@ -79,6 +79,32 @@ static inline bool q4b_launch_ok(const char *what) {
 
 #ifdef __CUDACC__
 
+// Launches that may start before the kernel ahead of them in the stream has ended (programmatic dependent launch):
+// the CTAs come up, and wait inside the kernel (q4b_pdl_wait) until that kernel is complete and its writes are
+// visible.  What is saved is the drain and the launch between two kernels of a chain, 1 to 1.5 us each.  Every
+// kernel launched this way calls q4b_pdl_wait in every thread before it reads or writes anything another kernel may
+// touch (prefetches into L2 may come before it), so completion stays transitive along the stream.
+template <typename... KA, typename... A>
+static inline void q4b_launch(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...);   // the caller checks q4b_launch_ok
+}
+// Lets the next kernel of the chain come up as soon as every CTA of this one is running, then waits for the one before.
+__device__ __forceinline__ void q4b_pdl_wait() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void q4b_l2_prefetch(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // The 512-entry codebook as packed 12-bit codes (four 3-bit codes per entry).
 // The library is compiled as ONE translation unit (q4cuda.cu includes every
 // other .cu), so this definition exists once.

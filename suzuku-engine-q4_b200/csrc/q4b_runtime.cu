@@ -391,6 +391,7 @@ extern "C" uint64_t q4_hip_vram_free(void) {
 }
 
 __global__ static void fill_k(float *d, float v, uint64_t n) {
+    q4b_pdl_wait();
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
     for (; i < n; i += step) d[i] = v;
@@ -399,7 +400,7 @@ extern "C" bool q4_hip_fill(float *d, float v, uint64_t n) {
     if (!g_q4b.ok || !d || n == 0) return false;
     uint64_t nb = (n + 255) / 256;
     if (nb > 4096) nb = 4096;
-    fill_k<<<(unsigned)nb, 256, 0, g_q4b.stream>>>(d, v, n);
+    q4b_launch(fill_k, (unsigned)nb, 256, 0, g_q4b.stream, d, v, n);
     g_q4b_launches++;
     return q4b_launch_ok("fill");
 }

@@ -174,33 +174,35 @@ __global__ void moe_gux_k(const uint8_t *__restrict__ bg, const uint8_t *__restr
                           const int8_t *__restrict__ xq, const float *__restrict__ xd, uint32_t in_dim,
                           uint32_t n_ff, const uint32_t *__restrict__ grid3, const uint2 *__restrict__ grid2,
                           float *__restrict__ h) {
-    const uint32_t e = blockIdx.y;
-    if (n_dev && e >= (uint32_t)*n_dev) return;
+    q4b_pdl_wait();
     const uint32_t f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (f >= n_ff) return;
-    const uint32_t lane = threadIdx.x & 31u, ng = in_dim >> 5;
+    const uint32_t lane = threadIdx.x & 31u, ng = in_dim >> 5, n = n_dev ? (uint32_t)*n_dev : gridDim.y;
     const uint64_t rb = small_row_bytes(T, in_dim);
-    const uint8_t *rg = bg + (uint64_t)slots[e] * stride + (uint64_t)f * rb;
-    const uint8_t *ru = bu + (uint64_t)slots[e] * stride + (uint64_t)f * rb;
-    const float unit = T == Q4_T_IQ3_XXS ? 0.25f : 0.125f;
-    float ag = 0.f, au = 0.f;
-    for (uint32_t g = lane; g < ng; g += 32) {
-        int qv[8];
+    for (uint32_t e = blockIdx.y; e < n; e += gridDim.y) {
+        const uint8_t *rg = bg + (uint64_t)slots[e] * stride + (uint64_t)f * rb;
+        const uint8_t *ru = bu + (uint64_t)slots[e] * stride + (uint64_t)f * rb;
+        const float unit = T == Q4_T_IQ3_XXS ? 0.25f : 0.125f;
+        float ag = 0.f, au = 0.f;
+#pragma unroll 2
+        for (uint32_t g = lane; g < ng; g += 32) {
+            int qv[8];
 #pragma unroll
-        for (int k = 0; k < 8; k++) qv[k] = reinterpret_cast<const int *>(xq)[g * 8u + k];
-        const float dx = xd[g];
-        SmallGroup G;
-        int lo, hi;
-        small_group<T>(rg, g, grid3, grid2, G);
-        small_group_isums(G, qv, &lo, &hi);
-        ag = fmaf(__fmul_rn(__fmul_rn(G.d, unit), dx), (float)(lo * G.ls0 + hi * G.ls1), ag);
-        small_group<T>(ru, g, grid3, grid2, G);
-        small_group_isums(G, qv, &lo, &hi);
-        au = fmaf(__fmul_rn(__fmul_rn(G.d, unit), dx), (float)(lo * G.ls0 + hi * G.ls1), au);
+            for (int k = 0; k < 8; k++) qv[k] = reinterpret_cast<const int *>(xq)[g * 8u + k];
+            const float dx = xd[g];
+            SmallGroup G;
+            int lo, hi;
+            small_group<T>(rg, g, grid3, grid2, G);
+            small_group_isums(G, qv, &lo, &hi);
+            ag = fmaf(__fmul_rn(__fmul_rn(G.d, unit), dx), (float)(lo * G.ls0 + hi * G.ls1), ag);
+            small_group<T>(ru, g, grid3, grid2, G);
+            small_group_isums(G, qv, &lo, &hi);
+            au = fmaf(__fmul_rn(__fmul_rn(G.d, unit), dx), (float)(lo * G.ls0 + hi * G.ls1), au);
+        }
+        ag = q4b_warp_sum(ag);
+        au = q4b_warp_sum(au);
+        if (lane == 0) h[(uint64_t)e * n_ff + f] = q4b_swiglu(ag, au);
     }
-    ag = q4b_warp_sum(ag);
-    au = q4b_warp_sum(au);
-    if (lane == 0) h[(uint64_t)e * n_ff + f] = q4b_swiglu(ag, au);
 }
 
 // ---- down projection with Q2_0 rows: the counterpart of moe_ya_k (same reduction shape) ----
@@ -209,6 +211,7 @@ __global__ void moe_ya20_k(const uint8_t *__restrict__ bd, uint64_t stride, cons
                            const int8_t *__restrict__ hq, const float *__restrict__ hd,
                            const int32_t *__restrict__ hbs, uint64_t q_slice, uint64_t d_slice, uint32_t n_ff,
                            uint32_t n_embd, float *__restrict__ y) {
+    q4b_pdl_wait();
     const uint32_t r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= n_embd) return;
     const uint32_t lane = threadIdx.x & 31u;
@@ -216,6 +219,7 @@ __global__ void moe_ya20_k(const uint8_t *__restrict__ bd, uint64_t stride, cons
     const uint32_t ng = n_ff >> 5;
     const uint64_t rb = small_row_bytes(Q4_T_Q2_0, n_ff);
     float acc = 0.f;
+#pragma unroll 4
     for (uint32_t it = lane; it < n * ng; it += 32) {
         const uint32_t e = it / ng, g = it - e * ng;
         const int *qg = reinterpret_cast<const int *>(hq + (uint64_t)e * q_slice) + g * 8u;
