@@ -616,6 +616,34 @@ __device__ __forceinline__ int32_t iq4_codes_idot(const uint8_t *codes, const ui
     }
     return acc;
 }
+// Four 4-bit codes, one per byte, through the codebook: its 16 values sit in four registers and two byte permutes pick
+// by the low three bits; bit 3 chooses between them.
+constexpr int8_t kIq4Values[16] = Q4B_IQ4NL_VALUES;
+__host__ __device__ constexpr uint32_t iq4_value_word(int i) {
+    return (uint32_t)(uint8_t)kIq4Values[i] | ((uint32_t)(uint8_t)kIq4Values[i + 1] << 8) |
+           ((uint32_t)(uint8_t)kIq4Values[i + 2] << 16) | ((uint32_t)(uint8_t)kIq4Values[i + 3] << 24);
+}
+__device__ __forceinline__ uint32_t iq4_values4(uint32_t nib) {
+    const uint32_t low = nib & 0x07070707u;
+    const uint32_t t = (low | (low >> 4)) & 0x00FF00FFu;
+    const uint32_t sel = (t | (t >> 8)) & 0xFFFFu;          // one selector nibble per byte
+    constexpr uint32_t T0 = iq4_value_word(0), T1 = iq4_value_word(4), T2 = iq4_value_word(8), T3 = iq4_value_word(12);
+    const uint32_t lo = __byte_perm(T0, T1, sel);
+    const uint32_t hi = __byte_perm(T2, T3, sel);
+    const uint32_t pick = ((nib >> 3) & 0x01010101u) * 0xFFu;
+    return (lo & ~pick) | (hi & pick);
+}
+// Integer dot of 16 code bytes (2-byte aligned) with their 32 activation bytes, without a table in memory.
+__device__ __forceinline__ int32_t iq4_codes_dot(const uint8_t *codes, const int *q) {
+    int32_t acc = 0;
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+        const uint32_t v = q4b_ld_u32_a2(codes + 4 * w);
+        acc = __dp4a((int)iq4_values4(v & 0x0f0f0f0fu), q[w], acc);
+        acc = __dp4a((int)iq4_values4((v >> 4) & 0x0f0f0f0fu), q[4 + w], acc);
+    }
+    return acc;
+}
 // Group g (32 weights) of a row of type T (20 or 23): where its codes are, its integer scale
 // factor and the fp16 block scale.
 template <uint32_t T>
@@ -680,9 +708,6 @@ __global__ void moe_gu4_k(const uint8_t *__restrict__ bg, const uint8_t *__restr
                           const int32_t *__restrict__ slots, const int32_t *__restrict__ n_dev,
                           const int8_t *__restrict__ xq, const float *__restrict__ xd, uint32_t in_dim,
                           uint32_t n_ff, float *__restrict__ h) {
-    __shared__ uint16_t pair[256];
-    iq4_fill_pair_table(pair);
-    __syncthreads();
     q4b_pdl_wait();
     const uint32_t f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (f >= n_ff) return;
@@ -701,9 +726,9 @@ __global__ void moe_gu4_k(const uint8_t *__restrict__ bg, const uint8_t *__restr
             int lsf;
             float d;
             const uint8_t *cg = iq4_group<T>(rg, g, &lsf, &d);
-            ag = fmaf(__fmul_rn(d, dx), (float)(iq4_codes_idot(cg, pair, qv) * lsf), ag);
+            ag = fmaf(__fmul_rn(d, dx), (float)(iq4_codes_dot(cg, qv) * lsf), ag);
             const uint8_t *cu = iq4_group<T>(ru, g, &lsf, &d);
-            au = fmaf(__fmul_rn(d, dx), (float)(iq4_codes_idot(cu, pair, qv) * lsf), au);
+            au = fmaf(__fmul_rn(d, dx), (float)(iq4_codes_dot(cu, qv) * lsf), au);
         }
         ag = q4b_warp_sum(ag);
         au = q4b_warp_sum(au);
@@ -711,25 +736,34 @@ __global__ void moe_gu4_k(const uint8_t *__restrict__ bg, const uint8_t *__restr
     }
 }
 
-// Down projection with rows of type T: the counterpart of moe_ya_k (same reduction shape).
+// The sum over the four warps that share an output row, added to it.
+__device__ __forceinline__ void down_row_add(float acc, float *y) {
+    __shared__ float part[8];
+    acc = q4b_warp_sum(acc);
+    if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if ((threadIdx.x & 127u) == 0 && y) {
+        const float *p = part + (threadIdx.x >> 5);
+        *y += (p[0] + p[1]) + (p[2] + p[3]);
+    }
+}
+// Down projection with rows of type T: the counterpart of moe_ya_k.  Two rows a CTA, four warps a row: with a warp a row
+// there were 14 warps an SM, each with five dependent trips (12 us for ten experts of 2048 x 512).  Codes become
+// values by byte permutes, so no table has to be filled.
 template <uint32_t T>
 __global__ void moe_ya4_k(const uint8_t *__restrict__ bd, uint64_t stride, const int32_t *__restrict__ slots,
                           const float *__restrict__ wts, uint32_t n_host, const int32_t *__restrict__ n_dev,
                           const int8_t *__restrict__ hq, const float *__restrict__ hd, uint64_t q_slice,
                           uint64_t d_slice, uint32_t n_ff, uint32_t n_embd, float *__restrict__ y) {
-    __shared__ uint16_t pair[256];
-    iq4_fill_pair_table(pair);
-    __syncthreads();
     q4b_pdl_wait();
-    const uint32_t r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (r >= n_embd) return;
-    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t row = blockIdx.x * 2u + (threadIdx.x >> 7), lane = threadIdx.x & 127u;
+    const uint32_t r = min(row, n_embd - 1u);   // an odd last CTA: its second half is computed and dropped
     const uint32_t n = n_dev ? (uint32_t)*n_dev : n_host;
     const uint32_t ng = n_ff >> 5;
     const uint64_t rb = iq4_row_bytes(T, n_ff);
     float acc = 0.f;
 #pragma unroll 4   // several items' loads in flight: a trip is a chain of three
-    for (uint32_t it = lane; it < n * ng; it += 32) {
+    for (uint32_t it = lane; it < n * ng; it += 128) {
         const uint32_t e = it / ng, g = it - e * ng;
         const int *qg = reinterpret_cast<const int *>(hq + (uint64_t)e * q_slice) + g * 8u;
         int qv[8];
@@ -738,12 +772,11 @@ __global__ void moe_ya4_k(const uint8_t *__restrict__ bd, uint64_t stride, const
         int lsf;
         float d;
         const uint8_t *codes = iq4_group<T>(bd + (uint64_t)slots[e] * stride + (uint64_t)r * rb, g, &lsf, &d);
-        const int I = iq4_codes_idot(codes, pair, qv);
+        const int I = iq4_codes_dot(codes, qv);
         const float dd = __fmul_rn(d, hd[(uint64_t)e * d_slice + g]);
         acc = fmaf(__fmul_rn(wts[e], dd), (float)(I * lsf), acc);
     }
-    acc = q4b_warp_sum(acc);
-    if (lane == 0) y[r] += acc;
+    down_row_add(acc, row < n_embd ? y + row : nullptr);
 }
 
 // IQ3_S row r times an fp32 vector, one warp (every lane gets its partial sum; the caller
@@ -838,12 +871,13 @@ bool moe_exec_tail(const uint8_t *base, uint64_t stride, const int32_t *d_slots,
     const size_t sm = 2048 + in_dim + 8 * (in_dim >> 5);
     const bool tiled = q4b_ptr_tiled(base);
     // a count on the device: the grid is cut for 16 experts, more are walked in strides of it
-    const dim3 gg((n_ff + 7) / 8, d_n ? 16u : n_host);
+    const uint32_t gn = d_n ? 16u : n_host;
+    const dim3 gg((n_ff + 7) / 8, gn), gx((n_ff + 15) / 16, gn);
     if (gt == Q4_T_IQ3_XXS)
-        q4b_launch(moe_gux_k<Q4_T_IQ3_XXS>, gg, 256, 0, s.stream, base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff,
+        q4b_launch(moe_gux_k<Q4_T_IQ3_XXS>, gx, 512, 0, s.stream, base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff,
                    s.grid3xxs_d, s.grid2s_d, d_h);
     else if (gt == Q4_T_IQ2_S)
-        q4b_launch(moe_gux_k<Q4_T_IQ2_S>, gg, 256, 0, s.stream, base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff,
+        q4b_launch(moe_gux_k<Q4_T_IQ2_S>, gx, 512, 0, s.stream, base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff,
                    s.grid3xxs_d, s.grid2s_d, d_h);
     else if (gt == Q4_T_IQ4_NL)
         q4b_launch(moe_gu4_k<Q4_T_IQ4_NL>, gg, 256, 0, s.stream, base + og, base + ou, stride, d_slots, d_n, xq, xd, in_dim, n_ff, d_h);
@@ -858,16 +892,16 @@ bool moe_exec_tail(const uint8_t *base, uint64_t stride, const int32_t *d_slots,
     if (!launch_quant8(d_h, n_ff, n_ff, ne, s.xq, s.xd, s.xbs, Q4B_XQ_MAXLEN, Q4B_XQ_MAXLEN / 32,
                        d_n))
         return false;
-    const unsigned gy = (n_embd + 7) / 8;
+    const unsigned gy = (n_embd + 7) / 8, g2 = (n_embd + 1) / 2;
     const uint64_t qsl = Q4B_XQ_MAXLEN, dsl = Q4B_XQ_MAXLEN / 32;
     if (dt == Q4_T_Q2_0)
-        q4b_launch(moe_ya20_k, gy, 256, 0, s.stream, base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, s.xbs, qsl, dsl, n_ff,
+        q4b_launch(moe_ya20_k, g2, 256, 0, s.stream, base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, s.xbs, qsl, dsl, n_ff,
                    n_embd, d_y);
     else if (dt == Q4_T_IQ4_NL)
-        q4b_launch(moe_ya4_k<Q4_T_IQ4_NL>, gy, 256, 0, s.stream, base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, qsl, dsl,
+        q4b_launch(moe_ya4_k<Q4_T_IQ4_NL>, g2, 256, 0, s.stream, base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, qsl, dsl,
                    n_ff, n_embd, d_y);
     else if (dt == Q4_T_IQ4_XS)
-        q4b_launch(moe_ya4_k<Q4_T_IQ4_XS>, gy, 256, 0, s.stream, base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, qsl, dsl,
+        q4b_launch(moe_ya4_k<Q4_T_IQ4_XS>, g2, 256, 0, s.stream, base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, qsl, dsl,
                    n_ff, n_embd, d_y);
     else if (tiled)
         q4b_launch(moe_ya_k<true>, gy, 256, 0, s.stream, base + od, stride, d_slots, d_wts, n_host, d_n, s.xq, s.xd, s.xbs, qsl, dsl,

@@ -43,24 +43,6 @@ __device__ __forceinline__ float ld_f16(const uint8_t *p) {
     return __half2float(__ushort_as_half((unsigned short)q4b_ld_u16(p)));
 }
 
-// four 4-bit codes, one per byte, through the IQ4_NL codebook: the 16 values sit in four
-// registers and two byte permutes pick by the low three bits; bit 3 chooses between them
-constexpr int8_t kNl[16] = Q4B_IQ4NL_VALUES;
-__host__ __device__ constexpr uint32_t nl_word(int i) {
-    return (uint32_t)(uint8_t)kNl[i] | ((uint32_t)(uint8_t)kNl[i + 1] << 8) | ((uint32_t)(uint8_t)kNl[i + 2] << 16) |
-           ((uint32_t)(uint8_t)kNl[i + 3] << 24);
-}
-__device__ __forceinline__ uint32_t nl_codes4(uint32_t nib) {
-    const uint32_t low = nib & 0x07070707u;
-    const uint32_t t = (low | (low >> 4)) & 0x00FF00FFu;
-    const uint32_t sel = (t | (t >> 8)) & 0xFFFFu;          // one selector nibble per byte
-    constexpr uint32_t T0 = nl_word(0), T1 = nl_word(4), T2 = nl_word(8), T3 = nl_word(12);
-    const uint32_t lo = __byte_perm(T0, T1, sel);
-    const uint32_t hi = __byte_perm(T2, T3, sel);
-    const uint32_t pick = ((nib >> 3) & 0x01010101u) * 0xFFu;
-    return (lo & ~pick) | (hi & pick);
-}
-
 // 6-bit scale and minimum of sub-block j in the 12 packed bytes of a Q4_K / Q5_K block
 __device__ __forceinline__ void k_scale_min(const uint8_t *p, int j, int *sc, int *mn) {
     if (j < 4) {
@@ -155,7 +137,7 @@ template <> struct Fmt<23u> {
         uint32_t v[4];
         ld16<8>(blk + 8u + 16u * ib, v);
 #pragma unroll
-        for (int i = 0; i < 4; i++) R.w[i] = nl_codes4((v[i] >> (4u * hi)) & 0x0F0F0F0Fu);
+        for (int i = 0; i < 4; i++) R.w[i] = iq4_values4((v[i] >> (4u * hi)) & 0x0F0F0F0Fu);
         const uint32_t sh = q4b_ld_u16(blk + 2);
         const int ls = (int)(((blk[4u + (ib >> 1)] >> (4u * (ib & 1u))) & 15u) | (((sh >> (2u * ib)) & 3u) << 4));
         R.a = __fmul_rn(ld_f16(blk), (float)(ls - 32));
@@ -171,7 +153,7 @@ template <> struct Fmt<20u> {
         uint32_t v[4];
         ld16<2>(blk + 2, v);
 #pragma unroll
-        for (int i = 0; i < 4; i++) R.w[i] = nl_codes4((v[i] >> (4u * r)) & 0x0F0F0F0Fu);
+        for (int i = 0; i < 4; i++) R.w[i] = iq4_values4((v[i] >> (4u * r)) & 0x0F0F0F0Fu);
         R.a = ld_f16(blk);
         R.c = 0.f;
     }

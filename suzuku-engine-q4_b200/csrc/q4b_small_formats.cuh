@@ -26,9 +26,6 @@ __host__ __device__ inline uint64_t small_row_bytes(uint32_t type, uint64_t ncol
     return type == Q4_T_IQ3_XXS ? (ncols / 256u) * 98u : type == Q4_T_IQ2_S ? (ncols / 256u) * 82u : (ncols / 64u) * 18u;
 }
 
-// q with the bytes negated where the mask byte is 0xFF
-__device__ __forceinline__ int neg_where(int q, uint32_t mask) { return (int)__vsub4((uint32_t)q ^ mask, mask); }
-
 // One 32-group: signed magnitudes as eight words (word k = values 4k..4k+3, already sign-applied is
 // not possible for unsigned magnitudes, so the signs come back as eight byte masks), the integer
 // sub-scale factor of each half, and the block's fp16 d.
@@ -40,7 +37,8 @@ struct SmallGroup {
     float d;
 };
 
-template <uint32_t T>
+// BOOK: the codebook is in shared memory
+template <uint32_t T, bool BOOK = false>
 __device__ __forceinline__ void small_group(const uint8_t *row, uint32_t g, const uint32_t *grid3,
                                             const uint2 *grid2, SmallGroup &G) {
     if (T == Q4_T_IQ3_XXS) {
@@ -54,8 +52,8 @@ __device__ __forceinline__ void small_group(const uint8_t *row, uint32_t g, cons
         for (int l = 0; l < 4; l++) {
             const uint32_t s7 = (aux >> (7 * l)) & 127u;
             const uint32_t sb = s7 | ((__popc(s7) & 1u) << 7);     // the sign table: even parity
-            G.mag[2 * l] = __ldg(grid3 + idx[2 * l]);
-            G.mag[2 * l + 1] = __ldg(grid3 + idx[2 * l + 1]);
+            G.mag[2 * l] = BOOK ? grid3[idx[2 * l]] : __ldg(grid3 + idx[2 * l]);
+            G.mag[2 * l + 1] = BOOK ? grid3[idx[2 * l + 1]] : __ldg(grid3 + idx[2 * l + 1]);
             G.neg[2 * l] = q4b_sign_mask4(sb);
             G.neg[2 * l + 1] = q4b_sign_mask4(sb >> 4);
         }
@@ -69,7 +67,7 @@ __device__ __forceinline__ void small_group(const uint8_t *row, uint32_t g, cons
 #pragma unroll
         for (int l = 0; l < 4; l++) {
             const uint32_t idx = ((qs >> (8 * l)) & 0xffu) | ((qh << (8 - 2 * l)) & 0x300u);
-            const uint2 m = __ldg(grid2 + idx);
+            const uint2 m = BOOK ? grid2[idx] : __ldg(grid2 + idx);
             const uint32_t s8 = (sg >> (8 * l)) & 0xffu;
             G.mag[2 * l] = m.x;
             G.mag[2 * l + 1] = m.y;
@@ -89,8 +87,9 @@ __device__ __forceinline__ void small_group_isums(const SmallGroup &G, const int
     int a = 0, b = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        a = __dp4a((int)G.mag[k], neg_where(q[k], G.neg[k]), a);
-        b = __dp4a((int)G.mag[4 + k], neg_where(q[4 + k], G.neg[4 + k]), b);
+        // -m = ~m + 1: the negated magnitudes' complements (magnitudes are below 128), then the q they belong to once more
+        a = __dp4a((int)(G.neg[k] & 0x01010101u), q[k], __dp4a((int)(G.mag[k] ^ G.neg[k]), q[k], a));
+        b = __dp4a((int)(G.neg[4 + k] & 0x01010101u), q[4 + k], __dp4a((int)(G.mag[4 + k] ^ G.neg[4 + k]), q[4 + k], b));
     }
     *lo = a;
     *hi = b;
@@ -169,11 +168,20 @@ __global__ void small_idot_k(const uint8_t *__restrict__ w, uint64_t nrows, uint
 
 // ---- gate/up + SwiGLU with rows of type T (IQ3_XXS or IQ2_S): one warp per (expert, hidden unit) ----
 template <uint32_t T>
-__global__ void moe_gux_k(const uint8_t *__restrict__ bg, const uint8_t *__restrict__ bu, uint64_t stride,
+__global__ void __launch_bounds__(512) moe_gux_k(const uint8_t *__restrict__ bg, const uint8_t *__restrict__ bu, uint64_t stride,
                           const int32_t *__restrict__ slots, const int32_t *__restrict__ n_dev,
                           const int8_t *__restrict__ xq, const float *__restrict__ xd, uint32_t in_dim,
                           uint32_t n_ff, const uint32_t *__restrict__ grid3, const uint2 *__restrict__ grid2,
                           float *__restrict__ h) {
+    // The codebook in shared memory, filled before the wait: 32 lanes that look up different entries are one request with
+    // a few bank conflicts here, and up to 32 requests of L1 as global loads (which bound the kernel: 13.7 us).
+    __shared__ __align__(16) uint32_t book[T == Q4_T_IQ3_XXS ? 256 : 2048];
+    if (T == Q4_T_IQ3_XXS) {
+        if (threadIdx.x < 64u) reinterpret_cast<uint4 *>(book)[threadIdx.x] = __ldg(reinterpret_cast<const uint4 *>(grid3) + threadIdx.x);
+    } else {
+        reinterpret_cast<uint4 *>(book)[threadIdx.x] = __ldg(reinterpret_cast<const uint4 *>(grid2) + threadIdx.x);
+    }
+    __syncthreads();
     q4b_pdl_wait();
     const uint32_t f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (f >= n_ff) return;
@@ -192,10 +200,10 @@ __global__ void moe_gux_k(const uint8_t *__restrict__ bg, const uint8_t *__restr
             const float dx = xd[g];
             SmallGroup G;
             int lo, hi;
-            small_group<T>(rg, g, grid3, grid2, G);
+            small_group<T, true>(rg, g, book, reinterpret_cast<const uint2 *>(book), G);
             small_group_isums(G, qv, &lo, &hi);
             ag = fmaf(__fmul_rn(__fmul_rn(G.d, unit), dx), (float)(lo * G.ls0 + hi * G.ls1), ag);
-            small_group<T>(ru, g, grid3, grid2, G);
+            small_group<T, true>(ru, g, book, reinterpret_cast<const uint2 *>(book), G);
             small_group_isums(G, qv, &lo, &hi);
             au = fmaf(__fmul_rn(__fmul_rn(G.d, unit), dx), (float)(lo * G.ls0 + hi * G.ls1), au);
         }
@@ -205,22 +213,21 @@ __global__ void moe_gux_k(const uint8_t *__restrict__ bg, const uint8_t *__restr
     }
 }
 
-// ---- down projection with Q2_0 rows: the counterpart of moe_ya_k (same reduction shape) ----
+// ---- down projection with Q2_0 rows: the counterpart of moe_ya4_k (same split) ----
 __global__ void moe_ya20_k(const uint8_t *__restrict__ bd, uint64_t stride, const int32_t *__restrict__ slots,
                            const float *__restrict__ wts, uint32_t n_host, const int32_t *__restrict__ n_dev,
                            const int8_t *__restrict__ hq, const float *__restrict__ hd,
                            const int32_t *__restrict__ hbs, uint64_t q_slice, uint64_t d_slice, uint32_t n_ff,
                            uint32_t n_embd, float *__restrict__ y) {
     q4b_pdl_wait();
-    const uint32_t r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (r >= n_embd) return;
-    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t row = blockIdx.x * 2u + (threadIdx.x >> 7), lane = threadIdx.x & 127u;
+    const uint32_t r = min(row, n_embd - 1u);   // an odd last CTA: its second half is computed and dropped   // (n_embd is even)
     const uint32_t n = n_dev ? (uint32_t)*n_dev : n_host;
     const uint32_t ng = n_ff >> 5;
     const uint64_t rb = small_row_bytes(Q4_T_Q2_0, n_ff);
     float acc = 0.f;
 #pragma unroll 4
-    for (uint32_t it = lane; it < n * ng; it += 32) {
+    for (uint32_t it = lane; it < n * ng; it += 128) {
         const uint32_t e = it / ng, g = it - e * ng;
         const int *qg = reinterpret_cast<const int *>(hq + (uint64_t)e * q_slice) + g * 8u;
         uint32_t cw[8];
@@ -231,6 +238,5 @@ __global__ void moe_ya20_k(const uint8_t *__restrict__ bd, uint64_t stride, cons
         const float dd = __fmul_rn(d, hd[(uint64_t)e * d_slice + g]);
         acc = fmaf(__fmul_rn(wts[e], dd), (float)(s - hbs[(uint64_t)e * d_slice + g]), acc);
     }
-    acc = q4b_warp_sum(acc);
-    if (lane == 0) y[r] += acc;
+    down_row_add(acc, row < n_embd ? y + row : nullptr);
 }
