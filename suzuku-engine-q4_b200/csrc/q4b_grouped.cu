@@ -614,9 +614,42 @@ __global__ void __launch_bounds__(256) grouped_rows4_k(const uint8_t *__restrict
     }
 }
 
+// Which grouped product runs.  The tensor-core kernel pays off once an expert has
+// enough rows to fill a useful part of a 128 x 64 MMA tile; below that the streaming
+// CUDA-core kernel (one decode, a handful of dot products from registers) is the
+// better fit, and the general CUDA-core kernel takes what neither accepts (arenas in
+// the engine's byte order, odd widths).  In the default mode a call is split by
+// entry: entries with TC_MIN_ROWS rows or more go to the tensor cores, the rest to
+// the streaming kernel; each kernel skips the other's entries.
+int g_tc_mode = -1;  // -1 split by rows, 0 CUDA cores only, 1 tensor cores whenever the shape
+                     // allows, 2 the general CUDA-core kernel only
+// The streaming kernels' view of a call.
+wide::Args stream_args(const uint8_t *w, uint64_t expert_stride, const int32_t *act, const uint32_t *n_act, uint32_t n_entries,
+                       const int32_t *bounds, Q8View xq, uint32_t cols, uint32_t w_rows, float *dst, uint64_t ld_dst) {
+    wide::Args a = {};
+    a.w = w;
+    a.expert_stride = expert_stride;
+    a.act = act;
+    a.n_act = n_act;
+    a.n_entries = n_entries;
+    a.bounds = bounds;
+    a.xq = xq.q;
+    a.xd = xq.d;
+    a.cols = cols;
+    a.w_rows = w_rows;
+    a.dst = dst;
+    a.ld_dst = ld_dst;
+    a.err = g_q4b.err_d;
+    return a;
+}
 bool launch_grouped4(uint32_t type, const uint8_t *w, uint64_t expert_stride, const int32_t *act,
                      const uint32_t *n_act, uint32_t n_entries, const int32_t *bounds, Q8View xq, uint32_t cols,
                      uint32_t w_rows, float *dst, uint64_t ld_dst) {
+    if (g_tc_mode != 2 &&
+        rows4::launch(type, stream_args(w, expert_stride, act, n_act, n_entries, bounds, xq, cols, w_rows, dst, ld_dst))) {
+        g_q4b_launches++;
+        return q4b_launch_ok("rows4");
+    }
     const dim3 grid((w_rows + 7u) / 8u, n_entries);
     if (type == Q4_T_IQ4_NL)
         grouped_rows4_k<Q4_T_IQ4_NL><<<grid, 256, 0, g_q4b.stream>>>(w, expert_stride, act, n_act, bounds, xq, cols,
@@ -647,15 +680,6 @@ bool launch_grouped(const uint8_t *w, uint64_t expert_stride, const int32_t *act
     return q4b_launch_ok("grouped_rows");
 }
 
-// Which grouped product runs.  The tensor-core kernel pays off once an expert has
-// enough rows to fill a useful part of a 128 x 64 MMA tile; below that the streaming
-// CUDA-core kernel (one decode, a handful of dot products from registers) is the
-// better fit, and the general CUDA-core kernel takes what neither accepts (arenas in
-// the engine's byte order, odd widths).  In the default mode a call is split by
-// entry: entries with TC_MIN_ROWS rows or more go to the tensor cores, the rest to
-// the streaming kernel; each kernel skips the other's entries.
-int g_tc_mode = -1;  // -1 split by rows, 0 CUDA cores only, 1 tensor cores whenever the shape
-                     // allows, 2 the general CUDA-core kernel only
 // An entry goes to the tensor cores from 12 rows: beyond the three rows it keeps in registers the
 // streaming kernel re-fetches the activation rows for every tile, which costs more than the
 // tensor-core kernel's fixed work per tile.  Measured (48 layers of 64 tokens / 48 layers of 4
@@ -691,13 +715,18 @@ bool launch_grouped_any(const uint8_t *w, uint64_t expert_stride, const int32_t 
         g_q4b_launches += 3;
         return ok && q4b_launch_ok("mmq_wide");
     }
-    const bool few_ok = wide_ok || (g_tc_mode != 2 && g_tc_mode != 1 && tiled && few::shape_ok(w_rows, cols, n_entries));
+    if (wide_ok) {
+        const bool ok = wide::launch(stream_args(w, expert_stride, act, n_act, n_entries, bounds, xq, cols, w_rows, dst, ld_dst));
+        g_q4b_launches++;
+        return ok && q4b_launch_ok("wide_rows");
+    }
+    const bool few_ok = g_tc_mode != 2 && g_tc_mode != 1 && tiled && few::shape_ok(w_rows, cols, n_entries);
     // rows an entry needs before the tensor cores take it
     uint32_t tc_min = 0xffffffffu;
     // a prefill-sized call (thousands of rows): the tensor-core kernel is running anyway and takes
     // entries from 6 rows (2048 tokens: 1.083 ms against 1.097 at 12, 1.086 at 4 and at 8)
     const uint32_t split_rows = total_rows >= 4096u ? 6u : TC_MIN_ROWS;
-    if (tc_ok && !wide_ok) tc_min = g_tc_mode == 1 ? 1u : (few_ok ? split_rows : 0xffffffffu);
+    if (tc_ok) tc_min = g_tc_mode == 1 ? 1u : (few_ok ? split_rows : 0xffffffffu);
     if (tc_ok && g_tc_mode == -1 && !few_ok && total_rows >= 8ull * n_entries) tc_min = 1u;
     const bool run_tc = tc_min != 0xffffffffu && max_rows_hint >= tc_min;
     // When a call is split, the two kernels touch disjoint entries and rows: the tensor-core
@@ -719,30 +748,6 @@ bool launch_grouped_any(const uint8_t *w, uint64_t expert_stride, const int32_t 
         g_q4b_launches++;
         if (!ok || !q4b_launch_ok("mmq_tc")) return false;
         if (tc_min <= 1u) return true;
-    }
-    if (wide_ok) {
-        wide::Args a = {};
-        a.w = w;
-        a.expert_stride = expert_stride;
-        a.act = act;
-        a.n_act = n_act;
-        a.n_entries = n_entries;
-        a.bounds = bounds;
-        a.xq = xq.q;
-        a.xd = xq.d;
-        a.cols = cols;
-        a.w_rows = w_rows;
-        a.dst = dst;
-        a.ld_dst = ld_dst;
-        a.err = g_q4b.err_d;
-        a.max_rows = run_tc ? tc_min - 1u : 0x7fffffffu;
-        const bool ok = wide::launch(a);
-        g_q4b_launches++;
-        if (!ok || !q4b_launch_ok("wide_rows")) return false;
-        if (side && (cudaEventRecord(g_q4b.ev_join, g_q4b.aux_stream) != cudaSuccess ||
-                     cudaStreamWaitEvent(g_q4b.stream, g_q4b.ev_join, 0) != cudaSuccess))
-            return false;
-        return true;
     }
     if (few_ok) {
         few::Args a;
@@ -802,7 +807,7 @@ bool q4b_mmq_tc_warm() {
         cudaGetLastError();
         return false;
     }
-    const bool f = few::warm() && wide::warm();
+    const bool f = few::warm() && wide::warm() && rows4::warm();
     return mmqtc::warm() && mmqtc::warm_wide() && f;
 }
 extern "C" bool q4_cuda_mmq_tc_mode(int mode) {

@@ -65,9 +65,11 @@ struct Args {
     float *dst;
     uint64_t ld_dst;
     uint32_t *err;
-    uint32_t max_rows;           // entries with more rows are left to the tensor-core kernel
-    uint32_t ct, n_stage;        // tiles per chunk (whole units), chunks in the ring
+    uint32_t ct;                 // tiles per chunk (whole units)
+    uint32_t n_stage;            // chunks in the ring
     uint32_t ks_log;             // log2 of the warps per unit of 16 weight rows in the mma form
+    uint32_t cpe;                // chunks of a matrix
+    uint32_t chunk_bytes, last_bytes;
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -126,8 +128,8 @@ __host__ __device__ inline uint32_t scale_stride(uint32_t cols) { return (cols >
 __host__ __device__ inline uint32_t act_bytes(uint32_t cols) {
     return (RBLK * (act_stride(cols) + scale_stride(cols)) + 127u) & ~127u;
 }
-__host__ __device__ inline uint32_t smem_bytes(uint32_t cols, uint32_t ct, uint32_t n_stage) {
-    return (uint32_t)((sizeof(Smem) + 127u) & ~127u) + 2u * act_bytes(cols) + n_stage * ct * Q4B_WIDE_BYTES;
+__host__ __device__ inline uint32_t smem_bytes(uint32_t cols, uint32_t chunk_bytes, uint32_t n_stage) {
+    return (uint32_t)((sizeof(Smem) + 127u) & ~127u) + 2u * act_bytes(cols) + n_stage * chunk_bytes;
 }
 // Relative cost of a chunk for a block of rows: the stream of its bytes until the rows' own work exceeds it
 // (370 experts, gate/up: 72 us with 1 row, 80 with 2, 105 with up to 8, 145 with up to 16).
@@ -147,20 +149,24 @@ __device__ __forceinline__ uint32_t entry_cost(uint32_t rows, uint32_t cpe) {
     return cpe * sp.nb * block_cost(sp.per);
 }
 
-// BB: super-blocks per weight row, 1, 2, 4 or 8; 0 = another number (mma form only).  TPW: tiles a warp takes
-// from a full chunk in the dp4a form.
-template <uint32_t BB, uint32_t TPW>
-__global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
-    extern __shared__ __align__(128) uint8_t smem_raw[];
+// One item as the body of a kernel sees it: rows, where its results go, its activation rows and their scales in shared
+// memory; the chunks [ch, ch_stop) of its weights are taken one after the other (acquire, release).
+struct Item {
+    uint32_t nr;
+    float *out;
+    const uint8_t *ab, *sbase;
+    uint32_t ch_stop;
+    float (*red)[32][4];
+};
+// Streams this CTA's share of the (item, chunk) list through the ring and hands every item to body(item, ch, acquire,
+// release); the body advances ch to ch_stop.
+template <typename Body> __device__ __forceinline__ void stream_items(const Args &a, uint8_t *smem_raw, const Body &body) {
     Smem &s = *reinterpret_cast<Smem *>(smem_raw);
     uint8_t *const actb = smem_raw + ((sizeof(Smem) + 127u) & ~127u);
     const uint32_t act_sz = act_bytes(a.cols), sc_off = RBLK * act_stride(a.cols);
     uint8_t *const stage = actb + 2u * act_sz;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t n_ent = a.n_act ? min(*a.n_act, a.n_entries) : a.n_entries;
-    const uint32_t B = BB ? BB : a.cols >> 8;
-    const uint32_t n_tiles = (a.w_rows >> 3) * B;
-    const uint32_t cpe = (n_tiles + a.ct - 1u) / a.ct;         // chunks per pass over a matrix
+    const uint32_t cpe = a.cpe;
     if (tid == 0) {
         for (uint32_t i = 0; i < a.n_stage; i++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s.full[i])), "r"(1u));
@@ -170,6 +176,8 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s.act_full[i])), "r"(1u));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    q4b_pdl_wait();
+    const uint32_t n_ent = a.n_act ? min(*a.n_act, a.n_entries) : a.n_entries;
     // ---- the live entries and the prefix of their costs: a thread takes two neighbouring entries ----
     uint32_t n_live, total_cost;
     {
@@ -178,7 +186,7 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
         for (uint32_t h = 0; h < 2; h++) {
             const uint32_t e = 2u * tid + h;
             const int32_t nr = e < n_ent ? a.bounds[e + 1] - a.bounds[e] : 0;
-            r[h] = nr > 0 && (uint32_t)nr <= a.max_rows ? (uint32_t)nr : 0u;
+            r[h] = nr > 0 ? (uint32_t)nr : 0u;
             if (r[h]) {
                 lv++;
                 cs += entry_cost(r[h], cpe);
@@ -238,8 +246,7 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
     // is last through an item's last chunk brings the activation rows of the item after the next into the buffer
     // that has become free (one lane; refills come in order, because a warp leaves chunk k + 1 only after it has
     // refilled behind chunk k).
-    const uint32_t blk_end = ix_end / cpe, ch_end = ix_end - blk_end * cpe, chunk_bytes = a.ct * Q4B_WIDE_BYTES;
-    const uint32_t last_tiles = n_tiles - (cpe - 1u) * a.ct;
+    const uint32_t blk_end = ix_end / cpe, ch_end = ix_end - blk_end * cpe, chunk_bytes = a.chunk_bytes;
     auto rows_of = [&](uint32_t e) { return (uint32_t)(__ldg(a.bounds + e + 1) - __ldg(a.bounds + e)); };
     auto refill = [&](uint32_t st) {
         uint32_t pl = s.p_li, pb = s.p_blk, pc = s.p_ch;
@@ -249,7 +256,7 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
             s.p_nb = split_rows(rows_of(e)).nb;
             s.p_mat = a.w + (uint64_t)(a.act ? __ldg(a.act + e) : (int32_t)e) * a.expert_stride;
         }
-        const uint32_t bytes = pc + 1u == cpe ? last_tiles * Q4B_WIDE_BYTES : chunk_bytes;
+        const uint32_t bytes = pc + 1u == cpe ? a.last_bytes : chunk_bytes;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&s.full[st])), "r"(bytes) : "memory");
         bulk_g2s(stage + st * chunk_bytes, s.p_mat + (uint64_t)pc * chunk_bytes, bytes, &s.full[st]);
         bool next = false;
@@ -286,11 +293,6 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
 
     // ---- the warps ----
     uint32_t st = 0, ph = 0, item = 0, limit = WAIT_LIMIT, blk = ix / cpe, ch = ix - blk * cpe;
-    const uint32_t rows_per_chunk = a.ct / B * 8u;
-    // mma form: lane (g, t) of a fragment; this warp's unit slot and its share of a unit's super-blocks
-    const uint32_t g = lane >> 2, t = lane & 3u;
-    const uint32_t ks = warp & ((1u << a.ks_log) - 1u), slot = warp >> a.ks_log, n_slot = NCW >> a.ks_log;
-    const uint32_t b_lo = (B * ks) >> a.ks_log, b_hi = (B * (ks + 1u)) >> a.ks_log;
     bool entry = true;
     uint32_t rows = 0;
     Split sp = {1u, 0u};
@@ -325,6 +327,31 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
             }
             if (++st == a.n_stage) st = 0, ph ^= 1u;
         };
+        const Item it = {nr, out, ab, sbase, ch_stop, s.red};
+        body(it, ch, acquire, release);
+        if (ch_stop != cpe) break;         // the end of this CTA's share
+        item++;
+        ch = 0, blk++;
+        if (blk == sp.nb) blk = 0, li++, entry = true;
+    }
+}
+
+// BB: super-blocks per weight row, 1, 2, 4 or 8; 0 = another number (mma form only).  TPW: tiles a warp takes
+// from a full chunk in the dp4a form.
+template <uint32_t BB, uint32_t TPW>
+__global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, cpe = a.cpe;
+    const uint32_t B = BB ? BB : a.cols >> 8, last_tiles = (a.w_rows >> 3) * B - (cpe - 1u) * a.ct;
+    const uint32_t rows_per_chunk = a.ct / B * 8u;
+    // mma form: lane (g, t) of a fragment; this warp's unit slot and its share of a unit's super-blocks
+    const uint32_t g = lane >> 2, t = lane & 3u;
+    const uint32_t ks = warp & ((1u << a.ks_log) - 1u), slot = warp >> a.ks_log, n_slot = NCW >> a.ks_log;
+    const uint32_t b_lo = (B * ks) >> a.ks_log, b_hi = (B * (ks + 1u)) >> a.ks_log;
+    stream_items(a, smem_raw, [&](const Item &it, uint32_t &ch, auto &acquire, auto &release) {
+        const uint32_t nr = it.nr, ch_stop = it.ch_stop;
+        float *const out = it.out;
+        const uint8_t *const ab = it.ab, *const sbase = it.sbase;
         auto few = [&](auto nr_tag) {
             constexpr uint32_t NR = decltype(nr_tag)::value, B1 = BB ? BB : 1u, lpr = 4u * B1, rpt = 8u / B1;
             const uint32_t p = lane & 3u, bl = lane >> 2;
@@ -481,11 +508,11 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
                         const uint32_t bar_n = 32u << a.ks_log, w0 = slot * ((1u << a.ks_log) - 1u);
 #pragma unroll
                         for (int j = 0; j < NTL; j++) {
-                            if (ks) *reinterpret_cast<float4 *>(s.red[w0 + ks - 1u][lane]) =
+                            if (ks) *reinterpret_cast<float4 *>(it.red[w0 + ks - 1u][lane]) =
                                 make_float4(sum[j][0], sum[j][1], sum[j][2], sum[j][3]);
                             asm volatile("bar.sync %0, %1;" ::"r"(1u + slot), "r"(bar_n) : "memory");
                             if (ks == 0) {
-                                auto part = [&](uint32_t i, int o) { return s.red[w0 + i - 1u][lane][o]; };
+                                auto part = [&](uint32_t i, int o) { return it.red[w0 + i - 1u][lane][o]; };
 #pragma unroll
                                 for (int o = 0; o < 4; o++) {
                                     if (BB == 0) {
@@ -523,11 +550,7 @@ __global__ void __launch_bounds__(NT, 1) wide_rows_k(const Args a) {
         else if (BB != 0 && nr == 2u) few(std::integral_constant<uint32_t, 2>{});
         else if (nr <= 8u) many(std::integral_constant<int, 1>{});
         else many(std::integral_constant<int, 2>{});
-        if (ch_stop != cpe) break;         // the end of this CTA's share
-        item++;
-        ch = 0, blk++;
-        if (blk == sp.nb) blk = 0, li++, entry = true;
-    }
+    });
 }
 
 // ---- host side ----
@@ -548,7 +571,7 @@ bool warm() {
 // four fragments a warp, were slower than two passes of 16: they spill, and their rows leave room for 32 tiles a
 // chunk only: 370 experts of 32 rows 425 us against 284.)
 static bool plan(Args &a) {
-    const uint32_t B = a.cols >> 8;
+    const uint32_t B = a.cols >> 8, n_tiles = (a.w_rows >> 3) * B;
     const uint64_t tiles = (uint64_t)(a.w_rows >> 3) * B * a.n_entries;
     const bool small = tiles / 64u < 20ull * (uint64_t)g_q4b.n_sm;
     for (uint32_t want = small ? 32u : 64u; want >= 8u; want /= 2u) {
@@ -558,10 +581,13 @@ static bool plan(Args &a) {
         a.ct = units * 2u * B;
         a.ks_log = 0;
         while ((units << (a.ks_log + 1u)) <= NCW && (2u << a.ks_log) <= B && a.ks_log < 3u) a.ks_log++;
+        a.chunk_bytes = a.ct * Q4B_WIDE_BYTES;
         a.n_stage = MAX_STAGE;
-        while (a.n_stage >= 2u && smem_bytes(a.cols, a.ct, a.n_stage) > SMEM_MAX) a.n_stage--;
+        while (a.n_stage >= 2u && smem_bytes(a.cols, a.chunk_bytes, a.n_stage) > SMEM_MAX) a.n_stage--;
         if (a.n_stage >= 2u || want < 4u * B) break;
     }
+    a.cpe = (n_tiles + a.ct - 1u) / a.ct;
+    a.last_bytes = (n_tiles - (a.cpe - 1u) * a.ct) * Q4B_WIDE_BYTES;
     return a.n_stage >= 2u;
 }
 bool shape_ok(const uint8_t *w, uint64_t stride, uint64_t w_rows, uint64_t w_cols, uint32_t n_entries) {
@@ -573,15 +599,15 @@ bool shape_ok(const uint8_t *w, uint64_t stride, uint64_t w_rows, uint64_t w_col
     return plan(a);
 }
 template <uint32_t BB> static void launch_b(const Args &a, size_t sm) {
-    if (a.ct > 32u || BB == 0) wide_rows_k<BB, 4><<<g_q4b.n_sm, NT, sm, g_q4b.stream>>>(a);
-    else wide_rows_k<BB, 2><<<g_q4b.n_sm, NT, sm, g_q4b.stream>>>(a);
+    if (a.ct > 32u || BB == 0) q4b_launch(wide_rows_k<BB, 4>, g_q4b.n_sm, NT, sm, g_q4b.stream, a);
+    else q4b_launch(wide_rows_k<BB, 2>, g_q4b.n_sm, NT, sm, g_q4b.stream, a);
 }
 // a.w and a.expert_stride as the caller has them (tiled bytes)
 bool launch(Args a) {
     a.w = q4b_wide_of(a.w);
     if (!a.w || !plan(a)) return false;
     a.expert_stride = a.expert_stride / Q4B_TILE_BYTES * Q4B_WIDE_BYTES;
-    const size_t sm = smem_bytes(a.cols, a.ct, a.n_stage);
+    const size_t sm = smem_bytes(a.cols, a.chunk_bytes, a.n_stage);
     switch (a.cols >> 8) {
     case 1: launch_b<1>(a, sm); break;
     case 2: launch_b<2>(a, sm); break;

@@ -11,6 +11,7 @@
 #include "q4b_router.cu"
 #include "q4b_few.cu"
 #include "q4b_wide.cu"
+#include "q4b_rows4.cu"
 #include "q4b_grouped.cu"
 #include "q4b_elem.cu"
 #include "q4b_mmvq.cu"
