@@ -88,6 +88,7 @@ template <bool COMPAT>
 __global__ void quantize_rows_k(const float *__restrict__ x, const int32_t *__restrict__ ids,
                                 uint64_t cols, uint64_t rows, int8_t *__restrict__ q,
                                 float *__restrict__ d, int32_t *__restrict__ bs) {
+    q4b_pdl_wait();
     const uint32_t gpr = (uint32_t)(cols >> 5);
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t g = t >> 2;                       // 32-group
@@ -245,6 +246,7 @@ template <bool COMPAT>
 __global__ void swiglu_quant_rows_k(const float *__restrict__ gu, uint64_t rows, uint64_t n_ff,
                                     int8_t *__restrict__ q, float *__restrict__ d,
                                     int32_t *__restrict__ bs) {
+    q4b_pdl_wait();
     const uint32_t gpr = (uint32_t)(n_ff >> 5);
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t g = t >> 2;
@@ -309,27 +311,44 @@ __global__ void expert_reduce_k(float *__restrict__ y, const float *__restrict__
     else
         y[(uint64_t)t * n_embd + c] = 0.f + acc;
 }
-// The same sums four columns per thread (n_embd % 4 == 0, 16-byte aligned rows): the picks'
-// rows are read as float4, each column still adds its picks in the order k = 0..topk-1.
+// The same sums four columns per thread (n_embd % 4 == 0, 16-byte aligned rows): the picks' rows are read as float4, up
+// to eight of them in flight (a pick's place and its row are two dependent loads; one pick after the other a token
+// of 11 picks took 7 us), each column still adds its picks in the order k = 0..topk-1.  cnt (optional): picks of
+// the token that count, the others are left out.
 template <bool ADD>
-__global__ void __launch_bounds__(256) expert_reduce4_k(float *__restrict__ y, const float *__restrict__ pd,
+__global__ void __launch_bounds__(128) expert_reduce4_k(float *__restrict__ y, const float *__restrict__ pd,
                                                         const int32_t *__restrict__ rsrc,
                                                         const float *__restrict__ rw, uint32_t topk,
-                                                        uint32_t n_embd) {
+                                                        uint32_t n_embd, const int32_t *__restrict__ cnt) {
+    __shared__ int32_t sp[64];
+    __shared__ float sw[64];
+    q4b_pdl_wait();
     const uint32_t t = blockIdx.y;
+    const uint32_t n = cnt ? min(topk, (uint32_t)max(cnt[t], 0)) : topk;
+    if (threadIdx.x < n) {
+        sp[threadIdx.x] = rsrc[(uint64_t)t * topk + threadIdx.x];
+        sw[threadIdx.x] = rw[(uint64_t)t * topk + threadIdx.x];
+    }
+    __syncthreads();
     const uint32_t c4 = blockIdx.x * blockDim.x + threadIdx.x;
     if (c4 >= n_embd / 4u) return;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (uint32_t k = 0; k < topk; k++) {
-        const int32_t p = rsrc[(uint64_t)t * topk + k];
-        if (p >= 0) {
-            const float w = rw[(uint64_t)t * topk + k];
-            const float4 v = __ldcs(reinterpret_cast<const float4 *>(pd + (uint64_t)p * n_embd) + c4);
-            acc.x += w * v.x;
-            acc.y += w * v.y;
-            acc.z += w * v.z;
-            acc.w += w * v.w;
+    for (uint32_t k0 = 0; k0 < n; k0 += 8u) {
+        float4 v[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8; i++) {
+            const int32_t p = k0 + i < n ? sp[k0 + i] : -1;
+            if (p >= 0) v[i] = __ldcs(reinterpret_cast<const float4 *>(pd + (uint64_t)p * n_embd) + c4);
         }
+#pragma unroll
+        for (uint32_t i = 0; i < 8; i++)
+            if (k0 + i < n && sp[k0 + i] >= 0) {
+                const float w = sw[k0 + i];
+                acc.x += w * v[i].x;
+                acc.y += w * v[i].y;
+                acc.z += w * v[i].z;
+                acc.w += w * v[i].w;
+            }
     }
     float4 *o = reinterpret_cast<float4 *>(y + (uint64_t)t * n_embd) + c4;
     if (ADD) {
@@ -341,13 +360,12 @@ __global__ void __launch_bounds__(256) expert_reduce4_k(float *__restrict__ y, c
 }
 template <bool ADD>
 static void launch_expert_reduce(float *y, const float *pd, const int32_t *rsrc, const float *rw, uint32_t n_tok,
-                                 uint32_t topk, uint32_t n_embd) {
-    if ((n_embd & 3u) == 0 && (((uintptr_t)y | (uintptr_t)pd) & 15u) == 0)
-        expert_reduce4_k<ADD><<<dim3((n_embd / 4u + 255u) / 256u, n_tok), 256, 0, g_q4b.stream>>>(y, pd, rsrc, rw,
-                                                                                                topk, n_embd);
+                                 uint32_t topk, uint32_t n_embd, const int32_t *cnt = nullptr) {
+    if ((n_embd & 3u) == 0 && topk <= 64u && (((uintptr_t)y | (uintptr_t)pd) & 15u) == 0)
+        q4b_launch(expert_reduce4_k<ADD>, dim3((n_embd / 4u + 127u) / 128u, n_tok), 128, 0, g_q4b.stream, y, pd, rsrc, rw, topk,
+                   n_embd, cnt);
     else
-        expert_reduce_k<ADD><<<dim3((n_embd + 255) / 256, n_tok), 256, 0, g_q4b.stream>>>(y, pd, rsrc, rw, topk,
-                                                                                         n_embd);
+        expert_reduce_k<ADD><<<dim3((n_embd + 255) / 256, n_tok), 256, 0, g_q4b.stream>>>(y, pd, rsrc, rw, topk, n_embd);
 }
 
 // One block (256 threads, or 1024 for a large group) per group of gsz tokens: a stable counting
@@ -369,13 +387,14 @@ __global__ void __launch_bounds__(1024) assign_k(
     // [tok_first, tok_first + tok_count).  bounds_full (optional) receives the first row of
     // every expert and the total: n_exp + 1 values.  Rows of a_tok beyond the total get -1.
     extern __shared__ uint32_t sh[];  // hist[nw][n_exp], cnt[n_exp], rank[n_exp], wsum[40]
-    const uint32_t nw = blockDim.x >> 5;
+    q4b_pdl_wait();
+    const uint32_t nw = min(blockDim.x >> 5, (min(gsz, n_tok) * topk + 31u) >> 5);   // warps that place picks
     uint32_t *hist = sh, *cnt = sh + nw * n_exp, *rank = cnt + n_exp, *wsum = rank + n_exp;
     const uint32_t g = blockIdx.x, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t t0 = g * gsz, t1 = min(t0 + gsz, n_tok);
     const uint32_t seg = g * gsz * topk, rows = (t1 - t0) * topk;
     const uint32_t run = ((rows + nw - 1u) / nw + 31u) & ~31u;  // picks per warp, a multiple of 32
-    const uint32_t i_lo = warp * run, i_hi = min(rows, i_lo + run);
+    const uint32_t i_lo = warp < nw ? warp * run : 0u, i_hi = warp < nw ? min(rows, i_lo + run) : 0u;
     auto pick_id = [&](uint32_t i) -> int32_t {   // i = pick index within the group
         const uint32_t t = i / topk, k = i - t * topk;
         if (k >= topk_in)
@@ -483,55 +502,72 @@ __global__ void __launch_bounds__(1024) assign_k(
     }
 }
 
-// Verify window: per-token slot lists (stride 64, count per token; n_tok <= 8) ->
-// entries = distinct slots in order of first appearance, their rows in (token, pick)
-// order, bounds per entry.  One block of 512 threads, one per possible pick.
+// Verify window: per-token slot lists (stride 64, count per token; n_tok <= 8) -> entries = distinct slots in order of
+// first appearance, their rows in (token, pick) order, bounds per entry; a_tok of unused rows is -1.  One block of 512
+// threads, one per possible pick; the valid picks are packed first, so that the comparisons of a pick with the ones
+// before it run over picks only (some 40 of them in use, not 512: 8.9 -> 4 us).
 __global__ void __launch_bounds__(512) win_assign_k(
     const int32_t *__restrict__ es, const float *__restrict__ ew, const int32_t *__restrict__ nh,
     uint32_t n_tok, int32_t *__restrict__ act, uint32_t *__restrict__ n_act,
     int32_t *__restrict__ bounds, int32_t *__restrict__ a_tok, int32_t *__restrict__ rsrc,
     float *__restrict__ rw) {
-    __shared__ int32_t slot[512];
-    __shared__ int32_t lead[512];   // index of the first pick with the same slot, or -1 (invalid)
-    __shared__ int32_t ent[512];    // entry number of a leader
-    __shared__ int32_t size[513];
-    const uint32_t i = threadIdx.x, t = i >> 6, k = i & 63u;
+    __shared__ int32_t slot[512];   // packed picks
+    __shared__ int32_t ent[512];    // entry number of a leader (the first pick of a slot)
+    __shared__ int32_t size[512];   // rows of an entry, then its first row
+    __shared__ uint32_t wsum[16];
+    q4b_pdl_wait();
+    const uint32_t i = threadIdx.x, t = i >> 6, k = i & 63u, lane = i & 31u, warp = i >> 5;
     const bool valid = t < n_tok && (int32_t)k < nh[t];
-    slot[i] = valid ? es[i] : -1;
+    // exclusive prefix of a value over the block
+    auto prefix = [&](uint32_t v, uint32_t &total) {
+        uint32_t inc = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= (uint32_t)o) inc += x;
+        }
+        if (lane == 31u) wsum[warp] = inc;
+        __syncthreads();
+        uint32_t off = 0;
+        total = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 16u; j++) {
+            if (j < warp) off += wsum[j];
+            total += wsum[j];
+        }
+        __syncthreads();
+        return off + inc - v;
+    };
+    uint32_t n, n_ent, dummy;
+    const uint32_t c = prefix(valid ? 1u : 0u, n);
+    const int32_t mine = valid ? es[i] : -1;
+    if (valid) slot[c] = mine;
+    size[i] = 0;
     __syncthreads();
     int32_t first = -1, before = 0;
     if (valid) {
-        for (uint32_t j = 0; j < i; j++)
-            if (slot[j] == slot[i]) {
+        for (uint32_t j = 0; j < c; j++)
+            if (slot[j] == mine) {
                 if (first < 0) first = (int32_t)j;
                 before++;
             }
-        if (first < 0) first = (int32_t)i;
+        if (first < 0) first = (int32_t)c;
     }
-    lead[i] = first;
-    __syncthreads();
-    // entry number of leader i = number of leaders before it
-    int32_t my_ent = 0;
-    if (valid && first == (int32_t)i) {
-        for (uint32_t j = 0; j < i; j++) my_ent += lead[j] == (int32_t)j ? 1 : 0;
-        ent[i] = my_ent;
-        act[my_ent] = slot[i];
+    const bool leader = valid && first == (int32_t)c;
+    const uint32_t my_ent = prefix(leader ? 1u : 0u, n_ent);
+    if (leader) {
+        ent[c] = (int32_t)my_ent;
+        act[my_ent] = mine;
     }
-    size[i] = 0;
-    if (i == 0) size[512] = 0;
     __syncthreads();
     if (valid) atomicAdd(&size[ent[first]], 1);
     __syncthreads();
+    const uint32_t sz = (uint32_t)size[i], b = prefix(sz, dummy);
+    size[i] = (int32_t)b;
+    if (i < n_ent) bounds[i] = (int32_t)b;
     if (i == 0) {
-        int32_t n = 0, b = 0;
-        for (uint32_t j = 0; j < 512; j++) n += lead[j] == (int32_t)j ? 1 : 0;
-        for (int32_t j = 0; j < n; j++) {
-            bounds[j] = b;
-            b += size[j];
-            size[j] = bounds[j];   // becomes the entry's first row
-        }
-        bounds[n] = b;
-        *n_act = (uint32_t)n;
+        bounds[n_ent] = (int32_t)n;
+        *n_act = n_ent;
     }
     __syncthreads();
     if (valid) {
@@ -543,6 +579,7 @@ __global__ void __launch_bounds__(512) win_assign_k(
         rsrc[i] = -1;
         rw[i] = 0.f;
     }
+    if (i >= n) a_tok[i] = -1;
 }
 
 // The grouped product for IQ4_NL / IQ4_XS weights (type T; arenas in the engine's byte order): one
@@ -834,12 +871,8 @@ extern "C" bool q4_mmq_quantize(const float *x, const int32_t *ids, void *xq, ui
     if (w_type != Q4_T_IQ3_S && w_type != Q4_T_IQ4_NL && w_type != Q4_T_IQ4_XS) return false;
     const Q8View v = q8_view(xq, rows, cols);
     const uint64_t ngr = rows * (cols / 32u);
-    if (g_q8_compat)
-        quantize_rows_k<true><<<(unsigned)((ngr * 4 + 255) / 256), 256, 0, g_q4b.stream>>>(
-            x, ids, cols, rows, (int8_t *)v.q, (float *)v.d, (int32_t *)v.bs);
-    else
-        quantize_rows_k<false><<<(unsigned)((ngr * 4 + 255) / 256), 256, 0, g_q4b.stream>>>(
-            x, ids, cols, rows, (int8_t *)v.q, (float *)v.d, (int32_t *)v.bs);
+    q4b_launch(g_q8_compat ? quantize_rows_k<true> : quantize_rows_k<false>, (unsigned)((ngr * 4 + 255) / 256), 256, 0, g_q4b.stream,
+               x, ids, cols, rows, (int8_t *)v.q, (float *)v.d, (int32_t *)v.bs);
     g_q4b_launches++;
     return q4b_launch_ok("quantize_rows");
 }
@@ -887,12 +920,8 @@ extern "C" bool q4_cuda_mmq_swiglu_quantize(const float *gu, void *hq, uint64_t 
     if (!g_q4b.ok || !gu || !hq || rows == 0 || n_ff == 0 || (n_ff % 32u)) return false;
     const Q8View v = q8_view(hq, rows, n_ff);
     const uint64_t ngr = rows * (n_ff / 32u);
-    if (g_q8_compat)
-        swiglu_quant_rows_k<true><<<(unsigned)((ngr * 4 + 255) / 256), 256, 0, g_q4b.stream>>>(
-            gu, rows, n_ff, (int8_t *)v.q, (float *)v.d, (int32_t *)v.bs);
-    else
-        swiglu_quant_rows_k<false><<<(unsigned)((ngr * 4 + 255) / 256), 256, 0, g_q4b.stream>>>(
-            gu, rows, n_ff, (int8_t *)v.q, (float *)v.d, (int32_t *)v.bs);
+    q4b_launch(g_q8_compat ? swiglu_quant_rows_k<true> : swiglu_quant_rows_k<false>, (unsigned)((ngr * 4 + 255) / 256), 256, 0,
+               g_q4b.stream, gu, rows, n_ff, (int8_t *)v.q, (float *)v.d, (int32_t *)v.bs);
     g_q4b_launches++;
     return q4b_launch_ok("swiglu_quantize");
 }
@@ -930,10 +959,11 @@ static bool launch_assign(const int32_t *d_ids, const float *d_wts, int32_t *d_a
     const uint32_t n_g = (n_tok + gsz - 1u) / gsz;
     // a large group gets 32 warps (a histogram per warp: up to 34 x n_exp words of shared memory)
     const uint64_t rows = (uint64_t)(gsz < n_tok ? gsz : n_tok) * topk;
-    const uint32_t nt = rows > 4096u ? 1024u : 256u;
-    const size_t sm = ((nt / 32u + 2u) * n_exp + 48u) * sizeof(uint32_t);
+    // (a small one 16, so that a thread has one expert or two in the prefix; its histograms are for the warps with picks)
+    const uint32_t nt = rows > 4096u ? 1024u : 512u, nw = (uint32_t)(rows < nt ? (rows + 31u) / 32u : nt / 32u);
+    const size_t sm = ((nw + 2u) * n_exp + 48u) * sizeof(uint32_t);
     if (sm > ASSIGN_SMEM_MAX) return false;
-    assign_k<<<n_g, nt, sm, g_q4b.stream>>>(
+    q4b_launch(assign_k, n_g, nt, sm, g_q4b.stream,
         d_ids, d_wts, d_atok, d_rsrc, d_rw, d_stg, d_stgn, d_ek, d_cbounds, gsz, topk, n_exp, n_tok,
         ek_stride, topk_in ? topk_in : topk, extra_id, own_first, own_count, tok_first, tok_count,
         d_bounds_full);
@@ -1053,8 +1083,10 @@ extern "C" bool q4_cuda_moe_layer_nt(const uint8_t *base, uint64_t stride, uint3
     if ((gt != Q4_T_IQ3_S || dt != Q4_T_IQ3_S) && q4b_ptr_tiled(base)) return false;
     if (ou != og + (uint64_t)n_ff * grouped::row_bytes_t(gt, n_embd)) return false;  // gate|up contiguous
     if (shared_slot >= 0 && (uint32_t)shared_slot != n_expert) return false;  // shared = slot n_expert
-    const LayerWs w = carve((uint8_t *)d_ws, n_tok, topk, n_expert, n_embd, n_ff);
+    LayerWs w = carve((uint8_t *)d_ws, n_tok, topk, n_expert, n_embd, n_ff);
     if (ws_bytes < w.bytes) return false;
+    if (d_ids) w.ids = d_ids;   // the picks go straight where the caller wants them
+    if (d_wts) w.wts = d_wts;
     cudaStream_t st = g_q4b.stream;
     const bool sh = shared_slot >= 0;
     const uint32_t k1 = topk + (sh ? 1u : 0u), n_e = n_expert + (sh ? 1u : 0u);
@@ -1089,12 +1121,6 @@ extern "C" bool q4_cuda_moe_layer_nt(const uint8_t *base, uint64_t stride, uint3
                             q8_view(w.hq, rows, n_ff), rows, n_ff, n_embd, w.pd, n_embd, n_tok, dt))
         return false;
     if (!q4_cuda_expert_reduce_set(d_y, w.pd, w.rsrc, w.rw, n_tok, k1, n_embd)) return false;
-    if (d_ids && cudaMemcpyAsync(d_ids, w.ids, (uint64_t)n_tok * topk * 4, cudaMemcpyDeviceToDevice, st) !=
-                     cudaSuccess)
-        return false;
-    if (d_wts && cudaMemcpyAsync(d_wts, w.wts, (uint64_t)n_tok * topk * 4, cudaMemcpyDeviceToDevice, st) !=
-                     cudaSuccess)
-        return false;
     return true;
 }
 
@@ -1153,12 +1179,10 @@ extern "C" bool q4_hip_moe_exec_win(const uint8_t *base, uint64_t stride, const 
     int32_t *bounds = (int32_t *)take(514 * 4);
     void *xq = take(q8_bytes(rows, in_dim));
     float *gu = (float *)take(rows * 2 * n_ff * 4);
-    float *h = (float *)take(rows * n_ff * 4);
     void *hq = take(q8_bytes(rows, n_ff));
     float *pd = (float *)take(rows * n_embd * 4);
     if ((uint64_t)(p - g_win_ws) > g_win_ws_bytes) return false;
-    if (cudaMemsetAsync(atok, 0xff, rows * 4, st) != cudaSuccess) return false;  // -1: unplaced rows
-    win_assign_k<<<1, 512, 0, st>>>(d_es, d_ew, d_nh, n_tok, act, n_act, bounds, atok, rsrc, rw);
+    q4b_launch(win_assign_k, 1, 512, 0, st, d_es, d_ew, d_nh, n_tok, act, n_act, bounds, atok, rsrc, rw);
     g_q4b_launches++;
     if (!q4b_launch_ok("win_assign")) return false;
     const uint32_t n_pairs = n_tok * 64u;
@@ -1180,10 +1204,11 @@ extern "C" bool q4_hip_moe_exec_win(const uint8_t *base, uint64_t stride, const 
                                    gu + n_ff, 2ull * n_ff, n_tok, gt)) {
         return false;
     }
-    if (!q4_mmq_swiglu(gu, h, n_pairs, n_ff)) return false;
-    if (!q4_mmq_quantize(h, nullptr, hq, dt, n_ff, n_pairs)) return false;
+    if (!q4_cuda_mmq_swiglu_quantize(gu, hq, n_pairs, n_ff)) return false;
     if (!launch_grouped_any(base + od, stride, act, n_act, n_pairs, bounds, q8_view(hq, n_pairs, n_ff),
                             n_pairs, n_ff, n_embd, pd, n_embd, n_tok, dt))
         return false;
-    return q4_hip_expert_reduce(d_y, pd, rsrc, rw, n_tok, 64u, n_embd);
+    launch_expert_reduce<true>(d_y, pd, rsrc, rw, n_tok, 64u, n_embd, d_nh);
+    g_q4b_launches++;
+    return q4b_launch_ok("expert_reduce");
 }
