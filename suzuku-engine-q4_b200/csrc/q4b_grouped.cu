@@ -292,6 +292,87 @@ __global__ void swiglu_quant_rows_k(const float *__restrict__ gu, uint64_t rows,
     }
 }
 
+// Eight values of a row and their place in it, quantised and written as the tensor-core product's planes (what
+// quantize_rows_k or swiglu_quant_rows_k followed by mmqtc::planes_k<true> write, without the 8-bit rows in between:
+// 90,112 rows of 2048 took 167 + 218 us in two kernels).  All threads of the CTA call it; `per` threads (whole warps)
+// share row `sub` of the CTA.
+template <bool COMPAT>
+__device__ __forceinline__ void quant_planes(const float *v, bool live, uint32_t sub, uint32_t per, uint32_t c, __half *h1, __half *h2,
+                                             float *rs, float *red) {
+    float a = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) a = fmaxf(a, fabsf(v[i]));
+    a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 1));
+    a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 2));
+    const float sc = a > 0.f ? __fdiv_rn(127.f, a) : 0.f, d = q8_scale<COMPAT>(a, sc);
+    const float wm = q4b_warp_max(live ? d : 0.f);
+    if ((threadIdx.x & 31u) == 0) red[threadIdx.x >> 5] = wm;
+    __syncthreads();
+    float m = 0.f;
+    for (uint32_t i = 0; i < per >> 5; i++) m = fmaxf(m, red[sub * (per >> 5) + i]);
+    if (!live) return;
+    int e = 0;
+    if (m > 0.f) (void)frexpf(m * 127.f, &e);   // 127 d = the group's largest magnitude
+    const float s = d * ldexpf(1.f, -e);
+    if (c == 0) *rs = ldexpf(1.f, e);
+    uint32_t p1[4], p2[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {               // the order of planes_k<true>
+        const int j = 4 * (i & 1) + (i >> 1);
+        const float xa = (float)q8_round<COMPAT>(v[j], sc) * s, xb = (float)q8_round<COMPAT>(v[j + 2], sc) * s;
+        const __half2 a1 = __floats2half2_rn(xa, xb);
+        const float2 back = __half22float2(a1);
+        const __half2 a2 = __floats2half2_rn(xa - back.x, xb - back.y);
+        p1[i] = *reinterpret_cast<const uint32_t *>(&a1);
+        p2[i] = *reinterpret_cast<const uint32_t *>(&a2);
+    }
+    const uint32_t q = c >> 3, to = ((q & ~15u) | ((q & 3u) << 2) | ((q >> 2) & 3u)) << 3;
+    *reinterpret_cast<uint4 *>(h1 + to) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+    *reinterpret_cast<uint4 *>(h2 + to) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+}
+// Gathered rows -> planes, a CTA of n / 8 threads (whole warps, at most 512: n <= 4096, n % 256 == 0) per row.  (A row per
+// token, fetched by the product through TMA gathers of four rows, saves these writes and made the product 3.7 times
+// slower.)
+template <bool COMPAT>
+__global__ void __launch_bounds__(512) row_planes_k(const float *__restrict__ x, const int32_t *__restrict__ ids, uint32_t n,
+                                                    __half *__restrict__ h1, __half *__restrict__ h2, float *__restrict__ rs) {
+    __shared__ float red[16];
+    q4b_pdl_wait();
+    const int32_t src = __ldg(ids + blockIdx.x);
+    if (src < 0) return;    // a row that no expert owns
+    const uint32_t c = threadIdx.x * 8u;
+    const float4 *p = reinterpret_cast<const float4 *>(x + (uint64_t)src * n + c);
+    const float4 a = __ldg(p), b = __ldg(p + 1);
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    const uint64_t row = (uint64_t)blockIdx.x * n;
+    quant_planes<COMPAT>(v, true, 0, blockDim.x, c, h1 + row, h2 + row, rs + blockIdx.x, red);
+}
+// h = silu(g) * u and its planes: per = n_ff / 8 threads a row (n_ff % 256 == 0, n_ff <= 2048), 256 / per rows a CTA.
+template <bool COMPAT>
+__global__ void __launch_bounds__(256) swiglu_planes_k(const float *__restrict__ gu, uint64_t rows, uint32_t n_ff, uint32_t per,
+                                                       __half *__restrict__ h1, __half *__restrict__ h2,
+                                                       float *__restrict__ rs) {
+    __shared__ float red[8];
+    q4b_pdl_wait();
+    const uint32_t rpb = 256u / per, sub = threadIdx.x / per, c = (threadIdx.x - sub * per) * 8u;
+    const uint64_t r = (uint64_t)blockIdx.x * rpb + sub;
+    const bool live = sub < rpb && r < rows;
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = 0.f;
+    if (live) {
+        const float4 *pg = reinterpret_cast<const float4 *>(gu + r * 2 * n_ff + c);
+        const float4 *pu = reinterpret_cast<const float4 *>(gu + r * 2 * n_ff + n_ff + c);
+        const float4 g0 = __ldcs(pg), g1 = __ldcs(pg + 1), u0 = __ldcs(pu), u1 = __ldcs(pu + 1);
+        v[0] = q4b_swiglu(g0.x, u0.x), v[1] = q4b_swiglu(g0.y, u0.y);
+        v[2] = q4b_swiglu(g0.z, u0.z), v[3] = q4b_swiglu(g0.w, u0.w);
+        v[4] = q4b_swiglu(g1.x, u1.x), v[5] = q4b_swiglu(g1.y, u1.y);
+        v[6] = q4b_swiglu(g1.z, u1.z), v[7] = q4b_swiglu(g1.w, u1.w);
+    }
+    // (256 % per threads at the end of the CTA have no row)
+    quant_planes<COMPAT>(v, live, min(sub, rpb - 1u), per, c, h1 + r * n_ff, h2 + r * n_ff, rs + r, red);
+}
+
 // y[t][c] (+)= sum_k rw[t][k] * pd[rsrc[t][k]][c], picks in order k = 0..topk-1; ADD = false
 // overwrites y (same value as adding to a zeroed y).
 template <bool ADD>
@@ -498,6 +579,141 @@ __global__ void __launch_bounds__(1024) assign_k(
         }
         __syncwarp();
         if (e >= 0 && (same & ((1u << lane) - 1u)) == 0) hist[warp * n_exp + e] += __popc(same);
+        __syncwarp();
+    }
+}
+
+// The same assignment for a layer of many tokens (one group, every expert's picks): chunks of ASSIGN_CHUNK picks, a CTA
+// each.  hist: [chunks][n_exp] words of scratch -- counts, then (after the scan) the first row of each chunk's picks of an
+// expert.  90,112 picks: 36 us for the three kernels; one CTA for all of it took 216.
+constexpr uint32_t ASSIGN_CHUNK = 1024;
+__device__ __forceinline__ int32_t layer_pick(const int32_t *ids, uint32_t i, uint32_t topk, uint32_t topk_in, int32_t extra_id,
+                                              uint32_t n_exp) {
+    const uint32_t t = i / topk, k = i - t * topk;
+    const int32_t e = k >= topk_in ? extra_id : ids[(uint64_t)t * topk_in + k];
+    return e < 0 || (uint32_t)e >= n_exp ? -1 : e;
+}
+__global__ void __launch_bounds__(256) assign_count_k(const int32_t *__restrict__ ids, uint32_t rows, uint32_t topk,
+                                                      uint32_t topk_in, int32_t extra_id, uint32_t n_exp,
+                                                      uint32_t *__restrict__ hist) {
+    extern __shared__ uint32_t sh[];
+    q4b_pdl_wait();
+    for (uint32_t e = threadIdx.x; e < n_exp; e += 256u) sh[e] = 0;
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+    for (uint32_t j = 0; j < ASSIGN_CHUNK / 256u; j++) {
+        const uint32_t i = blockIdx.x * ASSIGN_CHUNK + j * 256u + threadIdx.x;
+        const int32_t e = i < rows ? layer_pick(ids, i, topk, topk_in, extra_id, n_exp) : -1;
+        const uint32_t same = __match_any_sync(0xffffffffu, e);
+        if (e >= 0 && (same & ((1u << lane) - 1u)) == 0) atomicAdd(sh + e, (uint32_t)__popc(same));
+    }
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < n_exp; e += 256u) hist[(uint64_t)blockIdx.x * n_exp + e] = sh[e];
+}
+__global__ void __launch_bounds__(1024) assign_scan_k(uint32_t *__restrict__ hist, uint32_t chunks, uint32_t n_exp, uint32_t rows,
+                                                      int32_t *__restrict__ stg, uint32_t *__restrict__ stgn,
+                                                      int32_t *__restrict__ cbounds, int32_t *__restrict__ a_tok) {
+    __shared__ uint32_t wsum[32];
+    q4b_pdl_wait();
+    const uint32_t e = threadIdx.x, lane = e & 31u, warp = e >> 5;   // n_exp <= 1024: a thread an expert
+    uint32_t tot = 0;
+    if (e < n_exp)
+        for (uint32_t c0 = 0; c0 < chunks; c0 += 16u) {
+            uint32_t v[16];
+#pragma unroll
+            for (uint32_t i = 0; i < 16; i++) v[i] = c0 + i < chunks ? hist[(uint64_t)(c0 + i) * n_exp + e] : 0u;
+#pragma unroll
+            for (uint32_t i = 0; i < 16; i++) tot += v[i];
+        }
+    // exclusive prefixes of the rows and of the used experts
+    uint32_t ic = tot, iu = tot ? 1u : 0u;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, ic, o), y = __shfl_up_sync(0xffffffffu, iu, o);
+        if (lane >= (uint32_t)o) ic += x, iu += y;
+    }
+    uint32_t off[2] = {0, 0}, all[2] = {0, 0};
+#pragma unroll
+    for (int pass = 0; pass < 2; pass++) {
+        if (lane == 31u) wsum[warp] = pass ? iu : ic;
+        __syncthreads();
+        for (uint32_t j = 0; j < 32u; j++) {
+            if (j < warp) off[pass] += wsum[j];
+            all[pass] += wsum[j];
+        }
+        __syncthreads();
+    }
+    uint32_t b = off[0] + ic - tot;
+    if (tot) {
+        const uint32_t u = off[1] + iu - 1u;
+        stg[u] = (int32_t)e;
+        cbounds[u] = (int32_t)b;
+    }
+    if (e == 0) {
+        cbounds[all[1]] = (int32_t)all[0];
+        *stgn = all[1];
+    }
+    if (e < n_exp)
+        for (uint32_t c0 = 0; c0 < chunks; c0 += 16u) {
+            uint32_t v[16];
+#pragma unroll
+            for (uint32_t i = 0; i < 16; i++) v[i] = c0 + i < chunks ? hist[(uint64_t)(c0 + i) * n_exp + e] : 0u;
+#pragma unroll
+            for (uint32_t i = 0; i < 16; i++)
+                if (c0 + i < chunks) {
+                    hist[(uint64_t)(c0 + i) * n_exp + e] = b;
+                    b += v[i];
+                }
+        }
+    for (uint32_t i = all[0] + e; i < rows; i += 1024u) a_tok[i] = -1;   // unused rows
+}
+__global__ void __launch_bounds__(256) assign_place_k(const int32_t *__restrict__ ids, const float *__restrict__ wts, uint32_t rows,
+                                                      uint32_t topk, uint32_t topk_in, int32_t extra_id, uint32_t n_exp,
+                                                      const uint32_t *__restrict__ hist, int32_t *__restrict__ a_tok,
+                                                      int32_t *__restrict__ rsrc, float *__restrict__ rw) {
+    extern __shared__ uint32_t sh[];   // [8 warps][n_exp]: next row of the warp's picks of an expert
+    q4b_pdl_wait();
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    constexpr uint32_t PER = ASSIGN_CHUNK / 256u;   // picks of a lane; a warp's are a contiguous run
+    for (uint32_t i = threadIdx.x; i < 8u * n_exp; i += 256u) sh[i] = 0;
+    __syncthreads();
+    int32_t e[PER];
+    uint32_t same[PER];
+#pragma unroll
+    for (uint32_t j = 0; j < PER; j++) {
+        const uint32_t i = blockIdx.x * ASSIGN_CHUNK + warp * (32u * PER) + j * 32u + lane;
+        e[j] = i < rows ? layer_pick(ids, i, topk, topk_in, extra_id, n_exp) : -1;
+        same[j] = __match_any_sync(0xffffffffu, e[j]);
+        if (e[j] >= 0 && (same[j] & ((1u << lane) - 1u)) == 0) sh[warp * n_exp + e[j]] += __popc(same[j]);
+        __syncwarp();
+    }
+    __syncthreads();
+    for (uint32_t x = threadIdx.x; x < n_exp; x += 256u) {
+        uint32_t b = hist[(uint64_t)blockIdx.x * n_exp + x];
+#pragma unroll
+        for (uint32_t w = 0; w < 8u; w++) {
+            const uint32_t c = sh[w * n_exp + x];
+            sh[w * n_exp + x] = b;
+            b += c;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t j = 0; j < PER; j++) {
+        const uint32_t i = blockIdx.x * ASSIGN_CHUNK + warp * (32u * PER) + j * 32u + lane;
+        const uint32_t t = i / topk, k = i - t * topk;
+        if (e[j] >= 0) {
+            const uint32_t pos = sh[warp * n_exp + e[j]] + __popc(same[j] & ((1u << lane) - 1u));
+            a_tok[pos] = (int32_t)t;
+            rsrc[i] = (int32_t)pos;
+            rw[i] = k < topk_in ? wts[(uint64_t)t * topk_in + k] : 1.0f;
+        } else if (i < rows) {
+            rsrc[i] = -1;
+            rw[i] = 0.f;
+        }
+        __syncwarp();
+        if (e[j] >= 0 && (same[j] & ((1u << lane) - 1u)) == 0) sh[warp * n_exp + e[j]] += __popc(same[j]);
         __syncwarp();
     }
 }
@@ -729,6 +945,12 @@ constexpr uint32_t TC_MIN_ROWS = 12;
 // 370 experts, gate/up + down, us: 16 rows 161 + 87 streamed, 17 rows 262 + 138, 20 rows 293 + 154 (two passes over the
 // weights), 32 rows 299 + 156; on the tensor cores 266 + 157, 264 + 160, 269 + 162, 283 + 165, and 338 + 190 with 64 rows.
 constexpr uint32_t WIDE_TC_ROWS = 20;
+// Does the tensor-core product on the wide form take a call of IQ3_S weights?
+bool takes_wide_tc(const uint8_t *w, uint64_t expert_stride, uint32_t n_entries, uint64_t total_rows, uint32_t cols, uint32_t w_rows) {
+    return g_tc_mode != 0 && g_tc_mode != 2 && q4b_ptr_tiled(w) &&
+           mmqtc::wide_ok(w, expert_stride, total_rows, w_rows, cols, n_entries) &&
+           (g_tc_mode == 1 || total_rows >= (uint64_t)WIDE_TC_ROWS * n_entries);
+}
 bool launch_grouped_any(const uint8_t *w, uint64_t expert_stride, const int32_t *act,
                         const uint32_t *n_act, uint32_t n_entries, const int32_t *bounds, Q8View xq,
                         uint64_t total_rows, uint32_t cols, uint32_t w_rows, float *dst,
@@ -745,13 +967,10 @@ bool launch_grouped_any(const uint8_t *w, uint64_t expert_stride, const int32_t 
     const bool wide_ok = g_tc_mode != 2 && g_tc_mode != 1 && tiled && wide::shape_ok(w, expert_stride, w_rows, cols, n_entries);
     // On the wide form one kernel takes the whole call: the tensor-core kernel from an average of
     // WIDE_TC_ROWS rows per possible entry on (or in mode 1), the streaming kernel below.
-    if (tiled && tc_ok && mmqtc::wide_ok(w, expert_stride, total_rows, w_rows, cols, n_entries) &&
-        (g_tc_mode == 1 || (wide_ok && total_rows >= (uint64_t)WIDE_TC_ROWS * n_entries))) {
-        const bool ok = mmqtc::launch_wide(w, expert_stride, act, n_act, n_entries, bounds, xq.q, xq.d, xq.h1, xq.h2, xq.rs,
-                                           total_rows, cols, w_rows, dst, ld_dst);
-        g_q4b_launches += 3;
-        return ok && q4b_launch_ok("mmq_wide");
-    }
+    if (takes_wide_tc(w, expert_stride, n_entries, total_rows, cols, w_rows))
+        return mmqtc::launch_planes_wide(xq.q, xq.d, xq.h1, xq.h2, xq.rs, total_rows, cols) &&
+               mmqtc::launch_wide(w, expert_stride, act, n_act, n_entries, bounds, xq.h1, xq.h2, xq.rs, total_rows, cols, w_rows, dst,
+                                  ld_dst);
     if (wide_ok) {
         const bool ok = wide::launch(stream_args(w, expert_stride, act, n_act, n_entries, bounds, xq, cols, w_rows, dst, ld_dst));
         g_q4b_launches++;
@@ -1102,24 +1321,56 @@ extern "C" bool q4_cuda_moe_layer_nt(const uint8_t *base, uint64_t stride, uint3
         if (!q4b_route_tokens(w.logits, w.ids, w.wts, n_tok, n_expert, topk)) return false;
     }
     // the shared expert is one more pick (id n_expert, weight 1) of every token, added on the fly
-    if (!launch_assign(w.ids, w.wts, w.atok, w.rsrc, w.rw, w.stg, w.stgn, nullptr, w.cbounds, n_tok, k1,
-                       n_e, n_tok, n_e, topk, sh ? (int32_t)n_expert : -1))
+    if (rows > 4096u) {
+        const uint32_t chunks = (uint32_t)((rows + ASSIGN_CHUNK - 1u) / ASSIGN_CHUNK);
+        uint32_t *hist = (uint32_t *)w.ids2;   // two sections of `rows` words: chunks * n_e <= rows + 1024 of them are used
+        q4b_launch(assign_count_k, chunks, 256, n_e * 4u, st, w.ids, (uint32_t)rows, k1, topk, (int32_t)n_expert, n_e, hist);
+        q4b_launch(assign_scan_k, 1, 1024, 0, st, hist, chunks, n_e, (uint32_t)rows, w.stg, w.stgn, w.cbounds, w.atok);
+        q4b_launch(assign_place_k, chunks, 256, 8u * n_e * 4u, st, w.ids, w.wts, (uint32_t)rows, k1, topk, (int32_t)n_expert, n_e, hist,
+                   w.atok, w.rsrc, w.rw);
+        g_q4b_launches += 3;
+        if (!q4b_launch_ok("assign")) return false;
+    } else if (!launch_assign(w.ids, w.wts, w.atok, w.rsrc, w.rw, w.stg, w.stgn, nullptr, w.cbounds, n_tok, k1,
+                              n_e, n_tok, n_e, topk, sh ? (int32_t)n_expert : -1)) {
         return false;
-    if (!q4_mmq_quantize(w.xn, w.atok, w.xq, gt, n_embd, rows)) return false;
-    if (gt == Q4_T_IQ3_S && !grouped::pow2_blocks(n_embd) &&
-        cudaMemsetAsync(w.gu, 0, rows * 2 * n_ff * 4, st) != cudaSuccess)
-        return false;
-    if (!launch_grouped_any(base + og, stride, w.stg, w.stgn, n_entries, w.cbounds,
-                            q8_view(w.xq, rows, n_embd), rows, n_embd, 2u * n_ff, w.gu, 2ull * n_ff,
-                            n_tok, gt))
-        return false;
-    if (!q4_cuda_mmq_swiglu_quantize(w.gu, w.hq, rows, n_ff)) return false;
-    if (dt == Q4_T_IQ3_S && !grouped::pow2_blocks(n_ff) &&
-        cudaMemsetAsync(w.pd, 0, rows * n_embd * 4, st) != cudaSuccess)
-        return false;
-    if (!launch_grouped_any(base + od, stride, w.stg, w.stgn, n_entries, w.cbounds,
-                            q8_view(w.hq, rows, n_ff), rows, n_ff, n_embd, w.pd, n_embd, n_tok, dt))
-        return false;
+    }
+    // A product that runs on the tensor cores and the wide form gets its activations as planes at once.
+    const Q8View xv = q8_view(w.xq, rows, n_embd), hv = q8_view(w.hq, rows, n_ff);
+    if (gt == Q4_T_IQ3_S && n_embd <= 4096u && takes_wide_tc(base + og, stride, n_entries, rows, n_embd, 2u * n_ff)) {
+        q4b_launch(g_q8_compat ? row_planes_k<true> : row_planes_k<false>, (unsigned)rows, n_embd / 8u, 0, st, w.xn, w.atok, n_embd,
+                   xv.h1, xv.h2, xv.rs);
+        g_q4b_launches++;
+        if (!q4b_launch_ok("row_planes") ||
+            !mmqtc::launch_wide(base + og, stride, w.stg, w.stgn, n_entries, w.cbounds, xv.h1, xv.h2, xv.rs, rows, n_embd, 2u * n_ff,
+                                w.gu, 2ull * n_ff))
+            return false;
+    } else {
+        if (!q4_mmq_quantize(w.xn, w.atok, w.xq, gt, n_embd, rows)) return false;
+        if (gt == Q4_T_IQ3_S && !grouped::pow2_blocks(n_embd) &&
+            cudaMemsetAsync(w.gu, 0, rows * 2 * n_ff * 4, st) != cudaSuccess)
+            return false;
+        if (!launch_grouped_any(base + og, stride, w.stg, w.stgn, n_entries, w.cbounds, xv, rows, n_embd, 2u * n_ff, w.gu,
+                                2ull * n_ff, n_tok, gt))
+            return false;
+    }
+    if (dt == Q4_T_IQ3_S && n_ff <= 2048u && takes_wide_tc(base + od, stride, n_entries, rows, n_ff, n_embd)) {
+        const uint32_t per = n_ff / 8u, rpb = 256u / per;
+        q4b_launch(g_q8_compat ? swiglu_planes_k<true> : swiglu_planes_k<false>, (unsigned)((rows + rpb - 1u) / rpb), 256, 0, st, w.gu,
+                   rows, n_ff, per, hv.h1, hv.h2, hv.rs);
+        g_q4b_launches++;
+        if (!q4b_launch_ok("swiglu_planes") ||
+            !mmqtc::launch_wide(base + od, stride, w.stg, w.stgn, n_entries, w.cbounds, hv.h1, hv.h2, hv.rs, rows, n_ff, n_embd, w.pd,
+                                n_embd))
+            return false;
+    } else {
+        if (!q4_cuda_mmq_swiglu_quantize(w.gu, w.hq, rows, n_ff)) return false;
+        if (dt == Q4_T_IQ3_S && !grouped::pow2_blocks(n_ff) &&
+            cudaMemsetAsync(w.pd, 0, rows * n_embd * 4, st) != cudaSuccess)
+            return false;
+        if (!launch_grouped_any(base + od, stride, w.stg, w.stgn, n_entries, w.cbounds, hv, rows, n_ff, n_embd, w.pd, n_embd, n_tok,
+                                dt))
+            return false;
+    }
     if (!q4_cuda_expert_reduce_set(d_y, w.pd, w.rsrc, w.rw, n_tok, k1, n_embd)) return false;
     return true;
 }

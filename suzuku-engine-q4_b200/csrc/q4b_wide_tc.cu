@@ -21,6 +21,9 @@
 //     evenly over its passes
 #include "q4b_tile.cuh"
 
+#include <atomic>
+
+extern std::atomic<uint64_t> g_q4b_launches;
 const uint8_t *q4b_wide_of(const void *p);
 
 namespace mmqtc {
@@ -74,6 +77,7 @@ __global__ void __launch_bounds__(1024) worklist_wide_k(const int32_t *__restric
                                                         uint4 *__restrict__ work,
                                                         uint32_t *__restrict__ n_work, uint32_t cap) {
     __shared__ uint32_t wsum[32];
+    q4b_pdl_wait();
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t n_ent = n_act ? min(*n_act, n_entries) : n_entries;
     uint32_t base = 0;
@@ -181,6 +185,7 @@ __global__ void __launch_bounds__(NT, 1) mmq_wide_k(const WArgs a, const __grid_
     uint8_t *const sb_base = smem_raw + W_B_OFF;
     constexpr uint32_t stage_bytes = W_STAGE_BYTES;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    q4b_pdl_wait();
     const uint32_t B = a.cols >> 8, n_it = a.cols / KS, n_s = n_it * a.mt;   // steps of a tile, of an item
     const uint32_t n_all = *a.n_work * a.groups;
     if (blockIdx.x >= n_all) return;
@@ -489,9 +494,10 @@ bool wide_ok(const uint8_t *w, uint64_t stride, uint64_t rows, uint64_t w_rows, 
     return g_wide_ready && shape_ok(w_rows, w_cols) && (stride % Q4B_TILE_BYTES) == 0 && rows < 0x7fffffffull &&
            (uint64_t)n_entries + rows / W_NB <= WORK_CAP && q4b_wide_of(w);
 }
+// h1, h2, rs: the rows' planes, as planes_k<true> writes them.
 bool launch_wide(const uint8_t *w, uint64_t expert_stride, const int32_t *act, const uint32_t *n_act, uint32_t n_entries,
-                 const int32_t *bounds, const int8_t *q, const float *dq, __half *h1, __half *h2, float *rs, uint64_t rows,
-                 uint32_t cols, uint32_t w_rows, float *dst, uint64_t ld_dst) {
+                 const int32_t *bounds, const __half *h1, const __half *h2, const float *rs, uint64_t rows, uint32_t cols,
+                 uint32_t w_rows, float *dst, uint64_t ld_dst) {
     WArgs a = {};
     a.w = q4b_wide_of(w);
     if (!a.w) return false;
@@ -514,13 +520,9 @@ bool launch_wide(const uint8_t *w, uint64_t expert_stride, const int32_t *act, c
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return false;
     }
-    {
-        const uint32_t tpr = cols / 8u < 256u ? cols / 8u : 256u, rpb = 256u / tpr;
-        planes_k<true><<<(unsigned)((rows + rpb - 1) / rpb), 256, 0, g_q4b.stream>>>(q, dq, rows, cols, tpr, h1, h2, rs);
-    }
     const uint32_t turn = g_wturn++ & 1u;
-    worklist_wide_k<<<1, 1024, 0, g_q4b.stream>>>(bounds, n_act, n_entries, g_wwork + turn * WORK_CAP,
-                                                  g_wn_work + turn, WORK_CAP);
+    q4b_launch(worklist_wide_k, 1, 1024, 0, g_q4b.stream, bounds, n_act, n_entries, g_wwork + turn * WORK_CAP, g_wn_work + turn,
+               WORK_CAP);
     a.work = g_wwork + turn * WORK_CAP;
     a.n_work = g_wn_work + turn;
     // about 16 steps an item, as many tiles as that takes
@@ -529,8 +531,16 @@ bool launch_wide(const uint8_t *w, uint64_t expert_stride, const int32_t *act, c
     for (uint32_t c = 1; c <= n_tiles && c * n_it <= 16u; c++)
         if (n_tiles % c == 0) a.mt = c;
     a.groups = n_tiles / a.mt;
-    mmq_wide_k<<<g_q4b.n_sm, NT, W_SMEM, g_q4b.stream>>>(a, maps[0], maps[1]);
-    return true;
+    q4b_launch(mmq_wide_k, g_q4b.n_sm, NT, W_SMEM, g_q4b.stream, a, maps[0], maps[1]);
+    g_q4b_launches += 2;
+    return q4b_launch_ok("mmq_wide");
+}
+// The planes of quantised rows.
+bool launch_planes_wide(const int8_t *q, const float *dq, __half *h1, __half *h2, float *rs, uint64_t rows, uint32_t cols) {
+    const uint32_t tpr = cols / 8u < 256u ? cols / 8u : 256u, rpb = 256u / tpr;
+    planes_k<true><<<(unsigned)((rows + rpb - 1) / rpb), 256, 0, g_q4b.stream>>>(q, dq, rows, cols, tpr, h1, h2, rs);
+    g_q4b_launches++;
+    return q4b_launch_ok("planes");
 }
 
 }  // namespace mmqtc
