@@ -77,6 +77,14 @@ template <bool COMPAT> __device__ __forceinline__ int q8_round(float v, float sc
     const float t = __fmul_rn(v, sc);
     return max(-128, min(127, COMPAT ? (int)roundf(t) : __float2int_rn(t)));
 }
+// The same value as a float, in fewer instructions: the conversion to s8 saturates, and an integer added to the bits of
+// 1.5 * 2^23 is a float.
+template <bool COMPAT> __device__ __forceinline__ float q8_round_f(float v, float sc) {
+    if (COMPAT) return (float)q8_round<true>(v, sc);
+    int q;
+    asm("{\n\t.reg .s8 b;\n\tcvt.rni.sat.s8.f32 b, %1;\n\tcvt.s32.s8 %0, b;\n\t}" : "=r"(q) : "f"(__fmul_rn(v, sc)));
+    return __int_as_float(0x4b400000 + q) - 12582912.f;
+}
 template <bool COMPAT> __device__ __forceinline__ float q8_scale(float amax, float sc) {
     return COMPAT ? (sc > 0.f ? __fdiv_rn(1.0f, sc) : 0.f) : __fdiv_rn(amax, 127.f);
 }
@@ -319,7 +327,7 @@ __device__ __forceinline__ void quant_planes(const float *v, bool live, uint32_t
 #pragma unroll
     for (int i = 0; i < 4; i++) {               // the order of planes_k<true>
         const int j = 4 * (i & 1) + (i >> 1);
-        const float xa = (float)q8_round<COMPAT>(v[j], sc) * s, xb = (float)q8_round<COMPAT>(v[j + 2], sc) * s;
+        const float xa = q8_round_f<COMPAT>(v[j], sc) * s, xb = q8_round_f<COMPAT>(v[j + 2], sc) * s;
         const __half2 a1 = __floats2half2_rn(xa, xb);
         const float2 back = __half22float2(a1);
         const __half2 a2 = __floats2half2_rn(xa - back.x, xb - back.y);
@@ -330,22 +338,71 @@ __device__ __forceinline__ void quant_planes(const float *v, bool live, uint32_t
     *reinterpret_cast<uint4 *>(h1 + to) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
     *reinterpret_cast<uint4 *>(h2 + to) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
 }
-// Gathered rows -> planes, a CTA of n / 8 threads (whole warps, at most 512: n <= 4096, n % 256 == 0) per row.  (A row per
-// token, fetched by the product through TMA gathers of four rows, saves these writes and made the product 3.7 times
-// slower.)
+// RMSNorm of a token's row and its planes, a CTA of n / 8 threads (whole warps, at most 512: n <= 4096, n % 256 == 0) per
+// token: x is read once, the normalised row (for the router) and the planes written once.
 template <bool COMPAT>
-__global__ void __launch_bounds__(512) row_planes_k(const float *__restrict__ x, const int32_t *__restrict__ ids, uint32_t n,
-                                                    __half *__restrict__ h1, __half *__restrict__ h2, float *__restrict__ rs) {
+__global__ void __launch_bounds__(512) norm_planes_k(const float *__restrict__ x, const float *__restrict__ w, float eps, uint32_t n,
+                                                     float *__restrict__ xn, __half *__restrict__ h1,
+                                                     __half *__restrict__ h2, float *__restrict__ rs) {
+    __shared__ double sh[16];
     __shared__ float red[16];
     q4b_pdl_wait();
-    const int32_t src = __ldg(ids + blockIdx.x);
-    if (src < 0) return;    // a row that no expert owns
     const uint32_t c = threadIdx.x * 8u;
-    const float4 *p = reinterpret_cast<const float4 *>(x + (uint64_t)src * n + c);
-    const float4 a = __ldg(p), b = __ldg(p + 1);
-    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     const uint64_t row = (uint64_t)blockIdx.x * n;
+    const float4 a = *reinterpret_cast<const float4 *>(x + row + c), b = *reinterpret_cast<const float4 *>(x + row + c + 4u);
+    float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, g[8];
+    if (w) {
+        const float4 ga = __ldg(reinterpret_cast<const float4 *>(w + c)), gb = __ldg(reinterpret_cast<const float4 *>(w + c + 4u));
+        g[0] = ga.x, g[1] = ga.y, g[2] = ga.z, g[3] = ga.w, g[4] = gb.x, g[5] = gb.y, g[6] = gb.z, g[7] = gb.w;
+    }
+    double ss = 0.0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) ss += (double)v[i] * (double)v[i];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((threadIdx.x & 31u) == 0) sh[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    double tot = 0.0;
+    for (uint32_t i = 0; i < (blockDim.x >> 5); i++) tot += sh[i];
+    const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn((float)(tot / (double)n), eps)));
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        v[i] = __fmul_rn(v[i], scale);
+        if (w) v[i] = __fmul_rn(v[i], g[i]);
+    }
+    *reinterpret_cast<float4 *>(xn + row + c) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4 *>(xn + row + c + 4u) = make_float4(v[4], v[5], v[6], v[7]);
     quant_planes<COMPAT>(v, true, 0, blockDim.x, c, h1 + row, h2 + row, rs + blockIdx.x, red);
+}
+// The planes of the picks' rows, copied from their tokens' planes: four rows a CTA, n / 8 threads a row, all its loads in
+// flight.  Bound by the bytes (8 n a row in and out).  (Quantising every pick's row anew took 231 us for 90,112 rows of
+// 2048.  Leaving the copies out and fetching the tokens' rows by TMA gathers of four made the product 3.7 times slower.)
+__global__ void __launch_bounds__(512) gather_planes_k(const __half *__restrict__ t1, const __half *__restrict__ t2,
+                                                       const float *__restrict__ trs, const int32_t *__restrict__ ids, uint32_t rows,
+                                                       uint32_t n, __half *__restrict__ h1, __half *__restrict__ h2,
+                                                       float *__restrict__ rs) {
+    q4b_pdl_wait();
+    const uint32_t r0 = blockIdx.x * 4u, c = threadIdx.x * 8u;
+    int32_t src[4];
+    uint4 a[4], b[4];
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) src[i] = r0 + i < rows ? __ldg(ids + r0 + i) : -1;   // -1: a row that no expert owns
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++)
+        if (src[i] >= 0) {
+            a[i] = __ldg(reinterpret_cast<const uint4 *>(t1 + (uint64_t)src[i] * n + c));
+            b[i] = __ldg(reinterpret_cast<const uint4 *>(t2 + (uint64_t)src[i] * n + c));
+        }
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++)
+        if (src[i] >= 0) {
+            __stcs(reinterpret_cast<uint4 *>(h1 + (uint64_t)(r0 + i) * n + c), a[i]);
+            __stcs(reinterpret_cast<uint4 *>(h2 + (uint64_t)(r0 + i) * n + c), b[i]);
+        }
+    if (threadIdx.x < 4u && r0 + threadIdx.x < rows) {
+        const int32_t s = __ldg(ids + r0 + threadIdx.x);
+        if (s >= 0) rs[r0 + threadIdx.x] = __ldg(trs + s);
+    }
 }
 // h = silu(g) * u and its planes: per = n_ff / 8 threads a row (n_ff % 256 == 0, n_ff <= 2048), 256 / per rows a CTA.
 template <bool COMPAT>
@@ -585,7 +642,7 @@ __global__ void __launch_bounds__(1024) assign_k(
 
 // The same assignment for a layer of many tokens (one group, every expert's picks): chunks of ASSIGN_CHUNK picks, a CTA
 // each.  hist: [chunks][n_exp] words of scratch -- counts, then (after the scan) the first row of each chunk's picks of an
-// expert.  90,112 picks: 36 us for the three kernels; one CTA for all of it took 216.
+// expert.  90,112 picks: 43 us for the three kernels; one CTA for all of it took 216.
 constexpr uint32_t ASSIGN_CHUNK = 1024;
 __device__ __forceinline__ int32_t layer_pick(const int32_t *ids, uint32_t i, uint32_t topk, uint32_t topk_in, int32_t extra_id,
                                               uint32_t n_exp) {
@@ -619,12 +676,12 @@ __global__ void __launch_bounds__(1024) assign_scan_k(uint32_t *__restrict__ his
     const uint32_t e = threadIdx.x, lane = e & 31u, warp = e >> 5;   // n_exp <= 1024: a thread an expert
     uint32_t tot = 0;
     if (e < n_exp)
-        for (uint32_t c0 = 0; c0 < chunks; c0 += 16u) {
-            uint32_t v[16];
+        for (uint32_t c0 = 0; c0 < chunks; c0 += 8u) {
+            uint32_t v[8];
 #pragma unroll
-            for (uint32_t i = 0; i < 16; i++) v[i] = c0 + i < chunks ? hist[(uint64_t)(c0 + i) * n_exp + e] : 0u;
+            for (uint32_t i = 0; i < 8; i++) v[i] = c0 + i < chunks ? hist[(uint64_t)(c0 + i) * n_exp + e] : 0u;
 #pragma unroll
-            for (uint32_t i = 0; i < 16; i++) tot += v[i];
+            for (uint32_t i = 0; i < 8; i++) tot += v[i];
         }
     // exclusive prefixes of the rows and of the used experts
     uint32_t ic = tot, iu = tot ? 1u : 0u;
@@ -655,12 +712,12 @@ __global__ void __launch_bounds__(1024) assign_scan_k(uint32_t *__restrict__ his
         *stgn = all[1];
     }
     if (e < n_exp)
-        for (uint32_t c0 = 0; c0 < chunks; c0 += 16u) {
-            uint32_t v[16];
+        for (uint32_t c0 = 0; c0 < chunks; c0 += 8u) {
+            uint32_t v[8];
 #pragma unroll
-            for (uint32_t i = 0; i < 16; i++) v[i] = c0 + i < chunks ? hist[(uint64_t)(c0 + i) * n_exp + e] : 0u;
+            for (uint32_t i = 0; i < 8; i++) v[i] = c0 + i < chunks ? hist[(uint64_t)(c0 + i) * n_exp + e] : 0u;
 #pragma unroll
-            for (uint32_t i = 0; i < 16; i++)
+            for (uint32_t i = 0; i < 8; i++)
                 if (c0 + i < chunks) {
                     hist[(uint64_t)(c0 + i) * n_exp + e] = b;
                     b += v[i];
@@ -1311,10 +1368,22 @@ extern "C" bool q4_cuda_moe_layer_nt(const uint8_t *base, uint64_t stride, uint3
     const uint32_t k1 = topk + (sh ? 1u : 0u), n_e = n_expert + (sh ? 1u : 0u);
     const uint64_t rows = (uint64_t)n_tok * k1;
     const uint32_t n_entries = (uint32_t)(rows < n_e ? rows : n_e);  // used experts <= rows
+    // Products that run on the tensor cores and the wide form get their activations as planes at once.  The tokens' planes
+    // lie where the down product's rows will be, their row scales in the space of the hidden rows.
+    const bool gu_tc = gt == Q4_T_IQ3_S && n_embd <= 4096u && takes_wide_tc(base + og, stride, n_entries, rows, n_embd, 2u * n_ff) &&
+                       (((uintptr_t)d_x | (uintptr_t)d_norm_w) & 15u) == 0;
+    const bool dn_tc = dt == Q4_T_IQ3_S && n_ff <= 2048u && takes_wide_tc(base + od, stride, n_entries, rows, n_ff, n_embd);
+    __half *const t1 = (__half *)w.pd, *const t2 = t1 + (uint64_t)n_tok * n_embd;
     // up to 256 tokens: norm, router and top-k as one launch (same values); else the three launches
-    if (!q4b_route_small(d_x, d_norm_w, eps, d_router, n_expert, topk, n_embd, n_tok, w.xn, w.logits, w.ids,
-                         w.wts)) {
-        if (!q4b_rms_rows(d_x, d_norm_w, w.xn, n_embd, eps, n_tok)) return false;
+    if (gu_tc || !q4b_route_small(d_x, d_norm_w, eps, d_router, n_expert, topk, n_embd, n_tok, w.xn, w.logits, w.ids, w.wts)) {
+        if (gu_tc) {
+            q4b_launch(g_q8_compat ? norm_planes_k<true> : norm_planes_k<false>, n_tok, n_embd / 8u, 0, st, d_x, d_norm_w, eps, n_embd,
+                       w.xn, t1, t2, w.h);
+            g_q4b_launches++;
+            if (!q4b_launch_ok("norm_planes")) return false;
+        } else if (!q4b_rms_rows(d_x, d_norm_w, w.xn, n_embd, eps, n_tok)) {
+            return false;
+        }
         if (!q4_hip_gemv_dd_n(Q4_T_F32, (const uint8_t *)d_router, n_expert, n_embd, w.xn, w.logits, 1.0f,
                               n_tok))
             return false;
@@ -1334,13 +1403,12 @@ extern "C" bool q4_cuda_moe_layer_nt(const uint8_t *base, uint64_t stride, uint3
                               n_e, n_tok, n_e, topk, sh ? (int32_t)n_expert : -1)) {
         return false;
     }
-    // A product that runs on the tensor cores and the wide form gets its activations as planes at once.
     const Q8View xv = q8_view(w.xq, rows, n_embd), hv = q8_view(w.hq, rows, n_ff);
-    if (gt == Q4_T_IQ3_S && n_embd <= 4096u && takes_wide_tc(base + og, stride, n_entries, rows, n_embd, 2u * n_ff)) {
-        q4b_launch(g_q8_compat ? row_planes_k<true> : row_planes_k<false>, (unsigned)rows, n_embd / 8u, 0, st, w.xn, w.atok, n_embd,
-                   xv.h1, xv.h2, xv.rs);
+    if (gu_tc) {
+        q4b_launch(gather_planes_k, (unsigned)((rows + 3u) / 4u), n_embd / 8u, 0, st, t1, t2, w.h, w.atok, (uint32_t)rows, n_embd, xv.h1,
+                   xv.h2, xv.rs);
         g_q4b_launches++;
-        if (!q4b_launch_ok("row_planes") ||
+        if (!q4b_launch_ok("gather_planes") ||
             !mmqtc::launch_wide(base + og, stride, w.stg, w.stgn, n_entries, w.cbounds, xv.h1, xv.h2, xv.rs, rows, n_embd, 2u * n_ff,
                                 w.gu, 2ull * n_ff))
             return false;
@@ -1353,7 +1421,7 @@ extern "C" bool q4_cuda_moe_layer_nt(const uint8_t *base, uint64_t stride, uint3
                                 2ull * n_ff, n_tok, gt))
             return false;
     }
-    if (dt == Q4_T_IQ3_S && n_ff <= 2048u && takes_wide_tc(base + od, stride, n_entries, rows, n_ff, n_embd)) {
+    if (dn_tc) {
         const uint32_t per = n_ff / 8u, rpb = 256u / per;
         q4b_launch(g_q8_compat ? swiglu_planes_k<true> : swiglu_planes_k<false>, (unsigned)((rows + rpb - 1u) / rpb), 256, 0, st, w.gu,
                    rows, n_ff, per, hv.h1, hv.h2, hv.rs);
