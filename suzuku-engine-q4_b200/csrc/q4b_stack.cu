@@ -483,10 +483,20 @@ __device__ __forceinline__ void stack_body(const Args &a, const float4 *xrow) {
     const uint32_t v0 = (uint32_t)((uint64_t)cta * (H / 4) / ncta) * ne;
     const uint32_t v1 = (uint32_t)((uint64_t)(cta + 1) * (H / 4) / ncta) * ne;
 
+    // The code table does not depend on anything a kernel before this one writes: it is filled before the wait.  Entry i
+    // replicated once per lane: thread t < 512 holds entry t, a warp broadcasts its 32 entries one by one.
+    {
+        const uint32_t code = __ldg(a.codes + tid);
+#pragma unroll 8
+        for (uint32_t i = 0; i < 32; i++) {
+            const uint32_t v = __shfl_sync(0xffffffffu, code, i);
+            tab[(warp * 32u + i) * 32u + lane] = v;
+        }
+    }
+    q4b_pdl_wait();
     // loads with nothing before them in the dependency chain go first
     Layer cur = a.layers ? a.layers[SESSION ? a.li0 : 0u] : a.l0;
     float4 xv = make_float4(0.f, 0.f, 0.f, 0.f), wv = make_float4(1.f, 1.f, 1.f, 1.f);
-    uint32_t code = 0;
     if (tid < H / 4) {
         if constexpr (XPARAM) {
             // The row sits in the parameter block (constant bank): a warp whose lanes ask for 32
@@ -502,7 +512,6 @@ __device__ __forceinline__ void stack_body(const Args &a, const float4 *xrow) {
             xv = xrow[tid];
         }
         if (cur.norm_w) wv = reinterpret_cast<const float4 *>(cur.norm_w)[tid];
-        code = a.codes[tid];
     }
     if (tid == 0) {
         for (uint32_t i = 0; i < N_MBAR; i++) mbar_init(&S.mbar[i], 1);
@@ -532,15 +541,6 @@ __device__ __forceinline__ void stack_body(const Args &a, const float4 *xrow) {
         // do not overlap, so old / grid is the same in all CTAs of a launch
         const unsigned long long old = atomicAdd(a.ctr, 1ull);
         S.ep0 = (uint32_t)(((old / ncta) * MAX_LAYERS) % 0xffffffffull) + 1u;   // never 0
-    }
-    // code table: entry i replicated once per lane: thread t < 512 holds entry t, a warp
-    // broadcasts its 32 entries one by one
-    if (tid < 512) {
-#pragma unroll 8
-        for (uint32_t i = 0; i < 32; i++) {
-            const uint32_t v = __shfl_sync(0xffffffffu, code, i);
-            tab[(warp * 32u + i) * 32u + lane] = v;
-        }
     }
     const uint32_t *tl = tab + lane;
     uint32_t par = 0;        // parity of the once-per-layer mbarriers
@@ -1178,11 +1178,15 @@ static bool stack_launch(const stk::Layer &l0, const stk::Layer *d_layers, uint3
     cfg.blockDim = dim3(NT);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s.stream;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeCooperative;  // all CTAs resident at once: they wait for one another's words
     at[0].val.cooperative = 1;
+    // a CTA comes up as the one of the kernel before leaves its SM, fills its code table and waits (not the host forms:
+    // they are waited for before the next call)
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = ses || h_x_param ? 1 : 2;
     cudaError_t le;
     if (ses) {
         session_args(ses, &a);
