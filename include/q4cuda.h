@@ -596,9 +596,10 @@ bool q4_cuda_assign_local(const int32_t *d_ids, const float *d_wts, int32_t *d_a
 
 /* Which grouped product q4_mmq_mul_id and q4_cuda_moe_layer_n run (no reference
  * counterpart; the reference picks its tile kernel by row count inside q4_mmq_mul_id,
- * src/q4_mmq.cu:387-470): -1 = by size (experts with 12 rows or more go to the tensor-core
- * kernel when the weight rows are a multiple of 128; the others to the streaming CUDA-core
- * kernel on tiled arenas, else to the general CUDA-core kernel),
+ * src/q4_mmq.cu:387-470): -1 = by size (on arenas with a wide copy, calls of 20 rows or more per
+ * expert go to the tensor-core kernel and the others to the streaming kernel; without one, experts
+ * with 12 rows or more go to the tensor-core kernel when the weight rows are a multiple of 128,
+ * the others to the streaming CUDA-core kernel on tiled arenas, else to the general CUDA-core kernel),
  * 0 = CUDA-core kernels only, 1 = the tensor-core kernel whenever the shape allows,
  * 2 = the general CUDA-core kernel only.  Returns false for an unknown mode, or for 1
  * when the tensor-core path could not be set up. */

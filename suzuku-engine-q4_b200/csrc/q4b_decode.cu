@@ -23,6 +23,7 @@ uint32_t q4b_next_flag_epoch();
 static bool decode_fused_on();
 
 bool q4b_router_tc(const float *W, uint64_t nrows, uint64_t ncols, const float *x, float *y, float scale, uint32_t n_tok);
+int q4b_tc_mode();   // q4b_grouped.cu: the mode of q4_cuda_mmq_tc_mode
 constexpr uint32_t ROUTE_MAX_TOK = 256;   // tokens of the one-launch routing; above, the router product runs on the tensor cores
 
 #define Q4B_X_SLICE 64u  // scratch slice that holds the quantised input row
@@ -1061,7 +1062,10 @@ extern "C" bool q4_hip_gemv_dd_n(uint32_t ggml_type, const uint8_t *d_w, uint64_
                                  uint32_t n_batch) {
     if (!g_q4b.ok || !d_w || !d_x || !d_y || nrows == 0 || ncols == 0 || n_batch == 0) return false;
     const dim3 grid((unsigned)((nrows + 7) / 8), n_batch);
-    if (ggml_type == Q4_T_F32 && n_batch > ROUTE_MAX_TOK &&
+    // The tensor-core product adds in another order.  From 512 tokens it runs in every mode; from 257 to 511 only where
+    // tensor cores are wanted, because modes 0 and 2 keep a row's bits independent of the batch below 512 tokens.
+    const bool free_order = n_batch >= 512 || (n_batch > ROUTE_MAX_TOK && q4b_tc_mode() != 0 && q4b_tc_mode() != 2);
+    if (ggml_type == Q4_T_F32 && free_order &&
         q4b_router_tc(reinterpret_cast<const float *>(d_w), nrows, ncols, d_x, d_y, scale, n_batch)) {
         // a large batch: one tensor-core product instead of n_batch matrix-vector passes over W
     } else if (ggml_type == Q4_T_F32 && n_batch >= 2 && ncols == 2048) {

@@ -1123,6 +1123,7 @@ bool q4b_mmq_tc_warm() {
     const bool f = few::warm() && wide::warm() && rows4::warm();
     return mmqtc::warm() && mmqtc::warm_wide() && f;
 }
+int q4b_tc_mode() { return grouped::g_tc_mode; }
 extern "C" bool q4_cuda_mmq_tc_mode(int mode) {
     if (mode < -1 || mode > 2 || (mode == 1 && !mmqtc::g_ready)) return false;
     grouped::g_tc_mode = mode;

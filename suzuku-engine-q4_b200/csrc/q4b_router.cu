@@ -1,6 +1,6 @@
 // The router product of a batch on the tensor cores: y[t][e] = scale * sum_h x[t][h] W[e][h] with fp32 operands,
-// for more than 256 tokens (q4_hip_gemv_dd_n; below that the matrix-vector kernels keep a row's bits independent of
-// the batch).
+// for more than 256 tokens (512 in modes 0 and 2 of q4_cuda_mmq_tc_mode; below that the matrix-vector kernels keep a
+// row's bits independent of the batch).
 //
 // Arithmetic: an fp32 value is the exact sum of three bf16 values, x = x1 + x2 + x3 (8 bits of mantissa each).  Of
 // the nine products of the parts the six down to 2^-18 of the largest are formed (the other three are below the last

@@ -132,7 +132,7 @@ __host__ __device__ inline uint32_t smem_bytes(uint32_t cols, uint32_t chunk_byt
     return (uint32_t)((sizeof(Smem) + 127u) & ~127u) + 2u * act_bytes(cols) + n_stage * chunk_bytes;
 }
 // Relative cost of a chunk for a block of rows: the stream of its bytes until the rows' own work exceeds it
-// (370 experts, gate/up: 72 us with 1 row, 80 with 2, 105 with up to 8, 145 with up to 16).
+// (370 experts, gate/up, events around one call: 90 us with 1 row, 92 with 2, 115 with 8, 152 with 16).
 __device__ __forceinline__ uint32_t block_cost(uint32_t rows) {
     return rows <= 2u ? 7u + rows : rows <= 8u ? 12u : 17u;
 }

@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(NT, 1) mmq_wide_k(const WArgs a, const __grid_
     tc_fence_after();
     const uint32_t tmem = s.tmem_base;
     // Bounded: half a second, then the error word, and from there on short waits.  A waiting warp sleeps between looks:
-    // polling took issue slots from the decode warps (measured with sleeping waits that had no time limit: 512 experts of 128 rows, 508 -> 463 us under ncu).
+    // polling took issue slots from the decode warps (512 experts of 128 rows, an earlier version under ncu: 508 -> 463 us).
     unsigned long long patience = 500000000ull;
     auto wait = [&](unsigned long long *bar, uint32_t parity, uint32_t code) {
         if (mbar_look(bar, parity)) return;

@@ -1,6 +1,7 @@
 """The router product of more than 256 tokens (csrc/q4b_router.cu: fp32 operands as three bf16 parts on the
 tensor cores) against the product in double: edges of its tiles (128 tokens, 64 experts, 128 columns), one
-row with an outlier, and error no larger than that of fp32 additions in sequence."""
+row with an outlier, and error no larger than that of fp32 additions in sequence.  Below 512 tokens the modes
+without tensor cores keep a row's bits independent of the batch."""
 import numpy as np
 import pytest
 
@@ -28,3 +29,21 @@ def test_batch_router_product(dev, n_tok, n_exp, n):
     assert err[5].max() <= max(err_seq[5].max(), 2.0 ** -21 * np.abs(want[5]).max())
     assert np.linalg.norm(err[plain]) <= np.linalg.norm(err_seq[plain])
     assert dev.lib.q4_cuda_device_error() == 0
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("n_tok", [257, 511])
+def test_row_bits_without_tensor_cores(dev, n_tok, mode):
+    n_exp, n = 130, 2048
+    rng = np.random.default_rng(n_tok)
+    d_w = dev.upload((rng.standard_normal((n_exp, n)) * 0.02).astype(np.float32))
+    d_x, d_y, d_1 = dev.upload(rng.standard_normal((n_tok, n)).astype(np.float32)), dev.malloc(n_tok * n_exp * 4), dev.malloc(n_exp * 4)
+    assert dev.lib.q4_cuda_mmq_tc_mode(mode)
+    try:
+        assert dev.lib.q4_hip_gemv_dd_n(0, d_w, n_exp, n, d_x, d_y, 1.0, n_tok)
+    finally:
+        assert dev.lib.q4_cuda_mmq_tc_mode(-1)
+    y = dev.download(d_y, (n_tok, n_exp), np.float32)
+    for t in (0, 128, n_tok - 1):
+        assert dev.lib.q4_hip_gemv_dd(0, d_w, n_exp, n, d_x + t * n * 4, d_1, 1.0)
+        assert np.array_equal(y[t].view(np.uint32), dev.download(d_1, (n_exp,), np.float32).view(np.uint32))
