@@ -119,3 +119,31 @@ def test_policy_hold_and_widest_row(dev, pkg, oracle, mv):
     assert mv.q4_mmvq_n(ty, d_w, R, K, d_x, d_y, 1.0, 3)
     assert not dev.download(d_y, (3, R), np.float32).any()
     assert lib.q4_cuda_device_error() == 0
+
+
+@pytest.mark.parametrize("ty,K", [(12, 256), (13, 768), (14, 2304), (23, 2048), (20, 32), (20, 1056)])
+@pytest.mark.parametrize("n,R", [(2, 1), (2, 149), (4, 2369), (3, 4737), (8, 4800)])
+def test_shares_of_rows_ties_and_held_rows(dev, pkg, oracle, mv, ty, K, n, R):
+    """Row counts around one row a CTA and one turn of its warps; widths with a part of a trip; activations aligned to a
+    float only and quotients that are exact ties; rows kept by q4_mmvq_hold."""
+    rng = np.random.default_rng(ty + K + R)
+    w = np.tile(_weights(pkg, rng, ty, min(R, 61), K), ((R + 60) // 61, 1))[:R].copy()
+    xs = _acts(rng, n, K)
+    xs[0, :32] = rng.integers(-127, 127, 32) + 0.5
+    xs[0, 3] = 127.0                                   # d = 1: the others are ties
+    xs[1, -32:] = np.float32(1e-41)                    # a scale without a reciprocal
+    d_w, d_y = dev.upload(w), dev.malloc(n * R * 4)
+    d_x = dev.upload(np.concatenate([[0.0], xs.ravel()]).astype(np.float32)) + 4
+    rows = sorted({0, R - 1, R // 2, min(R - 1, 2367), min(R - 1, 4735)})
+    ref = _bits(oracle.mv_rows(ty, w[rows], len(rows), K, xs))
+    got = []
+    for hold in (False, True):
+        if hold:
+            mv.q4_mmvq_hold(d_x)
+        dev.write(d_y, np.full((n, R), 7.5, np.float32))
+        assert mv.q4_mmvq_n(ty, d_w, R, K, d_x, d_y, 1.0, n)
+        got.append(_bits(dev.download(d_y, (n, R), np.float32)))
+        assert np.array_equal(got[-1][:, rows], ref)
+    assert np.array_equal(got[0], got[1])
+    assert np.array_equal(got[0][:, :min(R, 61)], got[0][:, (R - 1) // 61 * 61 - 61:][:, :min(R, 61)]) or R <= 122
+    assert dev.lib.q4_cuda_device_error() == 0
