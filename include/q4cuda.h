@@ -475,8 +475,11 @@ bool q4_cuda_moe_exec_noalloc(const uint8_t *base, uint64_t stride, const int32_
 /* A tiled arena also gets a second copy of its tiles in a form of 4.25 bits a weight that the streaming and
  * tensor-core products decode with a fraction of the instructions, while half of the device's memory stays
  * free after taking it (1.24 times the arena; Q4B_WIDE=0 in the environment turns it off, and the products
- * then decode the tiles).  It is brought up to date by q4_hip_experts_put*_a and retile_a, the two calls
- * that change a tiled arena's bytes, and freed with the arena.
+ * then decode the tiles).  It is freed with the arena.  Everything in this library that writes an arena's
+ * bytes brings it up to date on the same stream: q4_hip_experts_put*_a, retile_a, and q4_hip_h2d,
+ * q4_hip_h2d_async, q4_hip_copy_async and q4_hip_fill where their destination lies in the arena (tiled bytes,
+ * for instance a pack moved from slot to slot).  A program that writes tiled bytes with kernels or copies of
+ * its own calls refresh_a behind them.
  *
  * Resident storage format of an arena.  By default q4_hip_experts_put*_a rewrites
  * each pack, in place and at the same size, into the library's tiled form of
@@ -489,12 +492,17 @@ bool q4_cuda_moe_exec_noalloc(const uint8_t *base, uint64_t stride, const int32_
  *     Q4B_TILED=0); 2 = the caller vouches that the slots hold IQ3_S bytes only, and
  *     any slot size that is a multiple of the 880-byte tile is tiled (single matrices);
  *   tiled_a: 1 if the arena is tiled;
+ *   wide_a: 1 if the arena has the second copy;
+ *   refresh_a: bring the second copy of slots up to date (queued on the compute stream; nothing to do, and
+ *     true, where the arena has none);
  *   retile_a: convert slots that were filled on the device in engine byte order
  *     (e.g. by q4_cuda_synth_iq3s);
  *   get_a: copy a slot back to the host in the engine's byte order (synchronous). */
 void q4_cuda_set_tiled_default(int on);
 int q4_cuda_experts_tiled_a(int arena);
+int q4_cuda_experts_wide_a(int arena);
 bool q4_cuda_experts_retile_a(int arena, uint32_t first_slot, uint32_t n_slots);
+bool q4_cuda_experts_refresh_a(int arena, uint32_t first_slot, uint32_t n_slots);
 bool q4_cuda_experts_get_a(int arena, uint32_t slot, uint8_t *host, uint64_t n);
 
 /* The same layer for a caller that holds HOST buffers (h_x in, h_y out, n_embd

@@ -181,7 +181,9 @@ SIGNATURES = {
                                      vp]),
     "q4_cuda_set_tiled_default": (None, [C.c_int]),
     "q4_cuda_experts_tiled_a": (C.c_int, [C.c_int]),
+    "q4_cuda_experts_wide_a": (C.c_int, [C.c_int]),
     "q4_cuda_experts_retile_a": (b, [C.c_int, u32, u32]),
+    "q4_cuda_experts_refresh_a": (b, [C.c_int, u32, u32]),
     "q4_cuda_experts_get_a": (b, [C.c_int, u32, vp, u64]),
     "q4_cuda_moe_decode_host": (b, [vp, u64, u64, u64, u64, i32, vp, vp, f32, vp, u32, u32, u32,
                                     u32, vp]),

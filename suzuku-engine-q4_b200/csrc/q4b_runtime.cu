@@ -160,6 +160,23 @@ bool launch_widen(const Arena &a, uint64_t off, uint64_t bytes, cudaStream_t st)
     return q4b_launch_ok("tile_widen");
 }
 
+// A copy or fill of this library has been queued on st that writes [p, p + bytes).  A tiled arena's bytes may be
+// written that way (a pack moved or duplicated from slot to slot, tiles restored from a saved copy), so the tiles that
+// the range touches are widened again behind it: one-token calls read the tiles, many-token calls the wide copy.
+bool widen_written(const void *p, uint64_t bytes, cudaStream_t st) {
+    const uint64_t q = (uint64_t)(uintptr_t)p;
+    for (int i = 0; i < 4; i++) {
+        const Arena &a = g_arena[i];
+        if (!a.wide) continue;
+        const uint64_t lo = (uint64_t)(uintptr_t)a.base, hi = lo + (uint64_t)a.n_slots * a.stride;   // whole tiles
+        const uint64_t b = q > lo ? q : lo, e = q + bytes < hi ? q + bytes : hi;
+        if (b >= e) continue;
+        const uint64_t first = (b - lo) / Q4B_TILE_BYTES, end = (e - lo + Q4B_TILE_BYTES - 1u) / Q4B_TILE_BYTES;
+        if (!launch_widen(a, first * Q4B_TILE_BYTES, (end - first) * Q4B_TILE_BYTES, st)) return false;
+    }
+    return true;
+}
+
 // The wide copy of a new arena: taken while half of the device's memory stays free after it, so that a
 // program whose memory is planned for the packs alone keeps fitting; without it the kernels that decode
 // the tiles themselves run.  Q4B_WIDE=0 turns it off.
@@ -359,6 +376,7 @@ extern "C" void q4_hip_free(void *p) {
 extern "C" bool q4_hip_h2d(void *d, const void *h, size_t n) {
     if (!g_q4b.ok || !d || !h) return false;
     Q4B_CHECK(cudaMemcpyAsync(d, h, n, cudaMemcpyHostToDevice, g_q4b.stream));
+    if (!widen_written(d, n, g_q4b.stream)) return false;
     Q4B_CHECK(cudaStreamSynchronize(g_q4b.stream));
     return true;
 }
@@ -371,7 +389,7 @@ extern "C" bool q4_hip_d2h(void *h, const void *d, size_t n) {
 extern "C" bool q4_hip_h2d_async(void *d, const void *h, uint64_t n) {
     if (!g_q4b.ok || !d || !h) return false;
     Q4B_CHECK(cudaMemcpyAsync(d, h, n, cudaMemcpyHostToDevice, g_q4b.stream));
-    return true;
+    return widen_written(d, n, g_q4b.stream);
 }
 extern "C" bool q4_hip_d2h_async(void *h, const void *d, uint64_t n) {
     if (!g_q4b.ok || !d || !h) return false;
@@ -381,7 +399,7 @@ extern "C" bool q4_hip_d2h_async(void *h, const void *d, uint64_t n) {
 extern "C" bool q4_hip_copy_async(float *d, const float *s, uint64_t n) {
     if (!g_q4b.ok || !d || !s) return false;
     Q4B_CHECK(cudaMemcpyAsync(d, s, n * sizeof(float), cudaMemcpyDeviceToDevice, g_q4b.stream));
-    return true;
+    return widen_written(d, n * sizeof(float), g_q4b.stream);
 }
 extern "C" uint64_t q4_hip_vram_free(void) {
     if (!g_q4b.ok) return 0;
@@ -402,7 +420,7 @@ extern "C" bool q4_hip_fill(float *d, float v, uint64_t n) {
     if (nb > 4096) nb = 4096;
     q4b_launch(fill_k, (unsigned)nb, 256, 0, g_q4b.stream, d, v, n);
     g_q4b_launches++;
-    return q4b_launch_ok("fill");
+    return q4b_launch_ok("fill") && widen_written(d, n * sizeof(float), g_q4b.stream);
 }
 
 // ---- arenas ----
@@ -629,6 +647,15 @@ extern "C" bool q4_cuda_experts_retile_a(int arena, uint32_t first_slot, uint32_
     return launch_tile_permute(a.base + (uint64_t)first_slot * a.stride, (uint64_t)n_slots * a.stride,
                                true, g_q4b.stream) &&
            launch_widen(a, (uint64_t)first_slot * a.stride, (uint64_t)n_slots * a.stride, g_q4b.stream);
+}
+extern "C" int q4_cuda_experts_wide_a(int arena) {
+    return (arena >= 0 && arena < 4 && g_arena[arena].wide) ? 1 : 0;
+}
+extern "C" bool q4_cuda_experts_refresh_a(int arena, uint32_t first_slot, uint32_t n_slots) {
+    if (!g_q4b.ok || arena < 0 || arena >= 4) return false;
+    const Arena &a = g_arena[arena];
+    if (!a.base || !a.tiled || (uint64_t)first_slot + n_slots > a.n_slots || n_slots == 0) return false;
+    return launch_widen(a, (uint64_t)first_slot * a.stride, (uint64_t)n_slots * a.stride, g_q4b.stream);
 }
 extern "C" bool q4_cuda_experts_get_a(int arena, uint32_t slot, uint8_t *host, uint64_t n) {
     if (!g_q4b.ok || arena < 0 || arena >= 4 || !host) return false;

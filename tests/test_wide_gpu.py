@@ -37,3 +37,62 @@ def test_wide_product_equals_the_general_kernel(dev, pkg, H, F, per):
     finally:
         lib.q4_cuda_mmq_tc_mode(-1)
         layer.close()
+
+
+class _Bytes:
+    """Device bytes as an array another library can write."""
+
+    def __init__(self, ptr, n):
+        self.__cuda_array_interface__ = {"shape": (n,), "typestr": "|u1", "data": (ptr, False), "version": 3}
+
+
+@pytest.mark.parametrize("how", ["copy", "h2d", "h2d_async", "fill", "part of a tile", "own copy"])
+def test_bytes_written_into_a_tiled_arena_reach_both_forms(dev, pkg, how):
+    """Tiled bytes that are copied over a slot (a pack moved or duplicated) replace it for every kernel: the general one
+    reads the tiles, the streaming and the tensor-core product the wide copy."""
+    H, F, E, per = 2048, 512, 3, 24
+    rng = np.random.default_rng(11)
+    layer = pkg.MoeLayer(dev, pkg.synth.expert_packs(rng, E, H, F), None, np.zeros((E, H), np.float32), None, H, F, 1, arena=1)
+    lib, n = dev.lib, layer.pack
+    assert lib.q4_cuda_experts_wide_a(1) == 1
+    src, dst = (lib.q4_hip_experts_dev_a(1, s) for s in (0, 2))
+    x = rng.standard_normal((E * per, H)).astype(np.float32)
+    d_x, d_xq = dev.upload(x), dev.malloc(lib.q4_mmq_q8_bytes(E * per, H))
+    d_dst, bounds = dev.malloc(E * per * 2 * F * 4), dev.upload((np.arange(E + 1) * per).astype(np.int32))
+
+    def products():
+        out = []
+        for mode in (2, 0, 1):       # general, streaming, tensor cores
+            assert lib.q4_cuda_mmq_tc_mode(mode) and lib.q4_mmq_quantize(d_x, None, d_xq, IQ3_S, H, E * per)
+            assert lib.q4_mmq_mul_id(layer.base, IQ3_S, 2 * F, H, layer.stride, E, d_xq, bounds, per, E * per, d_dst, 2 * F)
+            out.append(dev.download(d_dst, (E, per, 2 * F), np.float32))
+        return out
+    try:
+        before = products()[0]
+        pack = dev.download(src, (n,), np.uint8)
+        if how == "copy":
+            assert lib.q4_hip_copy_async(dst, src, n // 4)
+        elif how == "h2d":
+            assert lib.q4_hip_h2d(dst, pack.ctypes.data, n)
+        elif how == "h2d_async":
+            assert lib.q4_hip_h2d_async(dst, pack.ctypes.data, n)
+        elif how == "fill":
+            assert lib.q4_hip_fill(dst, 0.0, n // 4)
+        elif how == "part of a tile":    # the tail of one tile, the next one, the head of a third; up to the arena's end too
+            assert lib.q4_hip_copy_async(dst + 440, src + 440, (880 + 660) // 4)
+            assert lib.q4_hip_copy_async(dst + n - 8, src + n - 8, 2)
+        else:
+            import torch
+            torch.as_tensor(_Bytes(dst, n), device="cuda").copy_(torch.as_tensor(_Bytes(src, n), device="cuda"))
+            torch.cuda.synchronize()
+            assert lib.q4_cuda_experts_refresh_a(1, 2, 1)
+        tiles, wide, tc = products()
+        assert not np.array_equal(tiles[2], before[2])
+        assert np.array_equal(tiles.view(np.uint32), wide.view(np.uint32))
+        assert np.linalg.norm(tiles - tc) <= 1e-5 * np.linalg.norm(tiles)
+        assert np.array_equal(tiles[0], before[0]) and np.array_equal(tiles[1], before[1])
+        assert not lib.q4_cuda_experts_refresh_a(1, 3, 1) and not lib.q4_cuda_experts_refresh_a(1, 0, 0)
+        assert lib.q4_cuda_device_error() == 0
+    finally:
+        lib.q4_cuda_mmq_tc_mode(-1)
+        layer.close()
