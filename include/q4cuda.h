@@ -264,7 +264,8 @@ bool q4_hip_moe_exec_tok(const uint8_t *base, uint64_t stride, const int32_t *d_
  * q4_mmvq_set(mode): 0 off, 1 (default) calls of 2..8 rows, 2 calls of 1..8 rows but only between
  * q4_mmvq_verify(1) and q4_mmvq_verify(0).  q4_mmvq_warm() allocates the row scratch (q4_hip_init
  * already does).  Between hold(x) and release() calls on the same x (same width, no more rows)
- * reuse its quantisation.  false: nothing was queued, the caller keeps its float path. */
+ * reuse its quantisation.  d_y may overlap d_x (all of x is read before any of y is written).
+ * false: nothing was queued, the caller keeps its float path. */
 bool q4_mmvq_n(uint32_t ty, const uint8_t *d_w, uint64_t nrows, uint64_t ncols, const float *d_x,
                float *d_y, float scale, uint32_t n);
 void q4_mmvq_warm(void);

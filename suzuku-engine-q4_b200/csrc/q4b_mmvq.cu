@@ -59,7 +59,7 @@ __device__ __forceinline__ float4 ld4(const float *x, uint32_t i, uint32_t n4) {
     if (((uintptr_t)x & 15u) == 0) return reinterpret_cast<const float4 *>(x)[i];
     return make_float4(x[4 * (size_t)i], x[4 * (size_t)i + 1], x[4 * (size_t)i + 2], x[4 * (size_t)i + 3]);
 }
-// rows that q4_mmvq_hold keeps between calls
+// rows that q4_mmvq_hold keeps between calls, and those of a call whose y overlaps its x
 __global__ void quant8d_k(const float *__restrict__ x, uint32_t n4, uint32_t *__restrict__ q, float2 *__restrict__ ds) {
     q4b_pdl_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -222,7 +222,7 @@ template <> struct Fmt<20u> {
 
 // ------------------------------------------------------------------ the product
 // One launch a call: a CTA per SM quantises the activation rows into its shared memory (or copies rows that
-// q4_mmvq_hold keeps) and takes a contiguous share of the weight rows, one or two rows a warp and turn.  With one, the
+// quant8d_k has written) and takes a contiguous share of the weight rows, one or two rows a warp and turn.  With one, the
 // rows are split evenly over the turns; with two, the last turn takes one a warp if that is enough (34.6 rows an SM and 32
 // in a turn: 6 rows of IQ4_NL 12.9 us a call, 11.6 split evenly).
 // A call is short (4096 x 2048 of Q4_K: 4.7 MB, 0.7 us of HBM), so what bounds it is the chain: launch, activations,
@@ -474,19 +474,24 @@ extern "C" bool q4_mmvq_n(uint32_t ty, const uint8_t *d_w, uint64_t nrows, uint6
     }
     if (!mv::g_q || !mv::dense_fits(ty, d_w, ncols)) return false;   // q4_mmvq_warm allocates, outside any stream capture
     const uint32_t K = (uint32_t)ncols, R = (uint32_t)nrows;
+    // Rows quantised by a launch of their own: those that hold keeps for further calls, and those of a call that writes
+    // its results over them (in dense_rows_k a CTA writes y while others may not have read their x yet).
     const bool keep = mv::g_hold && mv::g_hold == d_x;
-    if (keep && !held) {
+    const uintptr_t xa = (uintptr_t)d_x, ya = (uintptr_t)d_y;
+    const bool apart = ya >= xa + (uint64_t)n * K * sizeof(float) || xa >= ya + (uint64_t)n * R * sizeof(float);
+    if ((keep && !held) || (!keep && !apart)) {
         const uint32_t n4 = n * K / 4u;
         q4b_launch(mv::quant8d_k, (n4 + 255u) / 256u, 256, 0, g_q4b.stream, d_x, n4, (uint32_t *)mv::g_q, mv::g_ds);
         g_q4b_launches.fetch_add(1, std::memory_order_relaxed);
         if (!q4b_launch_ok("mmvq_quant")) return false;
         mv::g_cur_x = d_x, mv::g_cur_k = ncols, mv::g_cur_n = n, mv::g_cur_kind = 1;
     }
+    const bool own = keep || !apart;
     switch (ty) {
-    case 14u: return mv::launch<14u>(n, d_w, d_x, keep, d_y, K, R, scale);
-    case 12u: return mv::launch<12u>(n, d_w, d_x, keep, d_y, K, R, scale);
-    case 13u: return mv::launch<13u>(n, d_w, d_x, keep, d_y, K, R, scale);
-    case 23u: return mv::launch<23u>(n, d_w, d_x, keep, d_y, K, R, scale);
-    default: return mv::launch<20u>(n, d_w, d_x, keep, d_y, K, R, scale);
+    case 14u: return mv::launch<14u>(n, d_w, d_x, own, d_y, K, R, scale);
+    case 12u: return mv::launch<12u>(n, d_w, d_x, own, d_y, K, R, scale);
+    case 13u: return mv::launch<13u>(n, d_w, d_x, own, d_y, K, R, scale);
+    case 23u: return mv::launch<23u>(n, d_w, d_x, own, d_y, K, R, scale);
+    default: return mv::launch<20u>(n, d_w, d_x, own, d_y, K, R, scale);
     }
 }

@@ -147,3 +147,33 @@ def test_shares_of_rows_ties_and_held_rows(dev, pkg, oracle, mv, ty, K, n, R):
     assert np.array_equal(got[0], got[1])
     assert np.array_equal(got[0][:, :min(R, 61)], got[0][:, (R - 1) // 61 * 61 - 61:][:, :min(R, 61)]) or R <= 122
     assert dev.lib.q4_cuda_device_error() == 0
+
+
+@pytest.mark.parametrize("shift", [0, 1024, -1024])
+def test_results_written_over_the_activations(dev, pkg, mv, shift):
+    """y on top of x, and on parts of it: every row of weights sees the whole of the old x.  Work on another stream keeps
+    SMs busy, so that some blocks of the product start after others have written."""
+    import torch
+    ty, n, K, R = 12, 4, 2048, 2048
+    rng = np.random.default_rng(5)
+    xs = _acts(rng, n, K)
+    d_w, d_buf, d_y = dev.upload(_weights(pkg, rng, ty, R, K)), dev.malloc((n * K + 4096) * 4), dev.malloc(n * R * 4)
+    d_x, d_over = d_buf + 2048 * 4, d_buf + (2048 + shift) * 4
+    load = torch.randn(4096, 4096, device="cuda", dtype=torch.bfloat16)
+    dev.write(d_x, xs)
+    assert mv.q4_mmvq_n(ty, d_w, R, K, d_x, d_y, 1.0, n)
+    want = _bits(dev.download(d_y, (n, R), np.float32))
+    for _ in range(20):
+        dev.write(d_x, xs)
+        torch.matmul(load, load)
+        assert mv.q4_mmvq_n(ty, d_w, R, K, d_x, d_over, 1.0, n)
+        assert np.array_equal(_bits(dev.download(d_over, (n, R), np.float32)), want)
+    mv.q4_mmvq_hold(d_x)                 # rows of another x that are being kept
+    other = dev.upload(_acts(rng, n, K))
+    dev.write(d_x, xs)
+    assert mv.q4_mmvq_n(ty, d_w, R, K, d_x, d_y, 1.0, n)
+    assert mv.q4_mmvq_n(ty, d_w, R, K, other, other, 1.0, n)
+    assert mv.q4_mmvq_n(ty, d_w, R, K, d_x, d_y, 1.0, n)
+    assert np.array_equal(_bits(dev.download(d_y, (n, R), np.float32)), want)
+    torch.cuda.synchronize()
+    assert dev.lib.q4_cuda_device_error() == 0
