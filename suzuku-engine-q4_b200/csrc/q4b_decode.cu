@@ -32,10 +32,10 @@ namespace {
 
 // ------------------------------------------------------------------ Q8-A
 // One warp per 32 values.  Slice s reads x + s*xs, writes group s*gps + g.
-__global__ void quant8_k(const float *__restrict__ x, uint64_t xs, uint32_t gps,
+__global__ void quant8_k(const float *x, uint64_t xs, uint32_t gps,
                          uint64_t n_groups, int8_t *__restrict__ q, float *__restrict__ d,
                          int32_t *__restrict__ bs, uint64_t q_slice, uint64_t d_slice,
-                         const int32_t *__restrict__ n_dev) {
+                         const int32_t *n_dev) {
     q4b_pdl_wait();
     const uint64_t g = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (g >= n_groups) return;
@@ -60,7 +60,7 @@ __global__ void quant8_k(const float *__restrict__ x, uint64_t xs, uint32_t gps,
 // ------------------------------------------------------------------ RMSNorm (+ Q8-A)
 // One block of 256 per (group, token) row.  The sum of squares is kept in
 // fp64 like the scalar reference (src/q4_quant.c:697-706).
-__global__ void __launch_bounds__(256) rms_q8_k(const float *__restrict__ x, const float *__restrict__ w,
+__global__ void __launch_bounds__(256) rms_q8_k(const float *x, const float *__restrict__ w,
                          float *__restrict__ y, uint32_t n, uint32_t hc, float eps,
                          int8_t *__restrict__ q, float *__restrict__ d, int32_t *__restrict__ bs,
                          uint64_t q_slice, uint64_t d_slice) {
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(256) hc_streams_k(float *__restrict__ res, con
 // One warp per weight row, four a CTA (a router of 512 rows then covers 128 SMs); grid.y = batch.  The row is asked
 // into L2 before the wait for x.
 __global__ void __launch_bounds__(128) gemv_f32_k(const float *__restrict__ W, uint64_t nrows, uint64_t ncols,
-                           const float *__restrict__ x, float *__restrict__ y, float scale) {
+                           const float *x, float *__restrict__ y, float scale) {
     const uint64_t r = (uint64_t)blockIdx.x * 4u + (threadIdx.x >> 5);
     const uint32_t lane = threadIdx.x & 31u;
     const float *wr = W + r * ncols;
@@ -350,7 +350,7 @@ __device__ __forceinline__ void softmax_topk_regs(const float *__restrict__ l, u
     float m = -INFINITY;
 #pragma unroll
     for (uint32_t j = 0; j < NPL; j++) {
-        p[j] = lane + 32u * j < n ? __ldcg(l + lane + 32u * j) : -INFINITY;
+        p[j] = lane + 32u * j < n ? q4b_ld_cg(l + lane + 32u * j) : -INFINITY;
         m = fmaxf(m, p[j]);
     }
     m = q4b_warp_max(m);
@@ -406,7 +406,7 @@ __device__ __forceinline__ void softmax_topk_warp(const float *__restrict__ l, u
     else softmax_topk_regs<32>(l, n, k, ids, wts, shared_slot, n_out, lane);
 }
 // A warp per token.
-__global__ void __launch_bounds__(128) softmax_topk_k(const float *__restrict__ logits, uint32_t n, uint32_t k,
+__global__ void __launch_bounds__(128) softmax_topk_k(const float *logits, uint32_t n, uint32_t k,
                                                       int32_t *__restrict__ ids, float *__restrict__ wts,
                                                       uint32_t out_stride, int32_t shared_slot,
                                                       int32_t *__restrict__ n_out, uint32_t n_tok) {
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(128) softmax_topk_k(const float *__restrict__ 
 // warp per row, all loads in flight at once) into shared memory, then a warp takes one router row
 // through the eight tokens; the CTA that finishes a group last (a counter per group, no waiting) runs
 // the group's top-k, one warp per token.
-__global__ void __launch_bounds__(256) route_small_k(const float *__restrict__ x, const float *__restrict__ norm_w,
+__global__ void __launch_bounds__(256) route_small_k(const float *x, const float *__restrict__ norm_w,
                                                      float eps, const float *__restrict__ W, uint32_t n_expert,
                                                      uint32_t n_tok, uint32_t topk, float *__restrict__ xn_out,
                                                      float *__restrict__ logits, int32_t *__restrict__ ids,
@@ -502,9 +502,9 @@ __global__ void __launch_bounds__(256) route_small_k(const float *__restrict__ x
 // h[e][f] = silu(gate_f . xq) * (up_f . xq).
 template <bool TILED>
 __global__ void moe_gu_k(const uint8_t *__restrict__ bg, const uint8_t *__restrict__ bu,
-                         uint64_t stride, const int32_t *__restrict__ slots,
-                         const int32_t *__restrict__ n_dev, const int8_t *__restrict__ xq,
-                         const float *__restrict__ xd, const int32_t *__restrict__ xbs,
+                         uint64_t stride, const int32_t *slots,
+                         const int32_t *n_dev, const int8_t *xq,
+                         const float *xd, const int32_t *xbs,
                          uint32_t in_dim, uint32_t n_ff, float *__restrict__ h) {
     extern __shared__ __align__(16) uint8_t smem[];
     uint32_t *tab = reinterpret_cast<uint32_t *>(smem);
@@ -559,10 +559,10 @@ __global__ void moe_gu_k(const uint8_t *__restrict__ bg, const uint8_t *__restri
 // fixed lane assignment, so the result is reproducible run to run.
 template <bool TILED>
 __global__ void moe_ya_k(const uint8_t *__restrict__ bd, uint64_t stride,
-                         const int32_t *__restrict__ slots, const float *__restrict__ wts,
-                         uint32_t n_host, const int32_t *__restrict__ n_dev,
-                         const int8_t *__restrict__ hq, const float *__restrict__ hd,
-                         const int32_t *__restrict__ hbs, uint64_t q_slice, uint64_t d_slice,
+                         const int32_t *slots, const float *wts,
+                         uint32_t n_host, const int32_t *n_dev,
+                         const int8_t *hq, const float *hd,
+                         const int32_t *hbs, uint64_t q_slice, uint64_t d_slice,
                          uint32_t n_ff, uint32_t n_embd, float *__restrict__ y) {
     __shared__ uint32_t tab[512];
     q4b_fill_code_table(tab);
@@ -706,8 +706,8 @@ __global__ void iq4_idot_k(const uint8_t *__restrict__ w, uint64_t nrows, uint32
 // moe_gu_k.  h[e][f] = silu(gate_f . xq) * (up_f . xq).
 template <uint32_t T>
 __global__ void moe_gu4_k(const uint8_t *__restrict__ bg, const uint8_t *__restrict__ bu, uint64_t stride,
-                          const int32_t *__restrict__ slots, const int32_t *__restrict__ n_dev,
-                          const int8_t *__restrict__ xq, const float *__restrict__ xd, uint32_t in_dim,
+                          const int32_t *slots, const int32_t *n_dev,
+                          const int8_t *xq, const float *xd, uint32_t in_dim,
                           uint32_t n_ff, float *__restrict__ h) {
     q4b_pdl_wait();
     const uint32_t f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -752,9 +752,9 @@ __device__ __forceinline__ void down_row_add(float acc, float *y) {
 // there were 14 warps an SM, each with five dependent trips (12 us for ten experts of 2048 x 512).  Codes become
 // values by byte permutes, so no table has to be filled.
 template <uint32_t T>
-__global__ void moe_ya4_k(const uint8_t *__restrict__ bd, uint64_t stride, const int32_t *__restrict__ slots,
-                          const float *__restrict__ wts, uint32_t n_host, const int32_t *__restrict__ n_dev,
-                          const int8_t *__restrict__ hq, const float *__restrict__ hd, uint64_t q_slice,
+__global__ void moe_ya4_k(const uint8_t *__restrict__ bd, uint64_t stride, const int32_t *slots,
+                          const float *wts, uint32_t n_host, const int32_t *n_dev,
+                          const int8_t *hq, const float *hd, uint64_t q_slice,
                           uint64_t d_slice, uint32_t n_ff, uint32_t n_embd, float *__restrict__ y) {
     q4b_pdl_wait();
     const uint32_t row = blockIdx.x * 2u + (threadIdx.x >> 7), lane = threadIdx.x & 127u;

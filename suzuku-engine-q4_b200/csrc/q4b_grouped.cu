@@ -93,7 +93,7 @@ int g_q8_compat = 0;   // q4_cuda_mmq_q8_compat
 // Four lanes per 32 values of one gathered row, eight values each (a negative source row
 // gives zeros).
 template <bool COMPAT>
-__global__ void quantize_rows_k(const float *__restrict__ x, const int32_t *__restrict__ ids,
+__global__ void quantize_rows_k(const float *x, const int32_t *ids,
                                 uint64_t cols, uint64_t rows, int8_t *__restrict__ q,
                                 float *__restrict__ d, int32_t *__restrict__ bs) {
     q4b_pdl_wait();
@@ -107,8 +107,8 @@ __global__ void quantize_rows_k(const float *__restrict__ x, const int32_t *__re
     float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0;
     if (src >= 0) {
         const float4 *p = reinterpret_cast<const float4 *>(x + (uint64_t)src * cols + gl * 32u + part * 8u);
-        v0 = __ldg(p);
-        v1 = __ldg(p + 1);
+        v0 = p[0];
+        v1 = p[1];
     }
     float a = fmaxf(fmaxf(fmaxf(fabsf(v0.x), fabsf(v0.y)), fmaxf(fabsf(v0.z), fabsf(v0.w))),
                     fmaxf(fmaxf(fabsf(v1.x), fabsf(v1.y)), fmaxf(fabsf(v1.z), fabsf(v1.w))));
@@ -251,7 +251,7 @@ __global__ void swiglu_rows_k(const float *__restrict__ gu, float *__restrict__ 
 // h = silu(g) * u and its Q8-A quantisation in one pass (the values swiglu_rows_k followed by
 // quantize_rows_k would give): four lanes per 32 hidden values, eight each.
 template <bool COMPAT>
-__global__ void swiglu_quant_rows_k(const float *__restrict__ gu, uint64_t rows, uint64_t n_ff,
+__global__ void swiglu_quant_rows_k(const float *gu, uint64_t rows, uint64_t n_ff,
                                     int8_t *__restrict__ q, float *__restrict__ d,
                                     int32_t *__restrict__ bs) {
     q4b_pdl_wait();
@@ -267,7 +267,7 @@ __global__ void swiglu_quant_rows_k(const float *__restrict__ gu, uint64_t rows,
     if (live) {
         const float4 *pg = reinterpret_cast<const float4 *>(gu + r * 2 * n_ff + gl * 32u + part * 8u);
         const float4 *pu = reinterpret_cast<const float4 *>(gu + r * 2 * n_ff + n_ff + gl * 32u + part * 8u);
-        const float4 g0 = __ldg(pg), g1 = __ldg(pg + 1), u0 = __ldg(pu), u1 = __ldg(pu + 1);
+        const float4 g0 = pg[0], g1 = pg[1], u0 = pu[0], u1 = pu[1];
         v[0] = q4b_swiglu(g0.x, u0.x), v[1] = q4b_swiglu(g0.y, u0.y);
         v[2] = q4b_swiglu(g0.z, u0.z), v[3] = q4b_swiglu(g0.w, u0.w);
         v[4] = q4b_swiglu(g1.x, u1.x), v[5] = q4b_swiglu(g1.y, u1.y);
@@ -341,7 +341,7 @@ __device__ __forceinline__ void quant_planes(const float *v, bool live, uint32_t
 // RMSNorm of a token's row and its planes, a CTA of n / 8 threads (whole warps, at most 512: n <= 4096, n % 256 == 0) per
 // token: x is read once, the normalised row (for the router) and the planes written once.
 template <bool COMPAT>
-__global__ void __launch_bounds__(512) norm_planes_k(const float *__restrict__ x, const float *__restrict__ w, float eps, uint32_t n,
+__global__ void __launch_bounds__(512) norm_planes_k(const float *x, const float *__restrict__ w, float eps, uint32_t n,
                                                      float *__restrict__ xn, __half *__restrict__ h1,
                                                      __half *__restrict__ h2, float *__restrict__ rs) {
     __shared__ double sh[16];
@@ -377,8 +377,8 @@ __global__ void __launch_bounds__(512) norm_planes_k(const float *__restrict__ x
 // The planes of the picks' rows, copied from their tokens' planes: four rows a CTA, n / 8 threads a row, all its loads in
 // flight.  Bound by the bytes (8 n a row in and out).  (Quantising every pick's row anew took 231 us for 90,112 rows of
 // 2048.  Leaving the copies out and fetching the tokens' rows by TMA gathers of four made the product 3.7 times slower.)
-__global__ void __launch_bounds__(512) gather_planes_k(const __half *__restrict__ t1, const __half *__restrict__ t2,
-                                                       const float *__restrict__ trs, const int32_t *__restrict__ ids, uint32_t rows,
+__global__ void __launch_bounds__(512) gather_planes_k(const __half *t1, const __half *t2,
+                                                       const float *trs, const int32_t *ids, uint32_t rows,
                                                        uint32_t n, __half *__restrict__ h1, __half *__restrict__ h2,
                                                        float *__restrict__ rs) {
     q4b_pdl_wait();
@@ -386,12 +386,12 @@ __global__ void __launch_bounds__(512) gather_planes_k(const __half *__restrict_
     int32_t src[4];
     uint4 a[4], b[4];
 #pragma unroll
-    for (uint32_t i = 0; i < 4; i++) src[i] = r0 + i < rows ? __ldg(ids + r0 + i) : -1;   // -1: a row that no expert owns
+    for (uint32_t i = 0; i < 4; i++) src[i] = r0 + i < rows ? ids[r0 + i] : -1;   // -1: a row that no expert owns
 #pragma unroll
     for (uint32_t i = 0; i < 4; i++)
         if (src[i] >= 0) {
-            a[i] = __ldg(reinterpret_cast<const uint4 *>(t1 + (uint64_t)src[i] * n + c));
-            b[i] = __ldg(reinterpret_cast<const uint4 *>(t2 + (uint64_t)src[i] * n + c));
+            a[i] = *reinterpret_cast<const uint4 *>(t1 + (uint64_t)src[i] * n + c);
+            b[i] = *reinterpret_cast<const uint4 *>(t2 + (uint64_t)src[i] * n + c);
         }
 #pragma unroll
     for (uint32_t i = 0; i < 4; i++)
@@ -400,13 +400,13 @@ __global__ void __launch_bounds__(512) gather_planes_k(const __half *__restrict_
             __stcs(reinterpret_cast<uint4 *>(h2 + (uint64_t)(r0 + i) * n + c), b[i]);
         }
     if (threadIdx.x < 4u && r0 + threadIdx.x < rows) {
-        const int32_t s = __ldg(ids + r0 + threadIdx.x);
-        if (s >= 0) rs[r0 + threadIdx.x] = __ldg(trs + s);
+        const int32_t s = ids[r0 + threadIdx.x];
+        if (s >= 0) rs[r0 + threadIdx.x] = trs[s];
     }
 }
 // h = silu(g) * u and its planes: per = n_ff / 8 threads a row (n_ff % 256 == 0, n_ff <= 2048), 256 / per rows a CTA.
 template <bool COMPAT>
-__global__ void __launch_bounds__(256) swiglu_planes_k(const float *__restrict__ gu, uint64_t rows, uint32_t n_ff, uint32_t per,
+__global__ void __launch_bounds__(256) swiglu_planes_k(const float *gu, uint64_t rows, uint32_t n_ff, uint32_t per,
                                                        __half *__restrict__ h1, __half *__restrict__ h2,
                                                        float *__restrict__ rs) {
     __shared__ float red[8];
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(256) swiglu_planes_k(const float *__restrict__
     if (live) {
         const float4 *pg = reinterpret_cast<const float4 *>(gu + r * 2 * n_ff + c);
         const float4 *pu = reinterpret_cast<const float4 *>(gu + r * 2 * n_ff + n_ff + c);
-        const float4 g0 = __ldcs(pg), g1 = __ldcs(pg + 1), u0 = __ldcs(pu), u1 = __ldcs(pu + 1);
+        const float4 g0 = pg[0], g1 = pg[1], u0 = pu[0], u1 = pu[1];
         v[0] = q4b_swiglu(g0.x, u0.x), v[1] = q4b_swiglu(g0.y, u0.y);
         v[2] = q4b_swiglu(g0.z, u0.z), v[3] = q4b_swiglu(g0.w, u0.w);
         v[4] = q4b_swiglu(g1.x, u1.x), v[5] = q4b_swiglu(g1.y, u1.y);
@@ -454,10 +454,10 @@ __global__ void expert_reduce_k(float *__restrict__ y, const float *__restrict__
 // of 11 picks took 7 us), each column still adds its picks in the order k = 0..topk-1.  cnt (optional): picks of
 // the token that count, the others are left out.
 template <bool ADD>
-__global__ void __launch_bounds__(128) expert_reduce4_k(float *__restrict__ y, const float *__restrict__ pd,
-                                                        const int32_t *__restrict__ rsrc,
-                                                        const float *__restrict__ rw, uint32_t topk,
-                                                        uint32_t n_embd, const int32_t *__restrict__ cnt) {
+__global__ void __launch_bounds__(128) expert_reduce4_k(float *__restrict__ y, const float *pd,
+                                                        const int32_t *rsrc,
+                                                        const float *rw, uint32_t topk,
+                                                        uint32_t n_embd, const int32_t *cnt) {
     __shared__ int32_t sp[64];
     __shared__ float sw[64];
     q4b_pdl_wait();
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(128) expert_reduce4_k(float *__restrict__ y, c
 #pragma unroll
         for (uint32_t i = 0; i < 8; i++) {
             const int32_t p = k0 + i < n ? sp[k0 + i] : -1;
-            if (p >= 0) v[i] = __ldcs(reinterpret_cast<const float4 *>(pd + (uint64_t)p * n_embd) + c4);
+            if (p >= 0) v[i] = reinterpret_cast<const float4 *>(pd + (uint64_t)p * n_embd)[c4];
         }
 #pragma unroll
         for (uint32_t i = 0; i < 8; i++)
@@ -512,7 +512,7 @@ static void launch_expert_reduce(float *y, const float *pd, const int32_t *rsrc,
 // time, each lane finding its place among the lanes of the warp that picked the same
 // expert.  Rows of one expert therefore keep (token, pick) order.
 __global__ void __launch_bounds__(1024) assign_k(
-    const int32_t *__restrict__ ids, const float *__restrict__ wts, int32_t *__restrict__ a_tok,
+    const int32_t *ids, const float *wts, int32_t *__restrict__ a_tok,
     int32_t *__restrict__ rsrc, float *__restrict__ rw, int32_t *__restrict__ stg,
     uint32_t *__restrict__ stgn, uint32_t *__restrict__ ek, int32_t *__restrict__ cbounds,
     uint32_t gsz, uint32_t topk, uint32_t n_exp, uint32_t n_tok, uint32_t ek_stride,
@@ -650,7 +650,7 @@ __device__ __forceinline__ int32_t layer_pick(const int32_t *ids, uint32_t i, ui
     const int32_t e = k >= topk_in ? extra_id : ids[(uint64_t)t * topk_in + k];
     return e < 0 || (uint32_t)e >= n_exp ? -1 : e;
 }
-__global__ void __launch_bounds__(256) assign_count_k(const int32_t *__restrict__ ids, uint32_t rows, uint32_t topk,
+__global__ void __launch_bounds__(256) assign_count_k(const int32_t *ids, uint32_t rows, uint32_t topk,
                                                       uint32_t topk_in, int32_t extra_id, uint32_t n_exp,
                                                       uint32_t *__restrict__ hist) {
     extern __shared__ uint32_t sh[];
@@ -725,9 +725,9 @@ __global__ void __launch_bounds__(1024) assign_scan_k(uint32_t *__restrict__ his
         }
     for (uint32_t i = all[0] + e; i < rows; i += 1024u) a_tok[i] = -1;   // unused rows
 }
-__global__ void __launch_bounds__(256) assign_place_k(const int32_t *__restrict__ ids, const float *__restrict__ wts, uint32_t rows,
+__global__ void __launch_bounds__(256) assign_place_k(const int32_t *ids, const float *wts, uint32_t rows,
                                                       uint32_t topk, uint32_t topk_in, int32_t extra_id, uint32_t n_exp,
-                                                      const uint32_t *__restrict__ hist, int32_t *__restrict__ a_tok,
+                                                      const uint32_t *hist, int32_t *__restrict__ a_tok,
                                                       int32_t *__restrict__ rsrc, float *__restrict__ rw) {
     extern __shared__ uint32_t sh[];   // [8 warps][n_exp]: next row of the warp's picks of an expert
     q4b_pdl_wait();
@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(256) assign_place_k(const int32_t *__restrict_
 // threads, one per possible pick; the valid picks are packed first, so that the comparisons of a pick with the ones
 // before it run over picks only (some 40 of them in use, not 512: 8.9 -> 4 us).
 __global__ void __launch_bounds__(512) win_assign_k(
-    const int32_t *__restrict__ es, const float *__restrict__ ew, const int32_t *__restrict__ nh,
+    const int32_t *es, const float *ew, const int32_t *nh,
     uint32_t n_tok, int32_t *__restrict__ act, uint32_t *__restrict__ n_act,
     int32_t *__restrict__ bounds, int32_t *__restrict__ a_tok, int32_t *__restrict__ rsrc,
     float *__restrict__ rw) {

@@ -84,6 +84,9 @@ static inline bool q4b_launch_ok(const char *what) {
 // visible.  What is saved is the drain and the launch between two kernels of a chain, 1 to 1.5 us each.  Every
 // kernel launched this way calls q4b_pdl_wait in every thread before it reads or writes anything another kernel may
 // touch (prefetches into L2 may come before it), so completion stays transitive along the stream.
+// It reads what a kernel ahead wrote with plain loads (or the volatile one below) through pointers that are not
+// `const __restrict__`: __ldg, and the loads the compiler may make of such pointers, promise data that nobody writes
+// while the kernel runs, and may be moved over the wait.  Weights and tables may be read that way.
 template <typename... KA, typename... A>
 static inline void q4b_launch(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};
@@ -102,6 +105,12 @@ static inline void q4b_launch(void (*kernel)(KA...), dim3 grid, dim3 block, size
 __device__ __forceinline__ void q4b_pdl_wait() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// A load past L1: like the wait volatile, so that it stays behind it.
+__device__ __forceinline__ float q4b_ld_cg(const float *p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
 }
 __device__ __forceinline__ void q4b_l2_prefetch(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 

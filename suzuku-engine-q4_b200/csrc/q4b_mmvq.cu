@@ -60,7 +60,7 @@ __device__ __forceinline__ float4 ld4(const float *x, uint32_t i, uint32_t n4) {
     return make_float4(x[4 * (size_t)i], x[4 * (size_t)i + 1], x[4 * (size_t)i + 2], x[4 * (size_t)i + 3]);
 }
 // rows that q4_mmvq_hold keeps between calls, and those of a call whose y overlaps its x
-__global__ void quant8d_k(const float *__restrict__ x, uint32_t n4, uint32_t *__restrict__ q, float2 *__restrict__ ds) {
+__global__ void quant8d_k(const float *x, uint32_t n4, uint32_t *__restrict__ q, float2 *__restrict__ ds) {
     q4b_pdl_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     float2 v;
@@ -238,8 +238,8 @@ template <> struct Fmt<20u> {
 // alignment, which their narrow loads bound (IQ4_NL, 4 rows: 6.9 against 8.0).  4 rows of Q4_K: 6.1 with 512, 6.5 with 1024.
 template <uint32_t TY, int NT> constexpr uint32_t dense_threads = Fmt<TY>::align == 2 || NT <= 2 ? 1024u : 512u;
 template <uint32_t TY, int NT>
-__global__ void __launch_bounds__(dense_threads<TY, NT>, 1) dense_rows_k(const uint8_t *__restrict__ w, const float *__restrict__ x,
-                                                                        const int8_t *__restrict__ gq, const float2 *__restrict__ gds,
+__global__ void __launch_bounds__(dense_threads<TY, NT>, 1) dense_rows_k(const uint8_t *__restrict__ w, const float *x,
+                                                                        const int8_t *gq, const float2 *gds,
                                                                         float *__restrict__ y, uint32_t K, uint32_t rows, float scale) {
     constexpr uint32_t THREADS = dense_threads<TY, NT>;
     using F = Fmt<TY>;

@@ -169,8 +169,8 @@ __global__ void small_idot_k(const uint8_t *__restrict__ w, uint64_t nrows, uint
 // ---- gate/up + SwiGLU with rows of type T (IQ3_XXS or IQ2_S): one warp per (expert, hidden unit) ----
 template <uint32_t T>
 __global__ void __launch_bounds__(512) moe_gux_k(const uint8_t *__restrict__ bg, const uint8_t *__restrict__ bu, uint64_t stride,
-                          const int32_t *__restrict__ slots, const int32_t *__restrict__ n_dev,
-                          const int8_t *__restrict__ xq, const float *__restrict__ xd, uint32_t in_dim,
+                          const int32_t *slots, const int32_t *n_dev,
+                          const int8_t *xq, const float *xd, uint32_t in_dim,
                           uint32_t n_ff, const uint32_t *__restrict__ grid3, const uint2 *__restrict__ grid2,
                           float *__restrict__ h) {
     // The codebook in shared memory, filled before the wait: 32 lanes that look up different entries are one request with
@@ -214,10 +214,10 @@ __global__ void __launch_bounds__(512) moe_gux_k(const uint8_t *__restrict__ bg,
 }
 
 // ---- down projection with Q2_0 rows: the counterpart of moe_ya4_k (same split) ----
-__global__ void moe_ya20_k(const uint8_t *__restrict__ bd, uint64_t stride, const int32_t *__restrict__ slots,
-                           const float *__restrict__ wts, uint32_t n_host, const int32_t *__restrict__ n_dev,
-                           const int8_t *__restrict__ hq, const float *__restrict__ hd,
-                           const int32_t *__restrict__ hbs, uint64_t q_slice, uint64_t d_slice, uint32_t n_ff,
+__global__ void moe_ya20_k(const uint8_t *__restrict__ bd, uint64_t stride, const int32_t *slots,
+                           const float *wts, uint32_t n_host, const int32_t *n_dev,
+                           const int8_t *hq, const float *hd,
+                           const int32_t *hbs, uint64_t q_slice, uint64_t d_slice, uint32_t n_ff,
                            uint32_t n_embd, float *__restrict__ y) {
     q4b_pdl_wait();
     const uint32_t row = blockIdx.x * 2u + (threadIdx.x >> 7), lane = threadIdx.x & 127u;

@@ -44,7 +44,7 @@ struct Smem {
     uint32_t done[MAX_STAGE];                    // warps that are through with a stage's chunk
     // where the two streams stand (entry of the live list, block of rows): chunks, activation rows
     uint32_t p_li, p_blk, p_ch, p_nb, x_li, x_blk, x_item;
-    bool p_new;
+    uint32_t i_row[2], i_nr[2], i_nb[2];         // item in an activation buffer: first row, rows, blocks of its entry
     const uint8_t *p_mat;
     alignas(16) float red[NCW - 2][32][4];                // partial sums of warps that share a unit (all but one of each unit)
     uint32_t live[MAX_ENTRIES];                  // entries with rows
@@ -247,33 +247,38 @@ template <typename Body> __device__ __forceinline__ void stream_items(const Args
     // that has become free (one lane; refills come in order, because a warp leaves chunk k + 1 only after it has
     // refilled behind chunk k).
     const uint32_t blk_end = ix_end / cpe, ch_end = ix_end - blk_end * cpe, chunk_bytes = a.chunk_bytes;
-    auto rows_of = [&](uint32_t e) { return (uint32_t)(__ldg(a.bounds + e + 1) - __ldg(a.bounds + e)); };
+    auto enter = [&](uint32_t pl) {   // the entry whose chunks come next (behind the copy before: its loads take a while)
+        const uint32_t e = s.live[pl];
+        const int32_t b0 = a.bounds[e], b1 = a.bounds[e + 1], slot = a.act ? a.act[e] : (int32_t)e;
+        s.p_nb = split_rows((uint32_t)(b1 - b0)).nb;
+        s.p_mat = a.w + (uint64_t)slot * a.expert_stride;
+    };
     auto refill = [&](uint32_t st) {
         uint32_t pl = s.p_li, pb = s.p_blk, pc = s.p_ch;
         if (pl == li_end && pb == blk_end && pc == ch_end) return;
-        if (s.p_new) {
-            const uint32_t e = s.live[pl];
-            s.p_nb = split_rows(rows_of(e)).nb;
-            s.p_mat = a.w + (uint64_t)(a.act ? __ldg(a.act + e) : (int32_t)e) * a.expert_stride;
-        }
         const uint32_t bytes = pc + 1u == cpe ? a.last_bytes : chunk_bytes;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&s.full[st])), "r"(bytes) : "memory");
         bulk_g2s(stage + st * chunk_bytes, s.p_mat + (uint64_t)pc * chunk_bytes, bytes, &s.full[st]);
-        bool next = false;
         if (++pc == cpe) {
             pc = 0;
-            if (++pb == s.p_nb) pb = 0, pl++, next = true;
+            if (++pb == s.p_nb) {
+                pb = 0;
+                if (++pl < n_live) enter(pl);
+            }
         }
-        s.p_li = pl, s.p_blk = pb, s.p_ch = pc, s.p_new = next;
+        s.p_li = pl, s.p_blk = pb, s.p_ch = pc;
     };
     auto refill_rows = [&]() {
         uint32_t xl = s.x_li, xb = s.x_blk;
         if (xl > li_end || (xl == li_end && (xb > blk_end || (xb == blk_end && ch_end == 0)))) return;   // past the share
-        const uint32_t e = s.live[xl], rows = rows_of(e), buf = s.x_item & 1u, sb = (a.cols >> 5) * 4u;
+        const uint32_t e = s.live[xl], buf = s.x_item & 1u, sb = (a.cols >> 5) * 4u;
+        const int32_t b0 = a.bounds[e], b1 = a.bounds[e + 1];
+        const uint32_t rows = (uint32_t)(b1 - b0);
         const Split sp = split_rows(rows);
         const uint32_t nr = min(sp.per, rows - xb * sp.per);
-        const uint64_t r0 = (uint64_t)__ldg(a.bounds + e) + xb * sp.per;
+        const uint64_t r0 = (uint64_t)b0 + xb * sp.per;
         uint8_t *const ab = actb + buf * act_sz;
+        s.i_row[buf] = (uint32_t)r0, s.i_nr[buf] = nr, s.i_nb[buf] = sp.nb;   // seen by who waits for the copies
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&s.act_full[buf])),
                      "r"(nr * (a.cols + sb))
                      : "memory");
@@ -285,7 +290,8 @@ template <typename Body> __device__ __forceinline__ void stream_items(const Args
         s.x_li = xl, s.x_blk = xb, s.x_item++;
     };
     if (tid == 0 && (li != li_end || ix != ix_end)) {
-        s.p_li = s.x_li = li, s.p_blk = s.x_blk = ix / cpe, s.p_ch = ix % cpe, s.p_new = true, s.x_item = 0;
+        s.p_li = s.x_li = li, s.p_blk = s.x_blk = ix / cpe, s.p_ch = ix % cpe, s.x_item = 0;
+        enter(li);
         refill_rows();
         for (uint32_t i = 0; i < a.n_stage; i++) refill(i);
         refill_rows();
@@ -293,22 +299,13 @@ template <typename Body> __device__ __forceinline__ void stream_items(const Args
 
     // ---- the warps ----
     uint32_t st = 0, ph = 0, item = 0, limit = WAIT_LIMIT, blk = ix / cpe, ch = ix - blk * cpe;
-    bool entry = true;
-    uint32_t rows = 0;
-    Split sp = {1u, 0u};
     // one item: a chunk after the other
     while (li != li_end || blk != blk_end || ch != ch_end) {
-        const uint32_t e = s.live[li];
-        const int32_t r0 = __ldg(a.bounds + e);
-        if (entry) {
-            rows = (uint32_t)(__ldg(a.bounds + e + 1) - r0);
-            sp = split_rows(rows);
-        }
-        entry = false;
-        const uint32_t nr = min(sp.per, rows - blk * sp.per), buf = item & 1u;
-        float *const out = a.dst + (uint64_t)((uint32_t)r0 + blk * sp.per) * a.ld_dst;
+        const uint32_t buf = item & 1u;
         const uint8_t *const ab = actb + buf * act_sz, *const sbase = ab + sc_off;
         if (!mbar_wait(&s.act_full[buf], (item >> 1) & 1u, limit, a.err)) limit = 1024u;
+        const uint32_t nr = s.i_nr[buf], nb = s.i_nb[buf];
+        float *const out = a.dst + (uint64_t)s.i_row[buf] * a.ld_dst;
         const uint32_t ch_stop = li == li_end && blk == blk_end ? ch_end : cpe;
         auto acquire = [&]() {
             if (!mbar_wait(&s.full[st], ph, limit, a.err)) limit = 1024u;
@@ -332,7 +329,7 @@ template <typename Body> __device__ __forceinline__ void stream_items(const Args
         if (ch_stop != cpe) break;         // the end of this CTA's share
         item++;
         ch = 0, blk++;
-        if (blk == sp.nb) blk = 0, li++, entry = true;
+        if (blk == nb) blk = 0, li++;
     }
 }
 

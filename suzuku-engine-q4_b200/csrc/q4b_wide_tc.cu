@@ -72,8 +72,8 @@ constexpr uint32_t W_SMEM = W_B_OFF + W_STAGES * W_STAGE_BYTES + W_DG * NDW * 10
 static_assert(W_SMEM <= 227u * 1024u, "shared memory layout");
 
 // The passes of every entry: its rows split evenly over as few passes of nb rows as hold them.
-__global__ void __launch_bounds__(1024) worklist_wide_k(const int32_t *__restrict__ bounds,
-                                                        const uint32_t *__restrict__ n_act, uint32_t n_entries,
+__global__ void __launch_bounds__(1024) worklist_wide_k(const int32_t *bounds,
+                                                        const uint32_t *n_act, uint32_t n_entries,
                                                         uint4 *__restrict__ work,
                                                         uint32_t *__restrict__ n_work, uint32_t cap) {
     __shared__ uint32_t wsum[32];
@@ -172,6 +172,18 @@ __device__ __forceinline__ uint4 decode_word_h(uint32_t x, __half2 L, __half2 C,
     r.z = h2_bits(__hfma2(as_h2((u & 0x001e001eu) ^ 0x64116411u), L, C));
     r.w = h2_bits(__hfma2(as_h2((u & 0x01e001e0u) ^ 0x65106510u), L16, C16));
     return r;
+}
+
+// store_tile (q4b_mmq_tc.cu) with the row scales held by the warp's lanes: column j's by lane at + j.  (Loaded there, they
+// would have to be loaded before the first store, which could alias them.)
+__device__ __noinline__ void store_tile_lanes(float *o, uint64_t ld, float rs, uint32_t at, uint32_t n, float4 a0, float4 a1,
+                                              float4 a2, float4 a3) {
+    const float v[16] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w, a3.x, a3.y, a3.z, a3.w};
+#pragma unroll
+    for (uint32_t j = 0; j < 16; j++) {
+        const float s = __shfl_sync(0xffffffffu, rs, at + j);
+        if (j < n) o[(uint64_t)j * ld] = v[j] * s;
+    }
 }
 
 // An accumulator is one step (128 k): the MMAs of the second activation plane, whose products are 2^-11 of the others',
@@ -354,6 +366,12 @@ __global__ void __launch_bounds__(NT, 1) mmq_wide_k(const WArgs a, const __grid_
             // -- the super-blocks to retire
             uint32_t r_i = 0, r_tb = 0, r_m = 0;
             uint32_t r_rows = s.items[0].nrows;
+            static_assert(W_NSL == 2, "a lane holds the scale of one column of the two slabs");
+            auto row_scale = [&](uint32_t i) {     // of this warp's columns of item i
+                const uint32_t c = 16u * (e_cs + 4u * (lane >> 4)) + (lane & 15u);
+                return c < s.items[i].nrows ? a.rs[s.items[i].rc + (int32_t)c] : 0.f;
+            };
+            float r_scale = row_scale(0);
             auto fold = [&](uint32_t g, uint32_t half) {    // fold a complete step's accumulator into the sums
                 tc_fence_after();
                 const float dr = __half2float(__ushort_as_half(s.dr[g & 7u][e_row]));
@@ -377,19 +395,19 @@ __global__ void __launch_bounds__(NT, 1) mmq_wide_k(const WArgs a, const __grid_
                     for (uint32_t h = 0; h < W_NSL; h++) {
                         const uint32_t cs = e_cs + 4u * h;
                         if (16u * cs < r_rows)
-                            store_tile(a.dst + (uint64_t)(m.rc + 16 * (int32_t)cs) * a.ld_dst + m.row0 + r_m * MT + e_row,
-                                       a.ld_dst, a.rs + m.rc + 16 * (int32_t)cs, min(16u, r_rows - 16u * cs),
-                                       make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]),
-                                       make_float4(acc[h][4], acc[h][5], acc[h][6], acc[h][7]),
-                                       make_float4(acc[h][8], acc[h][9], acc[h][10], acc[h][11]),
-                                       make_float4(acc[h][12], acc[h][13], acc[h][14], acc[h][15]));
+                            store_tile_lanes(a.dst + (uint64_t)(m.rc + 16 * (int32_t)cs) * a.ld_dst + m.row0 + r_m * MT + e_row,
+                                             a.ld_dst, r_scale, 16u * h, min(16u, r_rows - 16u * cs),
+                                             make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]),
+                                             make_float4(acc[h][4], acc[h][5], acc[h][6], acc[h][7]),
+                                             make_float4(acc[h][8], acc[h][9], acc[h][10], acc[h][11]),
+                                             make_float4(acc[h][12], acc[h][13], acc[h][14], acc[h][15]));
 #pragma unroll
                         for (int c = 0; c < 16; c++) acc[h][c] = 0.f;
                     }
                     r_tb = 0;
                     if (++r_m == a.mt) {
                         r_m = 0;
-                        if (++r_i < n_here) r_rows = s.items[r_i].nrows;
+                        if (++r_i < n_here) r_rows = s.items[r_i].nrows, r_scale = row_scale(r_i);
                     }
                 }
             };
