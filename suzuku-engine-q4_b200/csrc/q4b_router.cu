@@ -8,6 +8,7 @@
 // its additions to nearest, the large products (x1 W1) have an accumulator of their own, an accumulator takes 128 h only,
 // and both are then added to fp32 registers on the CUDA cores (one accumulator for all six: 2.2 times the largest error of 257 x 48 logits).  The logits are as close to the exact product as those of the fp32 kernel it replaces, whose 2048 terms were
 // added one after the other, and there is no common scale per row, so a row with an outlier keeps its small values.
+// A logit that does not come out finite is formed again as that kernel did.
 //
 // The fp32 kernel was bound by shared-memory bandwidth (three 16-byte loads per 32 multiply-adds): 130 us for 2048 x 512
 // x 2048, 445 for 8192 tokens; this one takes 50 and 192.  A CTA here owns 128 tokens x 64 experts; its 8 warps load, split and store both
@@ -133,6 +134,17 @@ __global__ void __launch_bounds__(NT, 1) router_tc_k(const float *__restrict__ W
     fold(((nk - 1u) >> 1) & 1u);
     const uint32_t t = t0 + 32u * (warp & 3u) + lane, c0 = e0 + 32u * (warp >> 2);
     if (t < n_tok) {
+        // An operand that is infinite, or that bf16 rounds to infinity, leaves NaN in the parts that remain of it, and partial
+        // products may overflow where their sum does not: such logits are formed as one fp32 sum.
+        auto plain = [&](uint32_t e) {
+            const float *x = X + (uint64_t)t * ncols, *w = W + (uint64_t)e * ncols;
+            float v = 0.f;
+            for (uint32_t h = 0; h < ncols; h++) v = fmaf(x[h], w[h], v);
+            return v;
+        };
+#pragma unroll
+        for (int i = 0; i < 32; i++)
+            if (!isfinite(acc[i]) && c0 + i < nrows) acc[i] = plain(c0 + i);
         float *y = Y + (uint64_t)t * nrows + c0;
         if ((nrows & 3u) == 0 && c0 + 32u <= nrows) {
 #pragma unroll

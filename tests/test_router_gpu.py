@@ -47,3 +47,33 @@ def test_row_bits_without_tensor_cores(dev, n_tok, mode):
     for t in (0, 128, n_tok - 1):
         assert dev.lib.q4_hip_gemv_dd(0, d_w, n_exp, n, d_x + t * n * 4, d_1, 1.0)
         assert np.array_equal(y[t].view(np.uint32), dev.download(d_1, (n_exp,), np.float32).view(np.uint32))
+
+
+def test_infinite_operands_and_overflowing_parts(dev):
+    """Infinities, NaN and values at the top of the fp32 range give what a sum of fp32 products gives, and leave the other
+    logits alone."""
+    lib, (n, e, h) = dev.lib, (300, 72, 512)
+    rng = np.random.default_rng(3)
+    x, w = rng.standard_normal((n, h)).astype(np.float32), rng.standard_normal((e, h)).astype(np.float32)
+    x[5, 7], x[6, 8], x[9, 500] = np.inf, -np.inf, np.nan
+    x[10, 3], w[3, 3] = 3.4e38, 0.5                       # rounds to infinity as a bf16 value
+    w[:, 3] = np.where(np.arange(e) == 3, 0.5, 0.0)
+    w[11, 100], w[12, 101] = -np.inf, np.nan
+    x[20, :2], w[20, :] = 3e38, 0.0
+    w[20, :2] = 1.0, -1.0
+    with np.errstate(all="ignore"):
+        want = (x[:, None, :].astype(np.float64) * w[None]).sum(2)
+        want = np.where(np.abs(want) > np.finfo(np.float32).max, np.sign(want) * np.inf, want)
+    d_y = dev.malloc(n * e * 4)
+    assert lib.q4_hip_gemv_dd_n(0, dev.upload(w), e, h, dev.upload(x), d_y, 1.0, n)
+    y = dev.download(d_y, (n, e), np.float32)
+    keep = np.ones_like(y, bool)
+    keep[20] = False                                      # fp32 sums of this token overflow or not by their order ...
+    keep[20, 20] = True                                   # ... but for this expert
+    assert np.array_equal(np.isnan(y)[keep], np.isnan(want)[keep])
+    assert np.array_equal(y[keep & np.isinf(want)], want[keep & np.isinf(want)].astype(np.float32))
+    fin = keep & np.isfinite(want)
+    with np.errstate(all="ignore"):
+        mag, off = np.abs(x[:, None, :].astype(np.float64) * w[None]).sum(2), np.abs(y - want)
+    assert (off[fin] <= h * 2.0 ** -24 * mag[fin]).all()   # of h fp32 additions
+    assert lib.q4_cuda_device_error() == 0
