@@ -102,7 +102,7 @@ void q4_hip_graph_free(void *exec);
  * expert.  d_h receives the n*n_ff fp32 hidden rows.  d_h2/d_down are unused
  * scratch of the reference's unfused fallback and may be NULL.  n <= 64.
  * exec: slots/wts are HOST arrays.  exec_dev: device arrays and a device
- * count.  stage + exec_staged: the host writes the list into mapped memory,
+ * count (of which at most 64 entries are taken).  stage + exec_staged: the host writes the list into mapped memory,
  * the launch reads it at run time (graph replay with new routing). */
 bool q4_hip_moe_tok_ok(uint32_t gt, uint32_t ut, uint32_t dt, uint32_t in_dim, uint32_t n_ff);
 bool q4_hip_moe_exec(const uint8_t *base, uint64_t stride, const int32_t *slots,

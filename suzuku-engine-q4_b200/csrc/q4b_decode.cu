@@ -497,6 +497,11 @@ __global__ void __launch_bounds__(256) route_small_k(const float *x, const float
                           wts + (uint64_t)(t0 + warp) * topk, -1, nullptr, lane);
 }
 
+// Entries of an exec call: the host's number, or the device's, of which no more than the lists' and the hidden rows' 64 count.
+__device__ __forceinline__ uint32_t exec_count(const int32_t *n_dev, uint32_t n_host) {
+    return n_dev ? (uint32_t)max(0, min(*n_dev, 64)) : n_host;
+}
+
 // ------------------------------------------------------------------ gate/up + SwiGLU
 // grid (n_ff/8, experts or fewer), 8 warps per block, one warp per hidden unit f, experts in strides of grid.y:
 // h[e][f] = silu(gate_f . xq) * (up_f . xq).
@@ -514,7 +519,7 @@ __global__ void moe_gu_k(const uint8_t *__restrict__ bg, const uint8_t *__restri
     int *sb = reinterpret_cast<int *>(smem + 2048 + in_dim + 4 * ng);
     q4b_fill_code_table(tab);
     q4b_pdl_wait();
-    const uint32_t n = n_dev ? (uint32_t)*n_dev : gridDim.y;
+    const uint32_t n = exec_count(n_dev, gridDim.y);
     if (blockIdx.y >= n) return;
     for (uint32_t i = threadIdx.x; i < in_dim / 4; i += blockDim.x)
         sq[i] = reinterpret_cast<const int *>(xq)[i];
@@ -571,7 +576,7 @@ __global__ void moe_ya_k(const uint8_t *__restrict__ bd, uint64_t stride,
     const uint32_t r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= n_embd) return;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t n = n_dev ? (uint32_t)*n_dev : n_host;
+    const uint32_t n = exec_count(n_dev, n_host);
     const uint32_t ng = n_ff >> 5;
     const uint32_t nbr = n_ff >> 8;
     float acc = 0.f;
@@ -712,7 +717,7 @@ __global__ void moe_gu4_k(const uint8_t *__restrict__ bg, const uint8_t *__restr
     q4b_pdl_wait();
     const uint32_t f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (f >= n_ff) return;
-    const uint32_t lane = threadIdx.x & 31u, ng = in_dim >> 5, n = n_dev ? (uint32_t)*n_dev : gridDim.y;
+    const uint32_t lane = threadIdx.x & 31u, ng = in_dim >> 5, n = exec_count(n_dev, gridDim.y);
     const uint64_t rb = iq4_row_bytes(T, in_dim);
     for (uint32_t e = blockIdx.y; e < n; e += gridDim.y) {
         const uint8_t *rg = bg + (uint64_t)slots[e] * stride + (uint64_t)f * rb;
@@ -759,7 +764,7 @@ __global__ void moe_ya4_k(const uint8_t *__restrict__ bd, uint64_t stride, const
     q4b_pdl_wait();
     const uint32_t row = blockIdx.x * 2u + (threadIdx.x >> 7), lane = threadIdx.x & 127u;
     const uint32_t r = min(row, n_embd - 1u);   // an odd last CTA: its second half is computed and dropped
-    const uint32_t n = n_dev ? (uint32_t)*n_dev : n_host;
+    const uint32_t n = exec_count(n_dev, n_host);
     const uint32_t ng = n_ff >> 5;
     const uint64_t rb = iq4_row_bytes(T, n_ff);
     float acc = 0.f;

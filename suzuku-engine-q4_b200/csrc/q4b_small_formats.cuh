@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(512) moe_gux_k(const uint8_t *__restrict__ bg,
     q4b_pdl_wait();
     const uint32_t f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (f >= n_ff) return;
-    const uint32_t lane = threadIdx.x & 31u, ng = in_dim >> 5, n = n_dev ? (uint32_t)*n_dev : gridDim.y;
+    const uint32_t lane = threadIdx.x & 31u, ng = in_dim >> 5, n = exec_count(n_dev, gridDim.y);
     const uint64_t rb = small_row_bytes(T, in_dim);
     for (uint32_t e = blockIdx.y; e < n; e += gridDim.y) {
         const uint8_t *rg = bg + (uint64_t)slots[e] * stride + (uint64_t)f * rb;
@@ -222,7 +222,7 @@ __global__ void moe_ya20_k(const uint8_t *__restrict__ bd, uint64_t stride, cons
     q4b_pdl_wait();
     const uint32_t row = blockIdx.x * 2u + (threadIdx.x >> 7), lane = threadIdx.x & 127u;
     const uint32_t r = min(row, n_embd - 1u);   // an odd last CTA: its second half is computed and dropped   // (n_embd is even)
-    const uint32_t n = n_dev ? (uint32_t)*n_dev : n_host;
+    const uint32_t n = exec_count(n_dev, n_host);
     const uint32_t ng = n_ff >> 5;
     const uint64_t rb = small_row_bytes(Q4_T_Q2_0, n_ff);
     float acc = 0.f;

@@ -245,3 +245,47 @@ def test_many_token_layer_with_other_formats(dev, pkg, oracle, H, F, gu, dn, n_t
         assert lib.q4_cuda_device_error() == 0
     finally:
         lib.q4_hip_experts_free_a(3)
+
+
+@pytest.mark.parametrize("gu,dn,tiled", [(IQ3_S, IQ3_S, 2), (IQ3_S, IQ3_S, 0), (IQ4_XS, IQ4_NL, 0), (IQ2_S, Q2_0, 0)])
+def test_device_counts_up_to_and_beyond_the_lists(dev, pkg, gu, dn, tiled):
+    """A count on the device: entries are walked in strides of 16 (the grid is cut for that many), none are left out up to
+    64, and a larger or a negative count neither computes nor writes a 65th hidden row."""
+    H, F, slots_n = 512, 256, 6
+    rng = np.random.default_rng(gu + dn + tiled)
+    packs = pkg.synth.expert_packs_typed(rng, slots_n, H, F, gu, dn)
+    lib = dev.lib
+    lib.q4_cuda_set_tiled_default(tiled)
+    try:
+        assert lib.q4_hip_experts_alloc_a(3, slots_n, packs.shape[1])
+    finally:
+        lib.q4_cuda_set_tiled_default(1)
+    try:
+        for e in range(slots_n):
+            row = np.ascontiguousarray(packs[e])
+            assert lib.q4_hip_experts_put_a(3, e, row.ctypes.data, row.nbytes)
+        base, stride, rb = lib.q4_hip_experts_base_a(3), lib.q4_hip_experts_stride_a(3), pkg.synth.row_bytes(gu, H)
+        slots, wts = rng.integers(0, slots_n, 72).astype(np.int32), rng.random(72).astype(np.float32)
+        d_x, d_s, d_w = dev.upload(rng.standard_normal(H).astype(np.float32)), dev.upload(slots), dev.upload(wts)
+        d_h, d_y, d_n = dev.malloc(72 * F * 4), dev.malloc(H * 4), dev.malloc(4)
+
+        def run(count, host):
+            dev.write(d_h, np.full((72, F), 7.5, np.float32))
+            dev.write(d_n, np.array([count], np.int32))
+            assert lib.q4_hip_fill(d_y, 0.0, H)
+            tail = (gu, 0, gu, F * rb, dn, 2 * F * rb, d_x, d_h, None, None, d_y, F, H, H)
+            if host:
+                assert lib.q4_hip_moe_exec(base, stride, slots.ctypes.data, wts.ctypes.data, count, *tail)
+            else:
+                assert lib.q4_hip_moe_exec_dev(base, stride, d_s, d_w, d_n, *tail)
+            return dev.download(d_y, (H,), np.float32), dev.download(d_h, (72, F), np.float32)
+        for count in (1, 15, 16, 17, 33, 64, 66):
+            y, h = run(count, False)
+            y0, h0 = run(min(count, 64), True)
+            assert np.array_equal(h, h0) and (h[min(count, 64):] == 7.5).all(), count
+            assert np.linalg.norm(y - y0) <= 1e-6 * np.linalg.norm(y0), count
+        y, h = run(-1, False)
+        assert (h[64:] == 7.5).all() and not y.any()
+        assert lib.q4_cuda_device_error() == 0
+    finally:
+        lib.q4_hip_experts_free_a(3)
