@@ -24,6 +24,20 @@ constexpr uint32_t A_PLANE = BM * 128u, B_PLANE = BN * 128u;            // [row]
 constexpr uint32_t BUF = 3u * (A_PLANE + B_PLANE), SMEM = 2u * BUF + 1024u;
 constexpr uint32_t ERR_ROUTER = 0x2000u;
 
+// An operand that is infinite, or that bf16 rounds to infinity, leaves NaN in the parts that remain of it, and partial
+// products may overflow where their sum does not: the logits of a token's 32 experts that did not come out finite are formed
+// again as fp32 sums.  (Not inlined: unrolled in the kernel it cost every call 6 us.)
+__device__ __noinline__ void plain_logits(const float *W, uint32_t nrows, uint32_t ncols, const float *x, float *y, uint32_t c0,
+                                          float scale) {
+    for (uint32_t i = 0; i < 32u && c0 + i < nrows; i++) {
+        if (isfinite(y[i])) continue;
+        const float *w = W + (uint64_t)(c0 + i) * ncols;
+        float v = 0.f;
+        for (uint32_t h = 0; h < ncols; h++) v = fmaf(x[h], w[h], v);
+        y[i] = scale * v;
+    }
+}
+
 __global__ void __launch_bounds__(NT, 1) router_tc_k(const float *__restrict__ W, uint32_t nrows, uint32_t ncols,
                                                      const float *__restrict__ X, uint32_t n_tok, float *__restrict__ Y,
                                                      float scale, uint32_t *__restrict__ err) {
@@ -134,17 +148,6 @@ __global__ void __launch_bounds__(NT, 1) router_tc_k(const float *__restrict__ W
     fold(((nk - 1u) >> 1) & 1u);
     const uint32_t t = t0 + 32u * (warp & 3u) + lane, c0 = e0 + 32u * (warp >> 2);
     if (t < n_tok) {
-        // An operand that is infinite, or that bf16 rounds to infinity, leaves NaN in the parts that remain of it, and partial
-        // products may overflow where their sum does not: such logits are formed as one fp32 sum.
-        auto plain = [&](uint32_t e) {
-            const float *x = X + (uint64_t)t * ncols, *w = W + (uint64_t)e * ncols;
-            float v = 0.f;
-            for (uint32_t h = 0; h < ncols; h++) v = fmaf(x[h], w[h], v);
-            return v;
-        };
-#pragma unroll
-        for (int i = 0; i < 32; i++)
-            if (!isfinite(acc[i]) && c0 + i < nrows) acc[i] = plain(c0 + i);
         float *y = Y + (uint64_t)t * nrows + c0;
         if ((nrows & 3u) == 0 && c0 + 32u <= nrows) {
 #pragma unroll
@@ -155,6 +158,10 @@ __global__ void __launch_bounds__(NT, 1) router_tc_k(const float *__restrict__ W
             for (int i = 0; i < 32; i++)
                 if (c0 + i < nrows) y[i] = scale * acc[i];
         }
+        float z = 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; i++) z = fmaf(acc[i], 0.f, z);
+        if (z != 0.f) plain_logits(W, nrows, ncols, X + (uint64_t)t * ncols, y, c0, scale);   // NaN: one is not finite
     }
     __syncthreads();
     if (warp == 0) {
