@@ -53,10 +53,67 @@ bool tiled_default() {
     return g_tiled_default != 0;
 }
 
-// In-place regrouping of runs of eight 110-byte super-blocks into tiles
-// (forward) or back (inverse).  One warp per tile via shared memory.
-template <bool FORWARD>
-__global__ void tile_permute_k(uint8_t *data, uint64_t n_tiles) {
+// The wide form of a tile (q4b_tile.cuh), a warp a tile: this lane's two groups, from their fields in tiled order.
+__device__ __forceinline__ void widen_groups(uint8_t *o, uint32_t lane, uint4 qs, uint2 sg, uint32_t qh, const uint32_t *tab) {
+    uint32_t n[2][8];   // c' of the groups, one nibble per byte, in weight order
+#pragma unroll
+    for (uint32_t h = 0; h < 2; h++)
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++) {
+            const uint32_t w = h ? (k < 4 ? qs.z : qs.w) : (k < 4 ? qs.x : qs.y);
+            const uint32_t idx = ((w >> (8u * (k & 3u))) & 0xffu) | (((qh >> (8u * h + k)) & 1u) << 8);
+            const uint32_t t4 = (h ? sg.y : sg.x) << k;
+            n[h][k] = (tab[idx] ^ q4b_prmt(t4, t4, 0xba98u)) & 0x0f0f0f0fu;   // c or ~c
+        }
+#pragma unroll
+    for (uint32_t t4 = 0; t4 < 4; t4++)
+        *reinterpret_cast<uint2 *>(o + Q4B_WIDE_PART * t4 + 8u * lane) =
+            make_uint2(n[0][2 * t4] | (n[0][2 * t4 + 1] << 4), n[1][2 * t4] | (n[1][2 * t4 + 1] << 4));
+}
+// ... and the record of super-block k: d and the four sub-scale bytes
+__device__ __forceinline__ void widen_record(uint8_t *o, uint32_t k, uint32_t d, uint32_t scales) {
+    *reinterpret_cast<uint2 *>(o + Q4B_WIDE_PART * (k >> 1) + 256u + 8u * (k & 1u)) = make_uint2(d, scales);
+}
+__device__ __forceinline__ void load_codes(uint32_t *tab, const uint32_t *codes) {
+    for (uint32_t i = threadIdx.x; i < 512u; i += blockDim.x) tab[i] = __ldg(codes + i);
+    __syncthreads();
+}
+
+// In-place regrouping of runs of eight 110-byte super-blocks into tiles, one warp per tile: the tile is brought into shared
+// memory, each lane picks the fields of its two groups and writes them as words.  wide (or NULL): where the
+// tiles' wide form goes, made from the same registers.  513 packs of 2048 x 512 (1.5 GB read and written): 519 us.  (984
+// us with every byte stored by itself, and 288 more for a second kernel that read the tiles back to widen them.)
+__global__ void __launch_bounds__(256) tile_put_k(uint8_t *data, uint64_t n_tiles, uint8_t *wide, const uint32_t *codes) {
+    __shared__ __align__(16) uint8_t buf[8][Q4B_TILE_BYTES];
+    __shared__ uint32_t tab[512];
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u, k = lane >> 2, q = lane & 3u;
+    if (wide) load_codes(tab, codes);
+    // engine layout of block k: 110k + {0: d, 2: qs[64], 66: qh[8], 74: signs[32], 106: scales[4]}
+    const uint8_t *const b = buf[w], *const blk = b + 110u * k;
+    for (uint64_t t = (uint64_t)blockIdx.x * 8u + w; t < n_tiles; t += (uint64_t)gridDim.x * 8u) {
+        uint8_t *const p = data + t * Q4B_TILE_BYTES, *const o = wide + t * Q4B_WIDE_BYTES;
+        for (uint32_t i = lane; i < Q4B_TILE_BYTES / 16; i += 32)
+            reinterpret_cast<uint4 *>(buf[w])[i] = reinterpret_cast<const uint4 *>(p)[i];
+        __syncwarp();
+        const uint8_t *const a = blk + 2u + 16u * q, *const g = blk + 74u + 8u * q;
+        const uint4 qs = make_uint4(q4b_ld_u32_a2(a), q4b_ld_u32_a2(a + 4), q4b_ld_u32_a2(a + 8), q4b_ld_u32_a2(a + 12));
+        const uint2 sg = make_uint2(q4b_sign_permute(q4b_ld_u32_a2(g)), q4b_sign_permute(q4b_ld_u32_a2(g + 4)));
+        const uint32_t qh = q4b_ld_u16(blk + 66u + 2u * q);
+        *reinterpret_cast<uint4 *>(p + Q4B_TILE_OFF_QS + 16u * lane) = qs;
+        *reinterpret_cast<uint2 *>(p + Q4B_TILE_OFF_SG + 8u * lane) = sg;
+        *reinterpret_cast<uint16_t *>(p + Q4B_TILE_OFF_QH + 2u * lane) = (uint16_t)qh;
+        if (wide) widen_groups(o, lane, qs, sg, qh, tab);
+        if (lane < 8) {
+            const uint32_t d = q4b_ld_u16(b + 110u * lane), sc = q4b_ld_u32_a2(b + 110u * lane + 106u);
+            *reinterpret_cast<uint16_t *>(p + Q4B_TILE_OFF_D + 2u * lane) = (uint16_t)d;
+            *reinterpret_cast<uint32_t *>(p + Q4B_TILE_OFF_SC + 4u * lane) = sc;
+            if (wide) widen_record(o, lane, d, sc);
+        }
+        __syncwarp();
+    }
+}
+// Back to the engine's order.
+__global__ void __launch_bounds__(256) tile_get_k(uint8_t *data, uint64_t n_tiles) {
     __shared__ __align__(16) uint8_t buf[8][Q4B_TILE_BYTES];
     const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint64_t t = (uint64_t)blockIdx.x * 8u + w;
@@ -66,86 +123,65 @@ __global__ void tile_permute_k(uint8_t *data, uint64_t n_tiles) {
     for (uint32_t i = lane; i < Q4B_TILE_BYTES / 16; i += 32)
         reinterpret_cast<uint4 *>(b)[i] = reinterpret_cast<const uint4 *>(p)[i];
     __syncwarp();
-    // engine layout of block k: 110k + {0: d, 2: qs[64], 66: qh[8], 74: signs[32], 106: scales[4]}
     for (uint32_t i = lane; i < Q4B_TILE_BYTES; i += 32) {
         const uint32_t k = i / 110u, o = i - k * 110u;
-        uint32_t to;
+        uint32_t from;
         if (o < 2)
-            to = Q4B_TILE_OFF_D + 2 * k + o;
+            from = Q4B_TILE_OFF_D + 2 * k + o;
         else if (o < 66)
-            to = Q4B_TILE_OFF_QS + 64 * k + (o - 2);
+            from = Q4B_TILE_OFF_QS + 64 * k + (o - 2);
         else if (o < 74)
-            to = Q4B_TILE_OFF_QH + 8 * k + (o - 66);
+            from = Q4B_TILE_OFF_QH + 8 * k + (o - 66);
         else if (o < 106)
-            to = Q4B_TILE_OFF_SG + 32 * k + (o - 74);
+            continue;  // sign words: below
         else
-            to = Q4B_TILE_OFF_SC + 4 * k + (o - 106);
-        if (o >= 74 && o < 106) continue;  // sign words: handled below, as words
-        if (FORWARD)
-            p[to] = b[i];
-        else
-            p[i] = b[to];
+            from = Q4B_TILE_OFF_SC + 4 * k + (o - 106);
+        p[i] = b[from];
     }
     for (uint32_t g = lane; g < 64; g += 32) {  // 64 sign words per tile
-        const uint32_t k = g >> 3, ib = g & 7u;
-        const uint32_t eng = 110u * k + 74u + 4u * ib, til = Q4B_TILE_OFF_SG + 32u * k + 4u * ib;
-        if (FORWARD) {
-            const uint32_t w32 = b[eng] | (b[eng + 1] << 8) | (b[eng + 2] << 16) | ((uint32_t)b[eng + 3] << 24);
-            *reinterpret_cast<uint32_t *>(p + til) = q4b_sign_permute(w32);
-        } else {
-            const uint32_t w32 = q4b_sign_unpermute(*reinterpret_cast<const uint32_t *>(b + til));
-            p[eng] = (uint8_t)w32;
-            p[eng + 1] = (uint8_t)(w32 >> 8);
-            p[eng + 2] = (uint8_t)(w32 >> 16);
-            p[eng + 3] = (uint8_t)(w32 >> 24);
-        }
+        const uint32_t w32 = q4b_sign_unpermute(*reinterpret_cast<const uint32_t *>(b + Q4B_TILE_OFF_SG + 4u * g));
+        const uint32_t eng = 110u * (g >> 3) + 74u + 4u * (g & 7u);
+        for (uint32_t i = 0; i < 4; i++) p[eng + i] = (uint8_t)(w32 >> (8u * i));
     }
 }
 
-bool launch_tile_permute(uint8_t *data, uint64_t bytes, bool forward, cudaStream_t st) {
-    const uint64_t n_tiles = bytes / Q4B_TILE_BYTES;
-    if (n_tiles == 0) return true;
-    const unsigned nb = (unsigned)((n_tiles + 7) / 8);
-    if (forward)
-        tile_permute_k<true><<<nb, 256, 0, st>>>(data, n_tiles);
-    else
-        tile_permute_k<false><<<nb, 256, 0, st>>>(data, n_tiles);
+unsigned tile_ctas(uint64_t n_tiles) {
+    const uint64_t nb = (n_tiles + 7) / 8;
+    return (unsigned)(nb < 8u * 148u ? nb : 8u * 148u);
+}
+// Arena bytes [off, off + bytes) are in engine byte order: tiles, and their wide form.
+bool launch_tile_put(const Arena &a, uint64_t off, uint64_t bytes, cudaStream_t st) {
+    const uint64_t n = bytes / Q4B_TILE_BYTES;
+    if (n == 0) return true;
+    tile_put_k<<<tile_ctas(n), 256, 0, st>>>(a.base + off, n, a.wide ? a.wide + off / Q4B_TILE_BYTES * Q4B_WIDE_BYTES : nullptr,
+                                             g_q4b.codes_d);
     g_q4b_launches++;
-    return q4b_launch_ok("tile_permute");
+    return q4b_launch_ok("tile_put");
+}
+bool launch_tile_get(uint8_t *data, uint64_t bytes, cudaStream_t st) {
+    const uint64_t n = bytes / Q4B_TILE_BYTES;
+    if (n == 0) return true;
+    tile_get_k<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(data, n);
+    g_q4b_launches++;
+    return q4b_launch_ok("tile_get");
 }
 
-// Tiled -> wide form, a warp per tile.  Runs behind every upload or conversion of arena bytes; bound by
+// Tiled -> wide form, a warp per tile, for tiles that a copy has brought.  Bound by
 // the bytes it moves (880 read, 1088 written per tile).
 __global__ void __launch_bounds__(256) tile_widen_k(const uint8_t *__restrict__ tiled, uint8_t *__restrict__ wide,
                                                     uint64_t n_tiles, const uint32_t *__restrict__ codes) {
     __shared__ uint32_t tab[512];
-    for (uint32_t i = threadIdx.x; i < 512u; i += blockDim.x) tab[i] = __ldg(codes + i);
-    __syncthreads();
+    load_codes(tab, codes);
     const uint32_t lane = threadIdx.x & 31u;
     for (uint64_t t = (uint64_t)blockIdx.x * 8u + (threadIdx.x >> 5); t < n_tiles; t += (uint64_t)gridDim.x * 8u) {
         const uint8_t *s = tiled + t * Q4B_TILE_BYTES;
         uint8_t *o = wide + t * Q4B_WIDE_BYTES;
-        const uint4 qs = *reinterpret_cast<const uint4 *>(s + Q4B_TILE_OFF_QS + 16u * lane);
-        const uint2 sg = *reinterpret_cast<const uint2 *>(s + Q4B_TILE_OFF_SG + 8u * lane);
-        const uint32_t qh = *reinterpret_cast<const uint16_t *>(s + Q4B_TILE_OFF_QH + 2u * lane);
-        uint32_t n[2][8];   // c' of the lane's two groups, one nibble per byte, in weight order
-#pragma unroll
-        for (uint32_t h = 0; h < 2; h++)
-#pragma unroll
-            for (uint32_t k = 0; k < 8; k++) {
-                const uint32_t w = h ? (k < 4 ? qs.z : qs.w) : (k < 4 ? qs.x : qs.y);
-                const uint32_t idx = ((w >> (8u * (k & 3u))) & 0xffu) | (((qh >> (8u * h + k)) & 1u) << 8);
-                const uint32_t t4 = (h ? sg.y : sg.x) << k;
-                n[h][k] = (tab[idx] ^ q4b_prmt(t4, t4, 0xba98u)) & 0x0f0f0f0fu;   // c or ~c
-            }
-#pragma unroll
-        for (uint32_t t4 = 0; t4 < 4; t4++)
-            *reinterpret_cast<uint2 *>(o + Q4B_WIDE_PART * t4 + 8u * lane) =
-                make_uint2(n[0][2 * t4] | (n[0][2 * t4 + 1] << 4), n[1][2 * t4] | (n[1][2 * t4 + 1] << 4));
+        widen_groups(o, lane, *reinterpret_cast<const uint4 *>(s + Q4B_TILE_OFF_QS + 16u * lane),
+                     *reinterpret_cast<const uint2 *>(s + Q4B_TILE_OFF_SG + 8u * lane),
+                     *reinterpret_cast<const uint16_t *>(s + Q4B_TILE_OFF_QH + 2u * lane), tab);
         if (lane < 8)
-            *reinterpret_cast<uint2 *>(o + Q4B_WIDE_PART * (lane >> 1) + 256u + 8u * (lane & 1u)) =
-                make_uint2(*reinterpret_cast<const uint16_t *>(s + Q4B_TILE_OFF_D + 2u * lane),
-                           *reinterpret_cast<const uint32_t *>(s + Q4B_TILE_OFF_SC + 4u * lane));
+            widen_record(o, lane, *reinterpret_cast<const uint16_t *>(s + Q4B_TILE_OFF_D + 2u * lane),
+                         *reinterpret_cast<const uint32_t *>(s + Q4B_TILE_OFF_SC + 4u * lane));
     }
 }
 
@@ -153,8 +189,7 @@ __global__ void __launch_bounds__(256) tile_widen_k(const uint8_t *__restrict__ 
 bool launch_widen(const Arena &a, uint64_t off, uint64_t bytes, cudaStream_t st) {
     const uint64_t n = bytes / Q4B_TILE_BYTES;
     if (!a.wide || n == 0) return true;
-    const uint64_t nb = (n + 7) / 8;
-    tile_widen_k<<<(unsigned)(nb < 8u * 148u ? nb : 8u * 148u), 256, 0, st>>>(
+    tile_widen_k<<<tile_ctas(n), 256, 0, st>>>(
         a.base + off, a.wide + off / Q4B_TILE_BYTES * Q4B_WIDE_BYTES, n, g_q4b.codes_d);
     g_q4b_launches++;
     return q4b_launch_ok("tile_widen");
@@ -470,10 +505,7 @@ extern "C" bool q4_hip_experts_put_async_a(int arena, uint32_t slot, const uint8
     if (a.tiled && (n % Q4B_TILE_BYTES)) return false;
     Q4B_CHECK(cudaMemcpyAsync(a.base + (uint64_t)slot * a.stride, host, n, cudaMemcpyHostToDevice,
                               g_q4b.copy_stream));
-    if (a.tiled && (!launch_tile_permute(a.base + (uint64_t)slot * a.stride, n, true, g_q4b.copy_stream) ||
-                    !launch_widen(a, (uint64_t)slot * a.stride, n, g_q4b.copy_stream)))
-        return false;
-    return true;
+    return !a.tiled || launch_tile_put(a, (uint64_t)slot * a.stride, n, g_q4b.copy_stream);
 }
 extern "C" bool q4_hip_experts_put_a(int arena, uint32_t slot, const uint8_t *host, uint64_t n) {
     if (!q4_hip_experts_put_async_a(arena, slot, host, n)) return false;
@@ -644,9 +676,7 @@ extern "C" bool q4_cuda_experts_retile_a(int arena, uint32_t first_slot, uint32_
     if (!g_q4b.ok || arena < 0 || arena >= 4) return false;
     Arena &a = g_arena[arena];
     if (!a.base || !a.tiled || (uint64_t)first_slot + n_slots > a.n_slots || n_slots == 0) return false;
-    return launch_tile_permute(a.base + (uint64_t)first_slot * a.stride, (uint64_t)n_slots * a.stride,
-                               true, g_q4b.stream) &&
-           launch_widen(a, (uint64_t)first_slot * a.stride, (uint64_t)n_slots * a.stride, g_q4b.stream);
+    return launch_tile_put(a, (uint64_t)first_slot * a.stride, (uint64_t)n_slots * a.stride, g_q4b.stream);
 }
 extern "C" int q4_cuda_experts_wide_a(int arena) {
     return (arena >= 0 && arena < 4 && g_arena[arena].wide) ? 1 : 0;
@@ -674,7 +704,7 @@ extern "C" bool q4_cuda_experts_get_a(int arena, uint32_t slot, uint8_t *host, u
         return false;
     }
     bool ok = cudaMemcpyAsync(tmp, src, n, cudaMemcpyDeviceToDevice, g_q4b.stream) == cudaSuccess &&
-              launch_tile_permute(tmp, n, false, g_q4b.stream) &&
+              launch_tile_get(tmp, n, g_q4b.stream) &&
               cudaMemcpyAsync(host, tmp, n, cudaMemcpyDeviceToHost, g_q4b.stream) == cudaSuccess &&
               cudaStreamSynchronize(g_q4b.stream) == cudaSuccess;
     cudaFree(tmp);

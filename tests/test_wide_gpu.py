@@ -46,10 +46,10 @@ class _Bytes:
         self.__cuda_array_interface__ = {"shape": (n,), "typestr": "|u1", "data": (ptr, False), "version": 3}
 
 
-@pytest.mark.parametrize("how", ["copy", "h2d", "h2d_async", "fill", "part of a tile", "own copy"])
+@pytest.mark.parametrize("how", ["put", "retile", "copy", "h2d", "h2d_async", "fill", "part of a tile", "own copy"])
 def test_bytes_written_into_a_tiled_arena_reach_both_forms(dev, pkg, how):
-    """Tiled bytes that are copied over a slot (a pack moved or duplicated) replace it for every kernel: the general one
-    reads the tiles, the streaming and the tensor-core product the wide copy."""
+    """Packs that are put into a slot, and tiled bytes that are copied over it (a pack moved or duplicated), replace it for
+    every kernel: the general one reads the tiles, the streaming and the tensor-core product the wide copy."""
     H, F, E, per = 2048, 512, 3, 24
     rng = np.random.default_rng(11)
     layer = pkg.MoeLayer(dev, pkg.synth.expert_packs(rng, E, H, F), None, np.zeros((E, H), np.float32), None, H, F, 1, arena=1)
@@ -70,7 +70,16 @@ def test_bytes_written_into_a_tiled_arena_reach_both_forms(dev, pkg, how):
     try:
         before = products()[0]
         pack = dev.download(src, (n,), np.uint8)
-        if how == "copy":
+        if how in ("put", "retile"):     # the wide copy is written by the kernel that writes the tiles
+            eng, n0 = np.zeros(n, np.uint8), lib.q4_cuda_launch_count()
+            assert lib.q4_cuda_experts_get_a(1, 0, eng.ctypes.data, n) and lib.q4_cuda_launch_count() == n0 + 1
+            if how == "put":
+                assert lib.q4_hip_experts_put_a(1, 2, eng.ctypes.data, n) and lib.q4_cuda_launch_count() == n0 + 2
+            else:
+                assert lib.q4_hip_h2d(dst, eng.ctypes.data, n)     # (widened as if they were tiles: one launch)
+                assert lib.q4_cuda_experts_retile_a(1, 2, 1) and lib.q4_cuda_launch_count() == n0 + 3
+            assert np.array_equal(dev.download(dst, (n,), np.uint8), pack)
+        elif how == "copy":
             assert lib.q4_hip_copy_async(dst, src, n // 4)
         elif how == "h2d":
             assert lib.q4_hip_h2d(dst, pack.ctypes.data, n)
