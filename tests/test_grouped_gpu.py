@@ -253,10 +253,14 @@ def test_verify_window_matches_single_token_path(dev, pkg, oracle):
         layer.close()
 
 
-@pytest.mark.parametrize("n_tok,n_expert,topk,tiled", [(4, 64, 10, True), (4, 64, 10, False),
-                                                         (1, 32, 4, True), (33, 48, 6, True)])
-def test_layer_n_matches_oracle_per_token(dev, pkg, oracle, n_tok, n_expert, topk, tiled):
+@pytest.mark.parametrize("n_tok,n_expert,topk,tiled,wide", [(4, 64, 10, True, 1), (4, 64, 10, False, 1),
+                                                              (1, 32, 4, True, 1), (33, 48, 6, True, 1),
+                                                              (4, 64, 10, True, 0), (33, 48, 6, True, 0)])
+def test_layer_n_matches_oracle_per_token(dev, pkg, oracle, monkeypatch, n_tok, n_expert, topk, tiled, wide):
+    """wide = 0: an arena without the wide copy of its tiles, whose products decode the tiles (grouped_few_k, mmq_tc_k
+    and, in the default mode with 33 tokens, both side by side)."""
     H, F = 2048, 512
+    monkeypatch.setenv("Q4B_WIDE", str(wide))
     L = pkg.synth.layer(40 + n_tok, n_expert, H, F)
     xs = pkg.synth.hidden(41, n_tok, H)
     lib = dev.lib
@@ -265,6 +269,7 @@ def test_layer_n_matches_oracle_per_token(dev, pkg, oracle, n_tok, n_expert, top
         layer = pkg.MoeLayer(dev, L["experts"], L["shared"], L["router"], L["norm_w"], H, F, topk, arena=1)
     finally:
         lib.q4_cuda_set_tiled_default(1)
+    assert lib.q4_cuda_experts_wide_a(1) == (1 if tiled and wide else 0)
     # the CUDA-core kernels first: with them a token's result does not depend on the batch
     assert lib.q4_cuda_mmq_tc_mode(0)
     try:
@@ -327,14 +332,16 @@ def test_layer_n_matches_oracle_per_token(dev, pkg, oracle, n_tok, n_expert, top
         layer.close()
 
 
+@pytest.mark.parametrize("wide", [1, 0])
 @pytest.mark.parametrize("per", [[0, 0, 0, 0], [2100, 11, 12, 5], [64, 0, 65, 1], [3, 0, 0, 129]])
-def test_grouped_product_edge_row_counts(dev, pkg, oracle, per):
+def test_grouped_product_edge_row_counts(dev, pkg, oracle, monkeypatch, per, wide):
     """Row counts at the edges of the kernels' ranges, on a tiled arena: no rows at all (nothing may
-    be written), 11 / 12 rows either side of the tensor-core threshold next to an expert with
-    2100 rows (one call, two kernels), 64 / 65 (one pass / two passes), 129 (three passes, the last
-    with one row).
+    be written); an expert with 2100 rows next to small ones; 64 / 65 rows, 128 / 129.  With the wide copy one kernel
+    takes a call (passes of up to 128 rows on the tensor cores, blocks of 16 streamed).  Without it (wide = 0) a
+    call is split by entry at 12 rows (one call, two kernels), and passes are of 64 rows.
     Every kernel choice must agree with the CPU path's int8 dot."""
     H, F, n_exp = 2048, 512, 4
+    monkeypatch.setenv("Q4B_WIDE", str(wide))
     rng = np.random.default_rng(7 + sum(per))
     packs = pkg.synth.expert_packs(rng, n_exp, H, F)
     layer = pkg.MoeLayer(dev, packs, None, np.zeros((n_exp, H), np.float32), None, H, F, 1, arena=1)

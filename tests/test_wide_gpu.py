@@ -1,6 +1,8 @@
-"""The streaming grouped product on the wide copy of an arena (csrc/q4b_wide.cu) against the general
-CUDA-core kernel, which decodes the tiles themselves: row counts at the edges of its inner forms (1 or 2
-rows, fragments of 8, blocks of 16), widths with 1, 2, 4, 8 super-blocks a row (bit for bit) and others."""
+"""The streaming grouped product on the wide copy of an arena (csrc/q4b_wide.cu), and the one that decodes the tiles where
+an arena has no such copy (csrc/q4b_few.cu), against the general CUDA-core kernel: row counts at the edges of their inner
+forms (1 or 2 rows, fragments of 8, blocks of 16; 1 to 3 rows in registers), widths with 1, 2, 4, 8 super-blocks a row (bit
+for bit) and others.  Then what keeps the wide copy and the tiles the same, and the tensor-core product on it
+(csrc/q4b_wide_tc.cu) beyond the items that a block takes in at a time."""
 import numpy as np
 import pytest
 
@@ -8,14 +10,17 @@ pytestmark = pytest.mark.gpu
 IQ3_S = 21
 
 
+@pytest.mark.parametrize("wide", [1, 0])
 @pytest.mark.parametrize("H,F", [(2048, 512), (1024, 256), (2560, 768), (512, 256)])
 @pytest.mark.parametrize("per", [[1, 2, 3, 0, 8, 9], [16, 17, 33, 1, 0, 70], [1, 1, 1, 1, 1, 1], [0, 0, 5, 0, 0, 0]])
-def test_wide_product_equals_the_general_kernel(dev, pkg, H, F, per):
+def test_wide_product_equals_the_general_kernel(dev, pkg, monkeypatch, H, F, per, wide):
+    monkeypatch.setenv("Q4B_WIDE", str(wide))
     rng = np.random.default_rng(H + F + sum(per))
     E, rows = len(per), sum(per)
     packs = pkg.synth.expert_packs(rng, E, H, F)
     layer = pkg.MoeLayer(dev, packs, None, np.zeros((E, H), np.float32), None, H, F, 1, arena=1)
     lib = dev.lib
+    assert lib.q4_cuda_experts_wide_a(1) == wide
     bounds = dev.upload(np.concatenate([[0], np.cumsum(per)]).astype(np.int32))
     try:
         for w_rows, w_cols, off in ((2 * F, H, layer.og), (H, F, layer.od)):
@@ -105,3 +110,40 @@ def test_bytes_written_into_a_tiled_arena_reach_both_forms(dev, pkg, how):
     finally:
         lib.q4_cuda_mmq_tc_mode(-1)
         layer.close()
+
+
+@pytest.mark.parametrize("cols,tiles", [(256, 41), (512, 19)])
+def test_tensor_core_product_with_several_batches_of_items(dev, pkg, cols, tiles):
+    """A block of the tensor-core product takes in the descriptors of 128 work items at a time: calls with 283 and 132 of
+    them a block, of 18 to 22 rows, whose pipeline runs on from one batch into the next.  The experts' matrices overlap (an
+    expert starts one tile after the one before)."""
+    import torch
+    lib, n_exp, w_rows = dev.lib, 1023, 128 * tiles
+    per = 20 + (np.arange(n_exp) * 7 % 5 - 2)
+    per[-1] += 20 * n_exp - per.sum()
+    rows, rb = int(per.sum()), cols // 256 * 110
+    assert n_exp * tiles > 128 * 148
+    rng = np.random.default_rng(cols)
+    pack = pkg.synth.iq3s_blocks(rng, (w_rows * rb + (n_exp - 1) * 880) // 110).reshape(-1)
+    lib.q4_cuda_set_tiled_default(2)
+    try:
+        assert lib.q4_hip_experts_alloc_a(1, 1, pack.nbytes)
+    finally:
+        lib.q4_cuda_set_tiled_default(1)
+    try:
+        assert lib.q4_hip_experts_put_a(1, 0, pack.ctypes.data, pack.nbytes) and lib.q4_cuda_experts_wide_a(1) == 1
+        x, d_xq = rng.standard_normal((rows, cols)).astype(np.float32), dev.malloc(lib.q4_mmq_q8_bytes(rows, cols))
+        bounds, out = dev.upload(np.concatenate([[0], np.cumsum(per)]).astype(np.int32)), []
+        for mode in (-1, 2):
+            y = torch.full((rows, w_rows), 7.5, device="cuda")
+            torch.cuda.synchronize()
+            assert lib.q4_cuda_mmq_tc_mode(mode) and lib.q4_mmq_quantize(dev.upload(x), None, d_xq, IQ3_S, cols, rows)
+            assert lib.q4_mmq_mul_id(lib.q4_hip_experts_base_a(1), IQ3_S, w_rows, cols, 880, n_exp, d_xq, bounds, 40, rows,
+                                     y.data_ptr(), w_rows)
+            assert lib.q4_cuda_device_error() == 0
+            out.append(y.view(rows, tiles, 128))
+        off, ref = (out[0] - out[1]).norm(dim=2), out[1].norm(dim=2)
+        assert (ref > 0).all() and (off <= 1e-5 * ref).all(), float((off / ref).max())
+    finally:
+        lib.q4_cuda_mmq_tc_mode(-1)
+        lib.q4_hip_experts_free_a(1)
