@@ -928,10 +928,11 @@ __global__ void __launch_bounds__(256) grouped_rows4_k(const uint8_t *__restrict
 // enough rows to fill a useful part of a 128 x 64 MMA tile; below that the streaming
 // CUDA-core kernel (one decode, a handful of dot products from registers) is the
 // better fit, and the general CUDA-core kernel takes what neither accepts (arenas in
-// the engine's byte order, odd widths).  In the default mode a call is split by
+// the engine's byte order, odd widths).  In the default mode one kernel takes a whole call on an arena
+// with a wide copy, by its average rows (WIDE_TC_ROWS).  Without one a call is split by
 // entry: entries with TC_MIN_ROWS rows or more go to the tensor cores, the rest to
 // the streaming kernel; each kernel skips the other's entries.
-int g_tc_mode = -1;  // -1 split by rows, 0 CUDA cores only, 1 tensor cores whenever the shape
+int g_tc_mode = -1;  // -1 by rows, 0 CUDA cores only, 1 tensor cores whenever the shape
                      // allows, 2 the general CUDA-core kernel only
 // The streaming kernels' view of a call.
 wide::Args stream_args(const uint8_t *w, uint64_t expert_stride, const int32_t *act, const uint32_t *n_act, uint32_t n_entries,
@@ -1001,6 +1002,10 @@ bool launch_grouped(const uint8_t *w, uint64_t expert_stride, const int32_t *act
 constexpr uint32_t TC_MIN_ROWS = 12;
 // 370 experts, gate/up + down, us: 16 rows 161 + 87 streamed, 17 rows 262 + 138, 20 rows 293 + 154 (two passes over the
 // weights), 32 rows 299 + 156; on the tensor cores 266 + 157, 264 + 160, 269 + 162, 283 + 165, and 338 + 190 with 64 rows.
+// The line is by the average, which is all the host knows of a layer's rows; a caller's max_rows_hint bounds the largest
+// entry only and is not looked at.  Uneven entries below the line, streamed / on the tensor cores, us: one expert of 512 /
+// 2048 / 8000 rows beside 511 of 2 (gate/up) 124 / 332, 165 / 350, 318 / 414; a layer of 512 experts whose picks follow
+// Zipf(1.1), 64 tokens 100 / 122, 260: 228 / 228, 550: 355 / 284, 920: 528 / 364 (fewer experts are live than could be).
 constexpr uint32_t WIDE_TC_ROWS = 20;
 // Does the tensor-core product on the wide form take a call of IQ3_S weights?
 bool takes_wide_tc(const uint8_t *w, uint64_t expert_stride, uint32_t n_entries, uint64_t total_rows, uint32_t cols, uint32_t w_rows) {

@@ -233,6 +233,8 @@ template <> struct Fmt<20u> {
 // reads of shared memory take longer than the instructions: 24 wavefronts a trip of 4 activation rows).
 // A trip's weights are loaded while the sums of the one before run.
 // Calls in a graph, 4 rows, 4096 x 2048 of Q4_K: 8.4 us for two launches, 6.1 now; 64 x 2048: 8.4 and 4.9.
+// Large matrices are bound by issue: 151,936 x 2048 of Q4_K, 2 / 4 / 8 rows 72 / 94 / 127 us (94, 112, 191 with two launches and
+// a warp a row; 27 of bytes), of Q6_K 115 / 144 / 214 (117, 152, 227; 39 of bytes); 4 rows of Q4_K: issue slots 74 % busy.
 // 512 threads and two rows a warp; 1024 threads and one row where more warps have to cover the loads and the reads of the
 // activations are few: 1 or 2 activation rows (4096 x 2048 of Q5_K, 2 rows: 5.5 us a call against 6.2), types of 2-byte
 // alignment, which their narrow loads bound (IQ4_NL, 4 rows: 6.9 against 8.0).  4 rows of Q4_K: 6.1 with 512, 6.5 with 1024.

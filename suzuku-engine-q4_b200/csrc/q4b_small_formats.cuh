@@ -221,7 +221,7 @@ __global__ void moe_ya20_k(const uint8_t *__restrict__ bd, uint64_t stride, cons
                            uint32_t n_embd, float *__restrict__ y) {
     q4b_pdl_wait();
     const uint32_t row = blockIdx.x * 2u + (threadIdx.x >> 7), lane = threadIdx.x & 127u;
-    const uint32_t r = min(row, n_embd - 1u);   // an odd last CTA: its second half is computed and dropped   // (n_embd is even)
+    const uint32_t r = min(row, n_embd - 1u);   // an odd last CTA: its second half is computed and dropped
     const uint32_t n = exec_count(n_dev, n_host);
     const uint32_t ng = n_ff >> 5;
     const uint64_t rb = small_row_bytes(Q4_T_Q2_0, n_ff);

@@ -20,8 +20,9 @@
 // additions of grouped_rows_k (pairs of groups, blocks of four pairs, blocks pairwise), so for 1, 2, 4 or 8
 // super-blocks a row the result is that kernel's, bit for bit.
 //
-// What bounds it: HBM, 1088 bytes a tile.  The tiled form costs 247 warp instructions a tile and 1.7
-// rows, more than the 190 issue slots that pass while its 880 bytes arrive; here it is about 90.
+// What bounds it: with 1 or 2 rows an entry start-up and HBM (1088 bytes a tile: 90 us for 370 experts' gate/up against 64
+// of bytes), from 3 rows on instruction issue.  64 tokens of 11 picks (369 experts, 1.9 rows): 137 warp instructions a
+// tile, issue slots 63 % busy, DRAM at 59 % of its peak, 88.6 us under the profiler.  The tiled form took 247 with 1.7 rows.
 #include "q4b_tile.cuh"
 
 #include <type_traits>

@@ -1,7 +1,7 @@
 // The tensor-core grouped product on the wide form of an arena (q4b_tile.cuh): the arithmetic of mmq_tc_k
 // (q4b_mmq_tc.cu: fp16 operands that carry the scales, two planes of the activations, fp32 accumulators in
-// tensor memory, one multiply by the super-block's d on the CUDA cores), for the calls in which an expert has
-// about ten rows or more.  mmq_tc_k stays for arenas without a wide copy and for engine byte order.
+// tensor memory, one multiply by the super-block's d on the CUDA cores), for the calls in which there are
+// 20 rows or more per possible entry (WIDE_TC_ROWS in q4b_grouped.cu, with both sides' times).  mmq_tc_k stays for arenas without a wide copy and for engine byte order.
 //
 // What bounded mmq_tc_k was neither its MMAs nor its decode but latency: with two steps of weight fields in
 // registers ahead, a step of 128 x 128 weights took 3200 cycles when they came from HBM (512 experts of 17
