@@ -478,8 +478,8 @@ bool q4_cuda_moe_exec_noalloc(const uint8_t *base, uint64_t stride, const int32_
  * free after taking it (1.24 times the arena; Q4B_WIDE=0 in the environment turns it off, and the products
  * then decode the tiles).  It is freed with the arena.  Everything in this library that writes an arena's
  * bytes brings it up to date on the same stream: q4_hip_experts_put*_a, retile_a, and q4_hip_h2d,
- * q4_hip_h2d_async, q4_hip_copy_async and q4_hip_fill where their destination lies in the arena (tiled bytes,
- * for instance a pack moved from slot to slot).  A program that writes tiled bytes with kernels or copies of
+ * q4_hip_h2d_async, q4_hip_copy_async, q4_hip_fill, q4_hip_copy_memset and q4_mmq_gather (into lent buffers)
+ * where their destination lies in the arena (tiled bytes, for instance a pack moved from slot to slot).  A program that writes tiled bytes with kernels or copies of
  * its own calls refresh_a behind them.
  *
  * Resident storage format of an arena.  By default q4_hip_experts_put*_a rewrites

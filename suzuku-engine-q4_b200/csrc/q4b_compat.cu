@@ -72,7 +72,7 @@ extern "C" bool q4_hip_copy_memset(void *dst, int v, size_t n) {
     if (!g_q4b.ok || !dst) return false;
     if (!n) return true;
     Q4B_CHECK(cudaMemsetAsync(dst, v, n, g_q4b.copy_stream));
-    return true;
+    return q4b_arena_written(dst, n, g_q4b.copy_stream);
 }
 extern "C" bool q4_hip_moe_act(float *d_g, const float *d_u, uint64_t n) { return q4_hip_silu_mul(d_g, d_u, n); }
 extern "C" void q4_hip_mark_pt(int slot) { (void)slot; }   // step-profile boundary marks: not kept

@@ -534,5 +534,8 @@ extern "C" bool q4_mmq_gather(const uint8_t *abase, uint64_t astride, uint64_t g
     elem::gather16_k<<<dim3((unsigned)bx, n), 256, 0, g_q4b.stream>>>(abase, astride, goff, gu_bytes, doff, d_bytes,
                                                                      gu_dst, d_dst, d_eid, d_slot, d_gu, d_d);
     g_q4b_launches++;
-    return q4b_launch_ok("mmq_gather");
+    // (lent buffers may be part of an arena)
+    return q4b_launch_ok("mmq_gather") &&
+           (!elem::g_wbuf_lent || ((d_gu != elem::g_wbuf_gu || q4b_arena_written(d_gu, elem::g_wbuf_gu_bytes, g_q4b.stream)) &&
+                                   (d_d != elem::g_wbuf_d || q4b_arena_written(d_d, elem::g_wbuf_d_bytes, g_q4b.stream))));
 }

@@ -53,6 +53,9 @@ struct Q4bState {
 };
 extern Q4bState g_q4b;
 
+// q4b_runtime.cu: [p, p + bytes) has been written on st; brings the wide copy of arena tiles in that range up to date.
+bool q4b_arena_written(const void *p, uint64_t bytes, cudaStream_t st);
+
 #define Q4B_XQ_SLICES 80u     // >= 64 experts per exec + shared + tokens of a window
 #define Q4B_XQ_MAXLEN 16384u  // widest activation row the decode path quantises
 #define Q4B_MAX_TOK 8u        // tokens per fused decode / verify call

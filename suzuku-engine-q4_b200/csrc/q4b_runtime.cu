@@ -436,6 +436,7 @@ extern "C" bool q4_hip_copy_async(float *d, const float *s, uint64_t n) {
     Q4B_CHECK(cudaMemcpyAsync(d, s, n * sizeof(float), cudaMemcpyDeviceToDevice, g_q4b.stream));
     return widen_written(d, n * sizeof(float), g_q4b.stream);
 }
+bool q4b_arena_written(const void *p, uint64_t bytes, cudaStream_t st) { return widen_written(p, bytes, st); }
 extern "C" uint64_t q4_hip_vram_free(void) {
     if (!g_q4b.ok) return 0;
     size_t f = 0, t = 0;

@@ -3,9 +3,12 @@ an arena has no such copy (csrc/q4b_few.cu), against the general CUDA-core kerne
 forms (1 or 2 rows, fragments of 8, blocks of 16; 1 to 3 rows in registers), widths with 1, 2, 4, 8 super-blocks a row (bit
 for bit) and others.  Then what keeps the wide copy and the tiles the same, and the tensor-core product on it
 (csrc/q4b_wide_tc.cu) beyond the items that a block takes in at a time."""
+import os
+
 import numpy as np
 import pytest
 
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 pytestmark = pytest.mark.gpu
 IQ3_S = 21
 
@@ -51,7 +54,7 @@ class _Bytes:
         self.__cuda_array_interface__ = {"shape": (n,), "typestr": "|u1", "data": (ptr, False), "version": 3}
 
 
-@pytest.mark.parametrize("how", ["put", "retile", "copy", "h2d", "h2d_async", "fill", "part of a tile", "own copy"])
+@pytest.mark.parametrize("how", ["put", "retile", "copy", "h2d", "h2d_async", "fill", "memset", "part of a tile", "own copy"])
 def test_bytes_written_into_a_tiled_arena_reach_both_forms(dev, pkg, how):
     """Packs that are put into a slot, and tiled bytes that are copied over it (a pack moved or duplicated), replace it for
     every kernel: the general one reads the tiles, the streaming and the tensor-core product the wide copy."""
@@ -92,6 +95,9 @@ def test_bytes_written_into_a_tiled_arena_reach_both_forms(dev, pkg, how):
             assert lib.q4_hip_h2d_async(dst, pack.ctypes.data, n)
         elif how == "fill":
             assert lib.q4_hip_fill(dst, 0.0, n // 4)
+        elif how == "memset":            # on the upload stream
+            assert lib.q4_hip_copy_memset(dst, 0, n)
+            lib.q4_hip_copy_wait()
         elif how == "part of a tile":    # the tail of one tile, the next one, the head of a third; up to the arena's end too
             assert lib.q4_hip_copy_async(dst + 440, src + 440, (880 + 660) // 4)
             assert lib.q4_hip_copy_async(dst + n - 8, src + n - 8, 2)
@@ -110,6 +116,52 @@ def test_bytes_written_into_a_tiled_arena_reach_both_forms(dev, pkg, how):
     finally:
         lib.q4_cuda_mmq_tc_mode(-1)
         layer.close()
+
+
+def test_gather_into_buffers_lent_from_an_arena(dev, pkg):
+    """The expert-indexed buffers may be memory that the caller lends, slots of the arena among it: the products read there
+    what was gathered.  In a child process: lending cannot be taken back."""
+    import subprocess
+    import sys
+    code = """
+import ctypes as C, sys
+import numpy as np
+sys.path.insert(0, %r)
+import __graft_entry__ as entry
+pkg = entry.load_package()
+dev = pkg.Device()
+lib, (H, F, E, per, ty) = dev.lib, (2048, 512, 3, 5, 21)
+rng = np.random.default_rng(2)
+layer = pkg.MoeLayer(dev, pkg.synth.expert_packs(rng, 2 * E + 2, H, F), None, np.zeros((2 * E + 2, H), np.float32), None, H, F, 1)
+gu, d = layer.od, layer.pack - layer.od
+slot = lambda i: layer.base + i * layer.stride
+assert lib.q4_cuda_experts_wide_a(0) == 1
+assert lib.q4_mmq_wbuf_lend(slot(E), E * gu, slot(2 * E), E * d)      # the slots from E on are lent
+p, q = C.c_void_p(), C.c_void_p()
+assert lib.q4_mmq_wbuf(gu, d, E, C.byref(p), C.byref(q))
+order = np.array([2, 0, 1], np.int32)
+assert lib.q4_mmq_gather(layer.base, layer.stride, 0, gu, layer.od, d, gu, d, dev.upload(np.arange(E, dtype=np.int32)),
+                         dev.upload(order), E, p, q)
+bounds = dev.upload((np.arange(E + 1) * per).astype(np.int32))
+for w, want, rows, cols, stride in ((p, 0, 2 * F, H, gu), (q, layer.od, H, F, d)):
+    x, xq = rng.standard_normal((E * per, cols)).astype(np.float32), dev.malloc(lib.q4_mmq_q8_bytes(E * per, cols))
+    assert lib.q4_mmq_quantize(dev.upload(x), None, xq, ty, cols, E * per)
+    out = dev.malloc(E * per * rows * 4)
+    assert lib.q4_cuda_mmq_tc_mode(2)
+    ref = np.zeros((E * per, rows), np.float32)
+    for e in range(E):
+        one = dev.upload(np.array([e * per, (e + 1) * per], np.int32))
+        assert lib.q4_mmq_mul_id(slot(int(order[e])) + want, ty, rows, cols, 0, 1, xq, one, per, E * per, out, rows)
+    ref = dev.download(out, (E * per, rows), np.float32)
+    for mode in (0, 2):
+        assert lib.q4_cuda_mmq_tc_mode(mode)
+        assert lib.q4_mmq_mul_id(w, ty, rows, cols, stride, E, xq, bounds, per, E * per, out, rows)
+        assert np.array_equal(dev.download(out, (E * per, rows), np.float32), ref), (mode, rows)
+assert lib.q4_cuda_device_error() == 0
+print("lent ok")
+""" % ROOT
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=ROOT)
+    assert r.returncode == 0 and "lent ok" in r.stdout, r.stdout + r.stderr
 
 
 @pytest.mark.parametrize("cols,tiles", [(256, 41), (512, 19)])
