@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(256) swiglu_planes_k(const float *gu, uint64_t
     if (live) {
         const float4 *pg = reinterpret_cast<const float4 *>(gu + r * 2 * n_ff + c);
         const float4 *pu = reinterpret_cast<const float4 *>(gu + r * 2 * n_ff + n_ff + c);
-        const float4 g0 = pg[0], g1 = pg[1], u0 = pu[0], u1 = pu[1];
+        const float4 g0 = q4b_ld_cs(pg), g1 = q4b_ld_cs(pg + 1), u0 = q4b_ld_cs(pu), u1 = q4b_ld_cs(pu + 1);
         v[0] = q4b_swiglu(g0.x, u0.x), v[1] = q4b_swiglu(g0.y, u0.y);
         v[2] = q4b_swiglu(g0.z, u0.z), v[3] = q4b_swiglu(g0.w, u0.w);
         v[4] = q4b_swiglu(g1.x, u1.x), v[5] = q4b_swiglu(g1.y, u1.y);

@@ -109,10 +109,15 @@ __device__ __forceinline__ void q4b_pdl_wait() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-// A load past L1: like the wait volatile, so that it stays behind it.
+// Loads past L1, and of data that is read once: like the wait volatile, so that they stay behind it.
 __device__ __forceinline__ float q4b_ld_cg(const float *p) {
     float v;
     asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 q4b_ld_cs(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
     return v;
 }
 __device__ __forceinline__ void q4b_l2_prefetch(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
