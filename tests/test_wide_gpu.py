@@ -199,3 +199,39 @@ def test_tensor_core_product_with_several_batches_of_items(dev, pkg, cols, tiles
     finally:
         lib.q4_cuda_mmq_tc_mode(-1)
         lib.q4_hip_experts_free_a(1)
+
+
+@pytest.mark.parametrize("H,F", [(2048, 512), (1024, 256), (2560, 768), (256, 256), (1280, 256)])
+@pytest.mark.parametrize("per", [[1, 31, 32, 33, 0, 63], [64, 65, 128, 2, 129, 0], [0, 16, 0, 0, 0, 0], [200, 1, 1, 95, 96, 97]])
+def test_tensor_core_product_at_the_edges_of_its_passes(dev, pkg, H, F, per):
+    """Rows at the edges of the MMA's N (32) and of a pass (64), rows of 1 to 10 super-blocks.  (An odd
+    number of 128-row tiles: the test above.)
+    Against the general kernel: activations carry 22 bits there (2^-23 of the row's largest group a term, of random
+    sign) and the tensor core truncates eight additions of 24 bits per 128 k: a few 1e-7 of the result; bound 1e-5."""
+    rng = np.random.default_rng(H + F + sum(per))
+    E, rows = len(per), sum(per)
+    packs = pkg.synth.expert_packs(rng, E, H, F)
+    layer = pkg.MoeLayer(dev, packs, None, np.zeros((E, H), np.float32), None, H, F, 1, arena=1)
+    lib = dev.lib
+    assert lib.q4_cuda_experts_wide_a(1) == 1
+    bounds = dev.upload(np.concatenate([[0], np.cumsum(per)]).astype(np.int32))
+    try:
+        for w_rows, w_cols, off in ((2 * F, H, layer.og), (H, F, layer.od)):
+            d_xq, d_dst = dev.malloc(lib.q4_mmq_q8_bytes(rows, w_cols)), dev.malloc(rows * (w_rows + 3) * 4)
+            x = rng.standard_normal((rows, w_cols)).astype(np.float32)
+            assert lib.q4_mmq_quantize(dev.upload(x), None, d_xq, IQ3_S, w_cols, rows)
+            got = {}
+            for mode in (1, 2):
+                dev.write(d_dst, np.full((rows, w_rows + 3), 7.5, np.float32))
+                assert lib.q4_cuda_mmq_tc_mode(mode)
+                assert lib.q4_mmq_mul_id(layer.base + off, IQ3_S, w_rows, w_cols, layer.stride, E, d_xq, bounds,
+                                         max(per), rows, d_dst, w_rows + 3)
+                got[mode] = dev.download(d_dst, (rows, w_rows + 3), np.float32)
+            if w_cols // 256 in (1, 2, 4, 8):     # (else the call clears the rows whole)
+                assert (got[1][:, w_rows:] == 7.5).all()
+            diff, ref = np.linalg.norm(got[1] - got[2], axis=1), np.linalg.norm(got[2], axis=1)
+            assert (diff <= 1e-5 * ref).all(), float((diff / ref).max())
+        assert lib.q4_cuda_device_error() == 0
+    finally:
+        lib.q4_cuda_mmq_tc_mode(-1)
+        layer.close()
