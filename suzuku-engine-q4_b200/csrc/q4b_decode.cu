@@ -420,10 +420,11 @@ __global__ void __launch_bounds__(128) softmax_topk_k(const float *logits, uint3
 // RMSNorm, router product and softmax / top-k of a batch of tokens in ONE launch (n_embd == 2048): what
 // rms_q8_k (norm only), gemv_f32_x16_k and softmax_topk_k do as three, with the same products and sums
 // in the same order (the sum of squares is formed in double in another order, which does not change
-// its float value).  grid (router rows / 8, tokens / 8): a CTA normalises its group's eight rows (a
-// warp per row, all loads in flight at once) into shared memory, then a warp takes one router row
+// its float value).  grid (router rows / 8 R, tokens / 8): a CTA normalises its group's eight rows (a
+// warp per row, all loads in flight at once) into shared memory, then a warp takes R router rows
 // through the eight tokens; the CTA that finishes a group last (a counter per group, no waiting) runs
 // the group's top-k, one warp per token.
+template <uint32_t R>
 __global__ void __launch_bounds__(256) route_small_k(const float *x, const float *__restrict__ norm_w,
                                                      float eps, const float *__restrict__ W, uint32_t n_expert,
                                                      uint32_t n_tok, uint32_t topk, float *__restrict__ xn_out,
@@ -434,8 +435,8 @@ __global__ void __launch_bounds__(256) route_small_k(const float *x, const float
     constexpr uint32_t n = 2048;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t t0 = blockIdx.y * 8u, nt = min(8u, n_tok - t0);
-    if (blockIdx.x * 8u + warp < n_expert)   // this warp's router row, into L2 before the wait
-        for (uint32_t i = lane * 32u; i < n; i += 1024u) q4b_l2_prefetch(W + (uint64_t)(blockIdx.x * 8u + warp) * n + i);
+    const uint32_t r0 = (blockIdx.x * 8u + warp) * R, nr = r0 < n_expert ? min(R, n_expert - r0) : 0u;
+    for (uint32_t i = lane * 32u; i < nr * n; i += 1024u) q4b_l2_prefetch(W + (uint64_t)r0 * n + i);   // this warp's router rows, before the wait
     q4b_pdl_wait();
     if (warp < nt) {
         const float4 *x4 = reinterpret_cast<const float4 *>(x + (uint64_t)(t0 + warp) * n);
@@ -467,9 +468,8 @@ __global__ void __launch_bounds__(256) route_small_k(const float *x, const float
         }
     }
     __syncthreads();
-    const uint32_t r = blockIdx.x * 8u + warp;
-    if (r < n_expert) {
-        const float4 *w4 = reinterpret_cast<const float4 *>(W + (uint64_t)r * n);
+    if (R == 1u && nr) {
+        const float4 *w4 = reinterpret_cast<const float4 *>(W + (uint64_t)r0 * n);
         float4 w[16];
 #pragma unroll
         for (int j = 0; j < 16; j++) w[j] = __ldg(w4 + lane + 32 * j);
@@ -482,8 +482,49 @@ __global__ void __launch_bounds__(256) route_small_k(const float *x, const float
                 acc += w[j].x * b.x + w[j].y * b.y + w[j].z * b.z + w[j].w * b.w;
             }
             acc = q4b_warp_sum(acc);
-            if (lane == 0) logits[(uint64_t)(t0 + t) * n_expert + r] = 1.0f * acc;
+            if (lane == 0) logits[(uint64_t)(t0 + t) * n_expert + r0] = 1.0f * acc;
         }
+    } else if (nr) {
+        constexpr uint32_t JC = 8u / R;      // float4 of a row that are loaded while as many are used
+        const float4 *w4[R];
+        float4 w[2][R][JC];
+        float acc[R][8];
+#pragma unroll
+        for (uint32_t r = 0; r < R; r++) {
+            w4[r] = reinterpret_cast<const float4 *>(W + (uint64_t)(r0 + min(r, nr - 1u)) * n) + lane;
+#pragma unroll
+            for (uint32_t t = 0; t < 8; t++) acc[r][t] = 0.f;
+#pragma unroll
+            for (uint32_t j = 0; j < JC; j++) w[0][r][j] = __ldg(w4[r] + 32u * j);
+        }
+        const float4 *x4 = reinterpret_cast<const float4 *>(rs_rows) + lane;
+#pragma unroll 2
+        for (uint32_t c = 0; c < 16u / JC; c++) {
+            if (c + 1u < 16u / JC) {
+#pragma unroll
+                for (uint32_t r = 0; r < R; r++)
+#pragma unroll
+                    for (uint32_t j = 0; j < JC; j++) w[(c + 1u) & 1u][r][j] = __ldg(w4[r] + 32u * ((c + 1u) * JC + j));
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < JC; j++)
+#pragma unroll
+                for (uint32_t t = 0; t < 8; t++) {      // (of a short group also the rows that nobody wrote; not stored)
+                    const float4 b = x4[t * (n / 4u) + 32u * (c * JC + j)];
+#pragma unroll
+                    for (uint32_t r = 0; r < R; r++) {
+                        const float4 a = w[c & 1u][r][j];
+                        acc[r][t] += a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
+                    }
+                }
+        }
+#pragma unroll
+        for (uint32_t t = 0; t < 8; t++)
+#pragma unroll
+            for (uint32_t r = 0; r < R; r++) {
+                const float v = q4b_warp_sum(acc[r][t]);
+                if (lane == 0 && r < nr && t < nt) logits[(uint64_t)(t0 + t) * n_expert + r0 + r] = 1.0f * v;
+            }
     }
     __threadfence();
     __syncthreads();
@@ -1364,7 +1405,9 @@ bool q4b_route_small_warm() {
     if (g_route_counter) return true;
     if (cudaMalloc(&g_route_counter, (ROUTE_MAX_TOK / 8u) * sizeof(unsigned int)) != cudaSuccess ||
         cudaMemset(g_route_counter, 0, (ROUTE_MAX_TOK / 8u) * sizeof(unsigned int)) != cudaSuccess ||
-        cudaFuncSetAttribute(route_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 2048 * 4) != cudaSuccess) {
+        cudaFuncSetAttribute(route_small_k<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 2048 * 4) != cudaSuccess ||
+        cudaFuncSetAttribute(route_small_k<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 2048 * 4) != cudaSuccess ||
+        cudaFuncSetAttribute(route_small_k<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 2048 * 4) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -1380,7 +1423,15 @@ bool q4b_route_small(const float *x, const float *norm_w, float eps, const float
     if (!g_route_counter || n_embd != 2048u || n_tok == 0 || n_tok > ROUTE_MAX_TOK || n_expert > 1024u ||
         topk > 64u || (((uintptr_t)router | (uintptr_t)x | (uintptr_t)norm_w | (uintptr_t)xn) & 15u))
         return false;
-    q4b_launch(route_small_k, dim3((n_expert + 7u) / 8u, (n_tok + 7u) / 8u), 256, 8u * 2048u * 4u, g_q4b.stream,
+    // Router rows a warp: one while that leaves about two CTAs an SM (each normalises eight tokens, and reads them from shared
+    // memory for every row), else two or four, which are read the tokens for at once.  512 experts, us a call: one row 33 tokens
+    // 15.8 (two rows, an earlier form: 19.9), 64 tokens 25.3, 128 43.5, 256 74.5; two rows 64 tokens 17.6; four 128 tokens
+    // 24.9, 256 44.2.  160 experts, 256 tokens: one row 34.1, four 23.4.
+    const uint32_t groups = (n_tok + 7u) / 8u, sm = (uint32_t)g_q4b.n_sm;
+    auto ctas = [&](uint32_t per) { return groups * ((n_expert + 8u * per - 1u) / (8u * per)); };
+    const uint32_t per = 4u * ctas(1) <= 9u * sm ? 1u : ctas(2) <= 2u * sm ? 2u : 4u;
+    q4b_launch(per == 1u ? route_small_k<1> : per == 2u ? route_small_k<2> : route_small_k<4>, dim3(ctas(per) / groups, groups), 256,
+        8u * 2048u * 4u, g_q4b.stream,
         x, norm_w, eps, router, n_expert, n_tok, topk, xn, logits, ids, wts, g_route_counter);
     g_q4b_launches++;
     return q4b_launch_ok("route_small");
