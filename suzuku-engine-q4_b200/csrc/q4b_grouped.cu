@@ -1000,12 +1000,14 @@ bool launch_grouped(const uint8_t *w, uint64_t expert_stride, const int32_t *act
 // an 8-way expert-parallel rank (8 own tokens, weights cold) moves to the tensor cores with its
 // four helper launches per layer: 9.3 ms per step against 7.8 ms with the split at 12.
 constexpr uint32_t TC_MIN_ROWS = 12;
-// 370 experts, gate/up + down, us: 16 rows 161 + 87 streamed, 17 rows 262 + 138, 20 rows 293 + 154 (two passes over the
-// weights), 32 rows 299 + 156; on the tensor cores 266 + 157, 264 + 160, 269 + 162, 283 + 165, and 338 + 190 with 64 rows.
+// 512 experts, gate/up + down, us under the profiler: 16 rows 203 + 107 streamed, 17 rows 281 + 145 (two passes over the
+// weights), 20 rows 339 + 171, 31 rows 392 + 202; on the tensor cores 236 + 136 with any number of rows up to 32, 283 + 157
+// with 64.  The line is not at 17, where the times cross, because the streamed sums are exact integers per group (error
+// against 64 bits 7e-8 of the result, on the tensor cores 1.9e-7).
 // The line is by the average, which is all the host knows of a layer's rows; a caller's max_rows_hint bounds the largest
-// entry only and is not looked at.  Uneven entries below the line, streamed / on the tensor cores, us: one expert of 512 /
-// 2048 / 8000 rows beside 511 of 2 (gate/up) 124 / 332, 165 / 350, 318 / 414; a layer of 512 experts whose picks follow
-// Zipf(1.1), 64 tokens 100 / 122, 260: 228 / 228, 550: 355 / 284, 920: 528 / 364 (fewer experts are live than could be).
+// entry only and is not looked at.  Uneven entries below the line, streamed / on the tensor cores, us, before either kernel
+// was changed last: one expert of 512 / 2048 / 8000 rows beside 511 of 2 (gate/up) 124 / 332, 165 / 350, 318 / 414; a layer of
+// 512 experts whose picks follow Zipf(1.1), 64 tokens 100 / 122, 260: 228 / 228, 550: 355 / 284, 920: 528 / 364.
 constexpr uint32_t WIDE_TC_ROWS = 20;
 // Does the tensor-core product on the wide form take a call of IQ3_S weights?
 bool takes_wide_tc(const uint8_t *w, uint64_t expert_stride, uint32_t n_entries, uint64_t total_rows, uint32_t cols, uint32_t w_rows) {
