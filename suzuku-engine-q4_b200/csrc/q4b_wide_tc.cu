@@ -68,8 +68,11 @@ struct WItem {
 struct __align__(1024) WSmem {
     uint16_t dr[8][MT];                // d of the last super-blocks, for the epilogue
     WItem items[W_ITEMS];
-    // a super-block decoded, a step of it multiplied; a part's MMAs complete (for the copies, and for the epilogue set that
-    // takes it), its accumulator read, its activations landed
+    // a super-block decoded, a step of it multiplied; a part's MMAs complete (for the copies, and for the epilogue set that takes
+    // it), its accumulator read, its activations landed.  A barrier is waited for by the parity of a phase, so none may be
+    // two phases from the one that a waiter looks for (tests/test_wide_pipeline.py runs the roles under random schedules).  Hence sums
+    // by set AND accumulator: the accumulator takes a part again only when the one before has been read, and its reader has
+    // then seen its phase.  (Four to a set in turn: what orders the parts of a set was in part the other issuing warp's wait.)
     unsigned long long a_full[2], a_free[4], done[W_NSB], sums[2][W_NACC], acc_empty[W_NACC], b_full[W_NSB];
     uint32_t tmem_base, n_items;
 };
@@ -331,7 +334,7 @@ __cluster_dims__(2, 1, 1) __global__ void __launch_bounds__(W_NT, 1) mmq_wide_k(
             });
         } else if (warp < W_ND + W_NE + 2u && !rank) {
             // ---- the first CTA: the MMAs of both, every second step a warp (one lane) ----
-            uint32_t u = 0, tile = 0, at_set[2] = {0, 0};     // parts, tiles, parts of each epilogue set before this tile
+            uint32_t u = 0, tile = 0;     // parts, tiles
             batches([&](uint32_t it, uint32_t n_here) {
                 if (elect_one()) {
                     const uint64_t b_d0 = smem_desc_sw128(smem_u32(sb_base));
@@ -346,10 +349,11 @@ __cluster_dims__(2, 1, 1) __global__ void __launch_bounds__(W_NT, 1) mmq_wide_k(
                                 for (uint32_t p = 0; p < parts; p++, u++) {
                                     const uint32_t np = (min(rows - W_HB * p, W_HB) + W_BOX - 1u) / W_BOX * W_BOX;
                                     const uint32_t idesc = instr_desc(np) + ((MT >> 4) << 24), atom = (np * 64u) >> 4, sb = u % W_NSB;
-                                    if (u >= W_NACC) wait(&s.acc_empty[u % W_NACC], (u / W_NACC - 1u) & 1u, 4u);
+                                    const uint32_t acc = u % W_NACC;
+                                    if (u >= W_NACC) wait(&s.acc_empty[acc], (u / W_NACC - 1u) & 1u, 4u);
                                     wait(&s.b_full[sb], (u / W_NSB) & 1u, 1u);
                                     tc_fence_after();
-                                    const uint32_t d_addr = tmem + (u % W_NACC) * W_HB, a_addr = tmem + W_A_COL + (j & 3u) * 64u;
+                                    const uint32_t d_addr = tmem + acc * W_HB, a_addr = tmem + W_A_COL + (j & 3u) * 64u;
                                     const uint32_t b_lo = b_lo0 + sb * (W_STAGE >> 4);
 #pragma unroll
                                     for (uint32_t c = 0; c < 16; c++) {    // the second plane's first
@@ -358,14 +362,11 @@ __cluster_dims__(2, 1, 1) __global__ void __launch_bounds__(W_NT, 1) mmq_wide_k(
                                                    desc64(b_lo + ((kc >> 2) + (c < 8u ? 2u : 0u)) * atom + (kc & 3u) * 2u, b_hi), idesc, c ? 1u : 0u);
                                     }
                                     mma_commit2(&s.done[sb]);
-                                    const uint32_t set = parts == 2u ? p : tile & 1u;
-                                    mma_commit2(&s.sums[set][((set ? at_set[1] : at_set[0]) + k) % W_NACC]);
+                                    mma_commit2(&s.sums[parts == 2u ? p : tile & 1u][acc]);
                                 }
                                 mma_commit2(&s.a_free[j & 3u]);
                             }
                             u -= (warp & 1u) * parts;
-                            if (parts == 2u || (tile & 1u) == 0) at_set[0] += n_it;
-                            if (parts == 2u || (tile & 1u)) at_set[1] += n_it;
                         }
                     }
                 }
@@ -410,16 +411,16 @@ __cluster_dims__(2, 1, 1) __global__ void __launch_bounds__(W_NT, 1) mmq_wide_k(
         const uint32_t q = warp & 3u, set = (warp >> 2) & 1u, e_row = 32u * q + lane;
         const uint32_t e_addr = tmem + ((32u * q) << 16);
         const uint32_t empty0 = leader_addr(&s.acc_empty[0]);
-        uint32_t u = 0, mine = 0, tile = 0;       // parts, this set's parts, tiles
+        uint32_t u = 0, tile = 0, seen = 0;       // parts, tiles, parity of the phases seen of each accumulator's sums
         batches([&](uint32_t it, uint32_t n_here) {
-            float acc[W_HB / 16u][16];
+            float sum[W_HB / 16u][16];
 #pragma unroll
             for (uint32_t h = 0; h < W_HB / 16u; h++)
 #pragma unroll
-                for (int c = 0; c < 16; c++) acc[h][c] = 0.f;
+                for (int c = 0; c < 16; c++) sum[h][c] = 0.f;
             auto add = [&](uint32_t h, const uint32_t *v, float dr) {
 #pragma unroll
-                for (int c = 0; c < 16; c++) acc[h][c] = fmaf(dr, __uint_as_float(v[c]), acc[h][c]);
+                for (int c = 0; c < 16; c++) sum[h][c] = fmaf(dr, __uint_as_float(v[c]), sum[h][c]);
             };
             uint32_t j = it;
             for (uint32_t i = 0; i < n_here; i++) {
@@ -435,11 +436,13 @@ __cluster_dims__(2, 1, 1) __global__ void __launch_bounds__(W_NT, 1) mmq_wide_k(
                         continue;
                     }
                     u += parts == 2u ? set : 0u;
-                    for (uint32_t k = 0; k < n_it; k++, j++, u += parts, mine++) {
-                        wait(&s.sums[set][mine % W_NACC], (mine / W_NACC) & 1u, 32u);
+                    for (uint32_t k = 0; k < n_it; k++, j++, u += parts) {
+                        const uint32_t acc = u % W_NACC;
+                        wait(&s.sums[set][acc], (seen >> acc) & 1u, 32u);
+                        seen ^= 1u << acc;
                         tc_fence_after();
                         const float dr = __half2float(__ushort_as_half(s.dr[(j >> 1) & 7u][e_row]));
-                        const uint32_t at = e_addr + (u % W_NACC) * W_HB, empty = empty0 + 8u * (u % W_NACC);
+                        const uint32_t at = e_addr + acc * W_HB, empty = empty0 + 8u * acc;
                         uint32_t v[2][16];
                         tmem_ld16(at, v[0]), tmem_ld16(at + 16u, v[1]);
                         tmem_ld_wait();
@@ -466,9 +469,9 @@ __cluster_dims__(2, 1, 1) __global__ void __launch_bounds__(W_NT, 1) mmq_wide_k(
 #pragma unroll
                     for (uint32_t c = 0; c < W_HB; c++) {
                         const float f = __shfl_sync(0xffffffffu, c < 32u ? sc0 : sc1, c & 31u);
-                        if (c < n_out) *o = acc[c >> 4][c & 15u] * f;
+                        if (c < n_out) *o = sum[c >> 4][c & 15u] * f;
                         o += a.ld_dst;
-                        acc[c >> 4][c & 15u] = 0.f;
+                        sum[c >> 4][c & 15u] = 0.f;
                     }
                 }
             }
