@@ -55,7 +55,8 @@ constexpr uint32_t W_NT = 32 * (W_ND + W_NE + 4);   // and a warpgroup: two that
 constexpr uint32_t W_DG = 2;           // pairs of super-blocks of weights in flight per decode warp
 constexpr uint32_t W_SLOT = 4096 + 512;   // their words and records
 constexpr uint32_t W_A_COL = 256;      // weight operand buffers, 128 columns a super-block; the accumulators take the columns below
-constexpr uint32_t W_NACC = W_A_COL / W_HB;   // accumulators
+constexpr uint32_t W_NACC = W_A_COL / W_HB;   // accumulators, two to an issuing warp
+static_assert(W_NACC == 4, "accumulators");
 constexpr uint32_t W_STAGE = W_HB / 2u * 512u;   // a CTA's half of a part's activations of a step: two planes of 128 k
 constexpr uint32_t W_NSB = 8;          // stages
 struct WItem {
@@ -73,6 +74,10 @@ struct __align__(1024) WSmem {
     // two phases from the one that a waiter looks for (tests/test_wide_pipeline.py runs the roles under random schedules).  Hence sums
     // by set AND accumulator: the accumulator takes a part again only when the one before has been read, and its reader has
     // then seen its phase.  (Four to a set in turn: what orders the parts of a set was in part the other issuing warp's wait.)
+    // And an accumulator is used by one issuing warp, two each: it has itself waited for the use before the last one to be read
+    // and issued the last one, so it is that one's phase it finds open or complete.  (All four in turn by either warp: a wait for
+    // a part that the other had still to issue was passed on an older phase, and sums not yet read were overwritten.)  The
+    // issuing warps are three steps apart at most (a_full, a_free), seven parts: a stage's landing is never two phases behind.
     unsigned long long a_full[2], a_free[4], done[W_NSB], sums[2][W_NACC], acc_empty[W_NACC], b_full[W_NSB];
     uint32_t tmem_base, n_items;
 };
@@ -334,7 +339,7 @@ __cluster_dims__(2, 1, 1) __global__ void __launch_bounds__(W_NT, 1) mmq_wide_k(
             });
         } else if (warp < W_ND + W_NE + 2u && !rank) {
             // ---- the first CTA: the MMAs of both, every second step a warp (one lane) ----
-            uint32_t u = 0, tile = 0;     // parts, tiles
+            uint32_t u = 0, v = 0, tile = 0;     // parts, this warp's parts, tiles
             batches([&](uint32_t it, uint32_t n_here) {
                 if (elect_one()) {
                     const uint64_t b_d0 = smem_desc_sw128(smem_u32(sb_base));
@@ -346,11 +351,11 @@ __cluster_dims__(2, 1, 1) __global__ void __launch_bounds__(W_NT, 1) mmq_wide_k(
                             u += (warp & 1u) * parts;
                             for (uint32_t k = warp & 1u; k < n_it; k += 2u, j += 2u, u += parts) {
                                 wait(&s.a_full[(j >> 1) & 1u], (j >> 2) & 1u, 1u);
-                                for (uint32_t p = 0; p < parts; p++, u++) {
+                                for (uint32_t p = 0; p < parts; p++, u++, v++) {
                                     const uint32_t np = (min(rows - W_HB * p, W_HB) + W_BOX - 1u) / W_BOX * W_BOX;
                                     const uint32_t idesc = instr_desc(np) + ((MT >> 4) << 24), atom = (np * 64u) >> 4, sb = u % W_NSB;
-                                    const uint32_t acc = u % W_NACC;
-                                    if (u >= W_NACC) wait(&s.acc_empty[acc], (u / W_NACC - 1u) & 1u, 4u);
+                                    const uint32_t acc = 2u * (warp & 1u) + (v & 1u);
+                                    if (v >= 2u) wait(&s.acc_empty[acc], (v / 2u - 1u) & 1u, 4u);
                                     wait(&s.b_full[sb], (u / W_NSB) & 1u, 1u);
                                     tc_fence_after();
                                     const uint32_t d_addr = tmem + acc * W_HB, a_addr = tmem + W_A_COL + (j & 3u) * 64u;
@@ -411,7 +416,7 @@ __cluster_dims__(2, 1, 1) __global__ void __launch_bounds__(W_NT, 1) mmq_wide_k(
         const uint32_t q = warp & 3u, set = (warp >> 2) & 1u, e_row = 32u * q + lane;
         const uint32_t e_addr = tmem + ((32u * q) << 16);
         const uint32_t empty0 = leader_addr(&s.acc_empty[0]);
-        uint32_t u = 0, tile = 0, seen = 0;       // parts, tiles, parity of the phases seen of each accumulator's sums
+        uint32_t v = 0, tile = 0, seen = 0;       // parts of an issuing warp, tiles, parity of the phases seen of each accumulator's sums
         batches([&](uint32_t it, uint32_t n_here) {
             float sum[W_HB / 16u][16];
 #pragma unroll
@@ -431,13 +436,14 @@ __cluster_dims__(2, 1, 1) __global__ void __launch_bounds__(W_NT, 1) mmq_wide_k(
                 const float sc0 = lane < n ? a.rs[rc + (int32_t)lane] : 0.f;
                 const float sc1 = lane + 32u < n ? a.rs[rc + 32 + (int32_t)lane] : 0.f;
                 for (uint32_t m = 0; m < a.mt; m++, tile++) {
+                    const uint32_t v0 = v + (parts == 2u ? set : 0u);
+                    v += n_it / 2u * parts;                  // (n_it is even: as many of either warp)
                     if (parts == 1u && (tile & 1u) != set) {
-                        u += n_it, j += n_it;
+                        j += n_it;
                         continue;
                     }
-                    u += parts == 2u ? set : 0u;
-                    for (uint32_t k = 0; k < n_it; k++, j++, u += parts) {
-                        const uint32_t acc = u % W_NACC;
+                    for (uint32_t k = 0; k < n_it; k++, j++) {
+                        const uint32_t acc = 2u * (k & 1u) + ((v0 + (k >> 1) * parts) & 1u);
                         wait(&s.sums[set][acc], (seen >> acc) & 1u, 32u);
                         seen ^= 1u << acc;
                         tc_fence_after();
@@ -461,7 +467,6 @@ __cluster_dims__(2, 1, 1) __global__ void __launch_bounds__(W_NT, 1) mmq_wide_k(
                             add(0, v[0], dr), add(1, v[1], dr);
                         }
                     }
-                    u -= parts == 2u ? set : 0u;
                     // the tile is complete: write its rows out
                     const uint32_t t_row = row0 + m * 2u * MT;
                     float *o = a.dst + (int64_t)rc * (int64_t)a.ld_dst + t_row + e_row;

@@ -201,6 +201,47 @@ def test_tensor_core_product_with_several_batches_of_items(dev, pkg, cols, tiles
         lib.q4_hip_experts_free_a(1)
 
 
+@pytest.mark.parametrize("cols,w_rows,n_exp", [(256, 256, 888), (256, 2816, 90), (512, 256, 600), (512, 384, 300), (2048, 128, 296)])
+def test_tensor_core_product_with_passes_of_one_and_two_parts(dev, pkg, cols, w_rows, n_exp):
+    """Entries of more than 64 rows (two parts) and of at most 64 (one part) in random order, several items to a pair of CTAs:
+    the two sets of adding warps take every part of the first and every second tile of the second, and an accumulator goes
+    from one set to the other.  Items of one super-block (256 columns, 256 and 2816 rows) up to eight."""
+    rng = np.random.default_rng(cols + w_rows)
+    per = np.where(rng.random(n_exp) < 0.5, rng.integers(1, 65, n_exp), rng.integers(65, 129, n_exp))
+    _tensor_core_against_general(dev, pkg, cols, w_rows, per, 1)
+
+
+def _tensor_core_against_general(dev, pkg, cols, w_rows, per, mode):
+    """A call of mmq_wide_k and of the general kernel, per[e] rows of expert e.  The experts' matrices overlap (an expert starts one tile after the one
+    before)."""
+    import torch
+    lib, n_exp, rows, rb = dev.lib, len(per), int(per.sum()), cols // 256 * 110
+    rng = np.random.default_rng(cols)
+    pack = pkg.synth.iq3s_blocks(rng, (w_rows * rb + (n_exp - 1) * 880) // 110).reshape(-1)
+    lib.q4_cuda_set_tiled_default(2)
+    try:
+        assert lib.q4_hip_experts_alloc_a(1, 1, pack.nbytes)
+    finally:
+        lib.q4_cuda_set_tiled_default(1)
+    try:
+        assert lib.q4_hip_experts_put_a(1, 0, pack.ctypes.data, pack.nbytes) and lib.q4_cuda_experts_wide_a(1) == 1
+        x, d_xq = rng.standard_normal((rows, cols)).astype(np.float32), dev.malloc(lib.q4_mmq_q8_bytes(rows, cols))
+        bounds, out = dev.upload(np.concatenate([[0], np.cumsum(per)]).astype(np.int32)), []
+        for m in (mode, 2):
+            y = torch.full((rows, w_rows), 7.5, device="cuda")
+            torch.cuda.synchronize()
+            assert lib.q4_cuda_mmq_tc_mode(m) and lib.q4_mmq_quantize(dev.upload(x), None, d_xq, IQ3_S, cols, rows)
+            assert lib.q4_mmq_mul_id(lib.q4_hip_experts_base_a(1), IQ3_S, w_rows, cols, 880, n_exp, d_xq, bounds, int(per.max()), rows,
+                                     y.data_ptr(), w_rows)
+            assert lib.q4_cuda_device_error() == 0
+            out.append(y.view(rows, w_rows // 128, 128))
+        off, ref = (out[0] - out[1]).norm(dim=2), out[1].norm(dim=2)
+        assert (ref > 0).all() and (off <= 1e-5 * ref).all(), float((off / ref).max())
+    finally:
+        lib.q4_cuda_mmq_tc_mode(-1)
+        lib.q4_hip_experts_free_a(1)
+
+
 @pytest.mark.parametrize("H,F", [(2048, 512), (1024, 256), (2560, 768), (256, 256), (1280, 256)])
 @pytest.mark.parametrize("per", [[1, 31, 32, 33, 0, 63], [64, 65, 128, 2, 129, 0], [0, 16, 0, 0, 0, 0], [200, 1, 1, 95, 96, 97]])
 def test_tensor_core_product_at_the_edges_of_its_passes(dev, pkg, H, F, per):

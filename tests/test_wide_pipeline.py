@@ -88,19 +88,15 @@ class Pair:
                 j += 2
 
     def issue(self, w):
-        u, j, tile = 0, w, 0
+        u, v, j, tile = 0, 0, w, 0
         for parts in self.tiles():
             u += w * parts
             for k in range(w, self.n_it, 2):
                 yield self.a_full[0][(j >> 1) & 1], (j >> 2) & 1
                 for p in range(parts):
-                    acc = u % NACC
-                    for n in range(5000):      # (how it waits for the part before is not in the model)
-                        if u < NACC or self.read.get(u - NACC) == 2:
-                            break
-                        yield 1.0
-                    else:
-                        raise AssertionError("an accumulator is never read")
+                    acc = 2 * w + (v & 1)
+                    if v >= 2:
+                        yield self.acc_empty[acc], (v // 2 - 1) & 1
                     yield self.b_full[0][u % NSB], (u // NSB) & 1
                     last = self.acc[acc]
                     assert last is None or self.read.get(last[0]) == 2, "an accumulator is overwritten before it is read"
@@ -108,7 +104,7 @@ class Pair:
                     self.pipe[w].put((acc, u, j))
                     s = p if parts == 2 else tile & 1
                     self.pipe[w].put([self.done[r][u % NSB] for r in (0, 1)] + [self.sums[r][s][acc] for r in (0, 1)])
-                    u += 1
+                    u, v = u + 1, v + 1
                 self.pipe[w].put([self.a_free[r][j & 3] for r in (0, 1)])
                 j += 2
                 u += parts
@@ -164,14 +160,15 @@ class Pair:
                 g += 1
 
     def add(self, r, s):
-        u = j = tile = seen = 0
+        v = j = tile = seen = first = 0                      # (first, u: which part it is, for the checks alone)
         for parts in self.tiles():
+            v0, u = v + (s if parts == 2 else 0), first + (s if parts == 2 else 0)
+            v, first = v + self.n_it // 2 * parts, first + self.n_it * parts
             if parts == 1 and (tile & 1) != s:
-                u, j = u + self.n_it, j + self.n_it
+                j += self.n_it
             else:
-                u += s if parts == 2 else 0
                 for k in range(self.n_it):
-                    acc = u % NACC
+                    acc = 2 * (k & 1) + ((v0 + (k >> 1) * parts) & 1)
                     yield self.sums[r][s][acc], (seen >> acc) & 1
                     seen ^= 1 << acc
                     assert self.acc[acc] == [u, True], "an accumulator of another part is read"
@@ -183,7 +180,6 @@ class Pair:
                     u, j = u + parts, j + 1
                     if self.rng.random() < 0.05:
                         yield 30.0
-                u -= s if parts == 2 else 0
                 yield 30.0                                   # a finished tile is stored
             tile += 1
 
@@ -231,7 +227,9 @@ def test_the_model_has_the_rules_of_the_kernel():
     for line in ("wait(&s.b_full[u % W_NSB], (u / W_NSB) & 1u, 1u)",
                  "wait(&s.a_full[(j >> 1) & 1u], (j >> 2) & 1u, 1u)",
                  "wait(&s.b_full[sb], (u / W_NSB) & 1u, 1u)",
-                 "const uint32_t acc = u % W_NACC",
+                 "const uint32_t acc = 2u * (warp & 1u) + (v & 1u); if (v >= 2u) wait(&s.acc_empty[acc], (v / 2u - 1u) & 1u, 4u);",
+                 "const uint32_t v0 = v + (parts == 2u ? set : 0u); v += n_it / 2u * parts;",
+                 "const uint32_t acc = 2u * (k & 1u) + ((v0 + (k >> 1) * parts) & 1u); wait(&s.sums[set][acc], (seen >> acc) & 1u, 32u);",
                  "mma_commit2(&s.done[sb]); mma_commit2(&s.sums[parts == 2u ? p : tile & 1u][acc]);",
                  "mma_commit2(&s.a_free[j & 3u])",
                  "if (u >= W_NSB) wait(&s.done[sb], (u / W_NSB - 1u) & 1u, 16u)",
