@@ -164,41 +164,20 @@ print("lent ok")
     assert r.returncode == 0 and "lent ok" in r.stdout, r.stdout + r.stderr
 
 
-@pytest.mark.parametrize("cols,tiles", [(256, 41), (512, 19)])
+@pytest.mark.parametrize("cols,tiles", [(256, 37), (512, 25)])
 def test_tensor_core_product_with_several_batches_of_items(dev, pkg, cols, tiles):
-    """A block of the tensor-core product takes in the descriptors of 128 work items at a time: calls with 283 and 132 of
-    them a block, of 18 to 22 rows, whose pipeline runs on from one batch into the next.  The experts' matrices overlap (an
-    expert starts one tile after the one before)."""
+    """A pair of CTAs takes in the descriptors of 128 work items at a time, and its pipeline runs on from one batch into the next.
+    The launcher makes an item of as many pairs of 128-row tiles as take 16 steps of 128 k and divide their number; 19 and 13
+    are prime, so an item is one: 263 and 180 a pair of CTAs on 148 SMs.  One entry in seven has two parts."""
     import torch
-    lib, n_exp, w_rows = dev.lib, 1023, 128 * tiles
-    per = 20 + (np.arange(n_exp) * 7 % 5 - 2)
+    n_exp, steps, pairs = 1023, cols // 128, (tiles + 1) // 2
+    per = np.where(np.arange(n_exp) % 7 == 0, 80, 10)
     per[-1] += 20 * n_exp - per.sum()
-    rows, rb = int(per.sum()), cols // 256 * 110
-    assert n_exp * tiles > 128 * 148
-    rng = np.random.default_rng(cols)
-    pack = pkg.synth.iq3s_blocks(rng, (w_rows * rb + (n_exp - 1) * 880) // 110).reshape(-1)
-    lib.q4_cuda_set_tiled_default(2)
-    try:
-        assert lib.q4_hip_experts_alloc_a(1, 1, pack.nbytes)
-    finally:
-        lib.q4_cuda_set_tiled_default(1)
-    try:
-        assert lib.q4_hip_experts_put_a(1, 0, pack.ctypes.data, pack.nbytes) and lib.q4_cuda_experts_wide_a(1) == 1
-        x, d_xq = rng.standard_normal((rows, cols)).astype(np.float32), dev.malloc(lib.q4_mmq_q8_bytes(rows, cols))
-        bounds, out = dev.upload(np.concatenate([[0], np.cumsum(per)]).astype(np.int32)), []
-        for mode in (-1, 2):
-            y = torch.full((rows, w_rows), 7.5, device="cuda")
-            torch.cuda.synchronize()
-            assert lib.q4_cuda_mmq_tc_mode(mode) and lib.q4_mmq_quantize(dev.upload(x), None, d_xq, IQ3_S, cols, rows)
-            assert lib.q4_mmq_mul_id(lib.q4_hip_experts_base_a(1), IQ3_S, w_rows, cols, 880, n_exp, d_xq, bounds, 40, rows,
-                                     y.data_ptr(), w_rows)
-            assert lib.q4_cuda_device_error() == 0
-            out.append(y.view(rows, tiles, 128))
-        off, ref = (out[0] - out[1]).norm(dim=2), out[1].norm(dim=2)
-        assert (ref > 0).all() and (off <= 1e-5 * ref).all(), float((off / ref).max())
-    finally:
-        lib.q4_cuda_mmq_tc_mode(-1)
-        lib.q4_hip_experts_free_a(1)
+    assert 0 < per.min() and per.max() <= 128                # a pass an entry
+    mt = max(c for c in range(1, pairs + 1) if c == 1 or (c * steps <= 16 and pairs % c == 0))
+    ctas = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    assert n_exp * (pairs // mt) > 128 * ctas                # more than one batch for every pair of CTAs
+    _tensor_core_against_general(dev, pkg, cols, 128 * tiles, per, -1)
 
 
 @pytest.mark.parametrize("cols,w_rows,n_exp", [(256, 256, 888), (256, 2816, 90), (512, 256, 600), (512, 384, 300), (2048, 128, 296)])
@@ -245,8 +224,8 @@ def _tensor_core_against_general(dev, pkg, cols, w_rows, per, mode):
 @pytest.mark.parametrize("H,F", [(2048, 512), (1024, 256), (2560, 768), (256, 256), (1280, 256)])
 @pytest.mark.parametrize("per", [[1, 31, 32, 33, 0, 63], [64, 65, 128, 2, 129, 0], [0, 16, 0, 0, 0, 0], [200, 1, 1, 95, 96, 97]])
 def test_tensor_core_product_at_the_edges_of_its_passes(dev, pkg, H, F, per):
-    """Rows at the edges of the MMA's N (32) and of a pass (64), rows of 1 to 10 super-blocks.  (An odd
-    number of 128-row tiles: the test above.)
+    """Rows at the edges of the MMA's N (32), of a part (64) and of a pass (128), rows of 1 to 10 super-blocks.  (An odd
+    number of 128-row tiles: the tests above.)
     Against the general kernel: activations carry 22 bits there (2^-23 of the row's largest group a term, of random
     sign) and the tensor core truncates eight additions of 24 bits per 128 k: a few 1e-7 of the result; bound 1e-5."""
     rng = np.random.default_rng(H + F + sum(per))
