@@ -30,14 +30,17 @@ def test_route_pf_matches_host_softmax_topk(dev, oracle):
     assert not dev.lib.q4_hip_route_pf(dev.upload(logits), d_ids, d_w, n_tok, n_exp, 0)
 
 
-@pytest.mark.parametrize("n_tok", [1, 4, 8, 9, 37, 64, 256])
-def test_one_launch_routing_is_the_three_launches_bit_for_bit(dev, n_tok):
+@pytest.mark.parametrize("n_exp,n_tok", [(512, n) for n in (1, 4, 8, 9, 37, 64, 256)] +
+                         [(509, 67), (101, 251), (509, 131), (510, 147), (163, 253)])
+def test_one_launch_routing_is_the_three_launches_bit_for_bit(dev, n_exp, n_tok):
     """q4_cuda_route_small (norm + router product + top-k in one launch, a counter per group of eight
     tokens) against q4_hip_grouped_rms_n + q4_hip_gemv_dd_n + q4_hip_route_pf on the same rows, twice in
-    a row (the counters must be back at zero); a batch beyond its limit is refused with nothing queued."""
+    a row (the counters must be back at zero), and nothing behind the last row; a batch beyond its limit is refused with nothing
+    queued.  The pairs behind the first seven: two router rows a warp (509 and 101 experts leave a warp one), and four (509 leave
+    one, 510 two, 163 three), with a last group of three or five tokens."""
     lib = dev.lib
     rng = np.random.default_rng(100 + n_tok)
-    n_exp, topk, n = 512, 10, 2048
+    topk, n = 10, 2048
     x = (rng.standard_normal((n_tok, n)) * rng.uniform(0.1, 30.0, (n_tok, 1))).astype(np.float32)
     nw = rng.uniform(0.5, 1.5, n).astype(np.float32)
     router = (rng.standard_normal((n_exp, n)) * 0.02).astype(np.float32)
@@ -57,13 +60,13 @@ def test_one_launch_routing_is_the_three_launches_bit_for_bit(dev, n_tok):
             ref = (dev.download(d_xn0, (n_tok, n), np.uint32), dev.download(d_lg0, (n_tok, n_exp), np.uint32),
                    dev.download(d_i0, (n_tok, topk), np.int32), dev.download(d_w0, (n_tok, topk), np.uint32))
         for rep in range(2):
-            d_xn, d_lg = dev.malloc(n_tok * n * 4), dev.malloc(n_tok * n_exp * 4)
-            d_i, d_w = dev.malloc(n_tok * topk * 4), dev.malloc(n_tok * topk * 4)
+            rows = (n_tok + 7) // 8 * 8 + 1
+            d_xn, d_lg, d_i, d_w = (dev.upload(np.full((rows, c), 0x7a7a7a7a, np.uint32)) for c in (n, n_exp, topk, topk))
             assert lib.q4_cuda_route_small(d_x, nw_ptr, 1e-6, d_r, n_exp, topk, n, n_tok, d_xn, d_lg, d_i, d_w)
-            got = (dev.download(d_xn, (n_tok, n), np.uint32), dev.download(d_lg, (n_tok, n_exp), np.uint32),
-                   dev.download(d_i, (n_tok, topk), np.int32), dev.download(d_w, (n_tok, topk), np.uint32))
-            for a, b, what in zip(got, ref, ("xn", "logits", "ids", "weights")):
-                assert (a == b).all(), (what, rep)
+            for d, b, what in zip((d_xn, d_lg, d_i, d_w), ref, ("xn", "logits", "ids", "weights")):
+                got = dev.download(d, (rows, b.shape[1]), b.dtype)
+                assert (got[:n_tok] == b).all(), (what, rep)
+                assert (got[n_tok:] == 0x7a7a7a7a).all(), (what, rep)
     assert not lib.q4_cuda_route_small(d_x, d_nw, 1e-6, d_r, n_exp, topk, n, 257, d_xn, d_lg, d_i, d_w)
     assert not lib.q4_cuda_route_small(d_x, d_nw, 1e-6, d_r, n_exp, topk, 1024, n_tok, d_xn, d_lg, d_i, d_w)
     assert lib.q4_cuda_device_error() == 0
