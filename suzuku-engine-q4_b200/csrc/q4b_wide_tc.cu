@@ -64,7 +64,6 @@ struct WItem {
     int32_t rc;                        // first activation row
     uint32_t nrows;                    // rows of the pass
     uint32_t row0;                     // first weight row
-    uint32_t pad;
 };
 struct __align__(1024) WSmem {
     uint16_t dr[8][MT];                // d of the last super-blocks, for the epilogue
@@ -79,7 +78,7 @@ struct __align__(1024) WSmem {
     // a part that the other had still to issue was passed on an older phase, and sums not yet read were overwritten.)  The
     // issuing warps are three steps apart at most (a_full, a_free), seven parts: a stage's landing is never two phases behind.
     unsigned long long a_full[2], a_free[4], done[W_NSB], sums[2][W_NACC], acc_empty[W_NACC], b_full[W_NSB];
-    uint32_t tmem_base, n_items;
+    uint32_t tmem_base;
 };
 constexpr uint32_t W_B_OFF = (uint32_t)((sizeof(WSmem) + 1023u) & ~1023u);   // then activation stages, weight ring
 
@@ -295,7 +294,8 @@ __cluster_dims__(2, 1, 1) __global__ void __launch_bounds__(W_NT, 1) mmq_wide_k(
     // this CTA's tile at or behind a row (of an odd number of tiles the second CTA's last one is the first CTA's, and not stored)
     auto tile_row = [&](uint32_t row) { return row < a.w_rows ? row : row - MT; };
     // A role's part of every batch of items: body(steps before the batch, items).  The counters of steps, and those of parts
-    // that roles keep, run on over the batches: barrier phases follow them.  (The threads of a warp may come to the barrier one by one: of some only one lane works.)
+    // that roles keep, run on over the batches: barrier phases follow them.  (The threads of a warp may come to the barrier
+    // one by one: of some only one lane works.)
     auto batches = [&](auto body) {
         uint32_t it = 0;
         for (uint32_t first = 0; first < n_mine; first += W_ITEMS) {

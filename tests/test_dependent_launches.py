@@ -8,7 +8,7 @@ import re
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "suzuku-engine-q4_b200", "csrc")
 CONSTANT = {"w", "W", "w4", "g4", "norm_w", "bg", "bu", "bd", "grid3", "grid2", "codes"}
 # device functions that such kernels run
-HELPERS = ("stream_items", "stack_body", "store_tile_lanes", "softmax_topk_regs", "small_group", "quant_planes", "layer_pick")
+HELPERS = ("stream_items", "stack_body", "softmax_topk_regs", "small_group", "quant_planes", "layer_pick")
 
 
 def _functions():
