@@ -1406,7 +1406,6 @@ bool q4b_route_small_warm() {
     if (cudaMalloc(&g_route_counter, (ROUTE_MAX_TOK / 8u) * sizeof(unsigned int)) != cudaSuccess ||
         cudaMemset(g_route_counter, 0, (ROUTE_MAX_TOK / 8u) * sizeof(unsigned int)) != cudaSuccess ||
         cudaFuncSetAttribute(route_small_k<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 2048 * 4) != cudaSuccess ||
-        cudaFuncSetAttribute(route_small_k<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 2048 * 4) != cudaSuccess ||
         cudaFuncSetAttribute(route_small_k<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 2048 * 4) != cudaSuccess) {
         cudaGetLastError();
         return false;
@@ -1423,15 +1422,16 @@ bool q4b_route_small(const float *x, const float *norm_w, float eps, const float
     if (!g_route_counter || n_embd != 2048u || n_tok == 0 || n_tok > ROUTE_MAX_TOK || n_expert > 1024u ||
         topk > 64u || (((uintptr_t)router | (uintptr_t)x | (uintptr_t)norm_w | (uintptr_t)xn) & 15u))
         return false;
-    // Router rows a warp: one while that leaves about two CTAs an SM (each normalises eight tokens, and reads them from shared
-    // memory for every row), else two or four, which are read the tokens for at once.  512 experts, us a call: one row 33 tokens
-    // 15.8 (two rows, an earlier form: 19.9), 64 tokens 25.3, 128 43.5, 256 74.5; two rows 64 tokens 17.6; four 128 tokens
-    // 24.9, 256 44.2.  160 experts, 256 tokens: one row 34.1, four 23.4.
-    const uint32_t groups = (n_tok + 7u) / 8u, sm = (uint32_t)g_q4b.n_sm;
-    auto ctas = [&](uint32_t per) { return groups * ((n_expert + 8u * per - 1u) / (8u * per)); };
-    const uint32_t per = 4u * ctas(1) <= 9u * sm ? 1u : ctas(2) <= 2u * sm ? 2u : 4u;
-    q4b_launch(per == 1u ? route_small_k<1> : per == 2u ? route_small_k<2> : route_small_k<4>, dim3(ctas(per) / groups, groups), 256,
-        8u * 2048u * 4u, g_q4b.stream,
+    // Router rows a warp: one, whose CTAs multiply with the tokens that there are only, for up to three groups of tokens while all
+    // its CTAs are resident at once (two an SM), and where it has few (a quarter of the SMs); else four, which read a
+    // token's shared memory once.  us of a whole layer call (experts x tokens), one row / four: 512 x 9 80.3 / 80.9, 512 x 16
+    // 99.3 / 99.8, 512 x 24 115.3 / 115.0, 512 x 32 131.5 / 131.0, 512 x 40 144.5 / 137.9 (320 CTAs), 256 x 9 76.9 / 78.6, 256 x 24
+    // 105.8 / 106.3, 256 x 40 127.2 / 126.4, 256 x 80 163.9 / 156.9, 160 x 64 134.5 / 133.4, 128 x 40 111.6 / 111.0.  Of this kernel alone,
+    // call behind call: 512 x 1 8.2 / 12.7, 1024 x 24 (384 CTAs) 27.0 / 18.0, 64 x 24 (24 CTAs) 12.1 / 13.8, 128 x 16 (32) 12.3 / 13.9,
+    // 48 x 256 (192) 17.0 / 14.1, 512 x 64 25.4 / 15.1, 512 x 256 73.7 / 43.8.  (Two rows: 17.4 and 48.0 for the last two.)
+    const uint32_t groups = (n_tok + 7u) / 8u, one = (n_expert + 7u) / 8u, four = (n_expert + 31u) / 32u, sm = (uint32_t)g_q4b.n_sm;
+    const bool by_one = (groups <= 3u && groups * one <= 2u * sm) || 4u * groups * one <= sm;
+    q4b_launch(by_one ? route_small_k<1> : route_small_k<4>, dim3(by_one ? one : four, groups), 256, 8u * 2048u * 4u, g_q4b.stream,
         x, norm_w, eps, router, n_expert, n_tok, topk, xn, logits, ids, wts, g_route_counter);
     g_q4b_launches++;
     return q4b_launch_ok("route_small");
