@@ -1005,9 +1005,9 @@ constexpr uint32_t TC_MIN_ROWS = 12;
 // with 64.  The line is not at 17, where the times cross, because the streamed sums are exact integers per group (error
 // against 64 bits 7e-8 of the result, on the tensor cores 1.9e-7).
 // The line is by the average, which is all the host knows of a layer's rows; a caller's max_rows_hint bounds the largest
-// entry only and is not looked at.  Uneven entries below the line, streamed / on the tensor cores, us, before either kernel
-// was changed last: one expert of 512 / 2048 / 8000 rows beside 511 of 2 (gate/up) 124 / 332, 165 / 350, 318 / 414; a layer of
-// 512 experts whose picks follow Zipf(1.1), 64 tokens 100 / 122, 260: 228 / 228, 550: 355 / 284, 920: 528 / 364.
+// entry only and is not looked at.  Uneven entries below the line, streamed / on the tensor cores, us a call: one expert of
+// 512 / 2048 / 8000 rows beside 511 of 2 (gate/up) 117 / 239, 158 / 252, 298 / 310; both products of a layer of 512
+// experts whose picks follow Zipf(1.1), 64 tokens 53 / 83, 260: 127 / 131, 400: 174 / 137, 550: 223 / 170, 920: 350 / 228.
 constexpr uint32_t WIDE_TC_ROWS = 20;
 // Does the tensor-core product on the wide form take a call of IQ3_S weights?
 bool takes_wide_tc(const uint8_t *w, uint64_t expert_stride, uint32_t n_entries, uint64_t total_rows, uint32_t cols, uint32_t w_rows) {
