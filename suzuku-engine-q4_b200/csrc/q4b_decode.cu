@@ -1422,15 +1422,15 @@ bool q4b_route_small(const float *x, const float *norm_w, float eps, const float
     if (!g_route_counter || n_embd != 2048u || n_tok == 0 || n_tok > ROUTE_MAX_TOK || n_expert > 1024u ||
         topk > 64u || (((uintptr_t)router | (uintptr_t)x | (uintptr_t)norm_w | (uintptr_t)xn) & 15u))
         return false;
-    // Router rows a warp: one, whose CTAs multiply with the tokens that there are only, for up to three groups of tokens while all
-    // its CTAs are resident at once (two an SM), and where it has few (a quarter of the SMs); else four, which read a
-    // token's shared memory once.  us of a whole layer call (experts x tokens), one row / four: 512 x 9 80.3 / 80.9, 512 x 16
-    // 99.3 / 99.8, 512 x 24 115.3 / 115.0, 512 x 32 131.5 / 131.0, 512 x 40 144.5 / 137.9 (320 CTAs), 256 x 9 76.9 / 78.6, 256 x 24
-    // 105.8 / 106.3, 256 x 40 127.2 / 126.4, 256 x 80 163.9 / 156.9, 160 x 64 134.5 / 133.4, 128 x 40 111.6 / 111.0.  Of this kernel alone,
-    // call behind call: 512 x 1 8.2 / 12.7, 1024 x 24 (384 CTAs) 27.0 / 18.0, 64 x 24 (24 CTAs) 12.1 / 13.8, 128 x 16 (32) 12.3 / 13.9,
-    // 48 x 256 (192) 17.0 / 14.1, 512 x 64 25.4 / 15.1, 512 x 256 73.7 / 43.8.  (Two rows: 17.4 and 48.0 for the last two.)
-    const uint32_t groups = (n_tok + 7u) / 8u, one = (n_expert + 7u) / 8u, four = (n_expert + 31u) / 32u, sm = (uint32_t)g_q4b.n_sm;
-    const bool by_one = (groups <= 3u && groups * one <= 2u * sm) || 4u * groups * one <= sm;
+    // Router rows a warp: one, whose CTAs (two an SM) multiply with the tokens that there are only, while they have no more to do than
+    // one wave of CTAs with eight tokens each; else four, which read a token's shared memory once.  us of a whole layer call (experts x
+    // tokens), one row / four, IQ4_XS + IQ4_NL experts: 512 x 25 193 / 198, 512 x 33 229 / 234, 512 x 36 243 / 248, 512 x 40 266 / 259,
+    // 512 x 64 354 / 344, 200 x 32 218 / 220, 200 x 72 297 / 296, 200 x 128 355 / 344; IQ3_S: 512 x 9 80.3 / 80.9, 512 x 24 115.3 / 115.0,
+    // 512 x 36 133.6 / 132.8, 512 x 38 140.1 / 135.5, 512 x 40 144.5 / 137.9, 256 x 9 76.9 / 78.6, 256 x 72 153.8 / 152.6, 256 x 76 157.8 /
+    // 154.8, 256 x 80 163.9 / 156.9, 160 x 112 153.0 / 150.8, 160 x 120 160.4 / 155.1.  Below the line the better form changes with what
+    // runs around it.  (Two rows, this kernel call behind call: 512 x 64 17.4, 512 x 256 48.0, with one 25.4 and 73.7, with four 15.1 and 43.8.)
+    const uint32_t groups = (n_tok + 7u) / 8u, one = (n_expert + 7u) / 8u, four = (n_expert + 31u) / 32u;
+    const bool by_one = n_tok * one <= 8u * 2u * (uint32_t)g_q4b.n_sm;
     q4b_launch(by_one ? route_small_k<1> : route_small_k<4>, dim3(by_one ? one : four, groups), 256, 8u * 2048u * 4u, g_q4b.stream,
         x, norm_w, eps, router, n_expert, n_tok, topk, xn, logits, ids, wts, g_route_counter);
     g_q4b_launches++;
